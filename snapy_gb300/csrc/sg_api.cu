@@ -1277,12 +1277,13 @@ int sg_stage(sg_handle* h, int32_t stage, const double* dt_dev,
                                     timed ? ev + 2 : nullptr);
     if (rc) return cuda_fail((cudaError_t)rc, "sg_stage: implicit solve");
     if (timed) cudaEventRecord(ev[4], s);
-    // assembly, solve, finish; the refined solve adds its FP32 sweep and a
-    // residual and a correction per correction
+    // assembly, solve, finish; the refined solve adds its FP32 sweep, a
+    // residual and a sweep per correction, the acceptance and the left-over
+    // columns' solve
     // (a wide batch's finish is three launches)
     launches += 3 + (h->wide ? 2 : 0) + (h->vic_kinds == 3 ? 1 : 0) +
                 (h->asm_kinds == 3 ? 1 : 0) +
-                (h->refine > 0 ? 2 + 2 * h->refine : (h->refine < 0 ? 3 : 0)) +
+                (h->refine ? 3 + 2 * std::max(h->refine, 0) : 0) +
                 (h->psw_on ? 1 : 0);
   }
   if (h->scalars) {

@@ -276,22 +276,17 @@ __global__ void __launch_bounds__(32)
   const unsigned full = 0xffffffffu;
   PswScratch W;
   int* maskp;
-  const float *A32 = nullptr, *B32 = nullptr, *C32 = nullptr;
+  const VicScratch32 F32 = BLK32 ? vic_scratch32(Bk, S, n) : VicScratch32{};
   if (BLK32) {
-    const VicScratch32 F32 = vic_scratch32(Bk, S, n);
     maskp = F32.mask + col;
     if (*maskp != 1) return;  // uniform over the warp
     W.E = S.A;
     W.F = S.B;
-    A32 = F32.A + col * n * kBlk32;
-    B32 = F32.B + col * n * kBlk32;
-    C32 = F32.C + col * n * kBlk32;
     if (threadIdx.x == 0) count_fp64_column(p, blockIdx.y);
   } else {
     W = psw_scratch(Bk, S.cells);
     maskp = W.mask + col;
   }
-  const int bst = BLK32 ? kBlk32 : 25;  // the row of a cell's block
   const int lane = threadIdx.x, g = lane / kVicLanes, q = lane % kVicLanes;
   const bool colane = q < 5;
   // chunks: m = n - 3 layers in four chunks of L or L + 1 layers; chunk g
@@ -306,9 +301,12 @@ __global__ void __launch_bounds__(32)
   const double* A = S.A + col * n * 25;
   const double* Bm = S.B + col * n * 25;
   const double* C = S.C + col * n * 25;
-  auto blkA = [&](int e) -> double { return BLK32 ? widen_exact(A32[e]) : A[e]; };
-  auto blkB = [&](int e) -> double { return BLK32 ? widen_exact(B32[e]) : Bm[e]; };
-  auto blkC = [&](int e) -> double { return BLK32 ? widen_exact(C32[e]) : C[e]; };
+  const VicCol32 A32(F32.A, ncol, col, n), B32(F32.B, ncol, col, n),
+      C32(F32.C, ncol, col, n);
+  // entry k of layer i
+  auto blkA = [&](int i, int k) -> double { return BLK32 ? A32(i, k) : A[i * 25 + k]; };
+  auto blkB = [&](int i, int k) -> double { return BLK32 ? B32(i, k) : Bm[i * 25 + k]; };
+  auto blkC = [&](int i, int k) -> double { return BLK32 ? C32(i, k) : C[i * 25 + k]; };
   const double* du = S.du + col * n;
   double* D = S.D + col * n * 5;
   double* Z0 = S.Z0 + col * n * 5;
@@ -332,12 +330,12 @@ __global__ void __launch_bounds__(32)
   {
     const int i = s0;
 #pragma unroll
-    for (int e = 0; e < 25; ++e) b[e] = blkB(i * bst + e);
+    for (int e = 0; e < 25; ++e) b[e] = blkB(i, e);
     if (colane) {
 #pragma unroll
       for (int r = 0; r < 5; ++r) {
-        xa[r] = blkA(i * bst + r * 5 + q);
-        xc[r] = blkC(i * bst + r * 5 + q);
+        xa[r] = blkA(i, r * 5 + q);
+        xc[r] = blkC(i, r * 5 + q);
       }
     }
   }
@@ -362,7 +360,7 @@ __global__ void __launch_bounds__(32)
       // the left separator's coupling moves to the right-hand side
       if (g > 0 && colane) {
 #pragma unroll
-        for (int r = 0; r < 5; ++r) v5[r] = -blkB(i * bst + r * 5 + q);
+        for (int r = 0; r < 5; ++r) v5[r] = -blkB(i, r * 5 + q);
       }
     } else {
       psw_sub_mv(x, b, s);
@@ -372,12 +370,12 @@ __global__ void __launch_bounds__(32)
     if (t + 1 < L) {
       const int i1 = i + 1;
 #pragma unroll
-      for (int e = 0; e < 25; ++e) b[e] = blkB(i1 * bst + e);
+      for (int e = 0; e < 25; ++e) b[e] = blkB(i1, e);
       if (colane) {
 #pragma unroll
         for (int r = 0; r < 5; ++r) {
-          xa[r] = blkA(i1 * bst + r * 5 + q);
-          xc[r] = blkC(i1 * bst + r * 5 + q);
+          xa[r] = blkA(i1, r * 5 + q);
+          xc[r] = blkC(i1, r * 5 + q);
         }
       }
     }
@@ -512,14 +510,14 @@ __global__ void __launch_bounds__(32)
     double bs[25], cs[25];
 #pragma unroll
     for (int k = 0; k < 25; ++k) {
-      bs[k] = blkB(sg * bst + k);
-      cs[k] = blkC(sg * bst + k);
+      bs[k] = blkB(sg, k);
+      cs[k] = blkC(sg, k);
     }
     if (colane) {
       double ah[5], bh[5], ch[5];
 #pragma unroll
       for (int r = 0; r < 5; ++r) {
-        double a = blkA(sg * bst + r * 5 + q), bb = 0., c = 0.;
+        double a = blkA(sg, r * 5 + q), bb = 0., c = 0.;
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
           a = fma(-bs[r * 5 + k], cpe[k], a);

@@ -2180,6 +2180,7 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 #include "sg_vic.cuh"
+#include "sg_rsolve.cuh"
 #include "sg_psolve.cuh"
 
 // an implicit block's scalars after its solve, one warp per column and
@@ -2528,21 +2529,17 @@ extern "C" int SG_NAME(sg_launch_vic)(const BlockDev* tab, StageParams p,
   // Woodbury step alone; the columns either leaves are solved directly
   int gs = (int)((max_cols + kVicCols - 1) / kVicCols);
   if (p.refine) {
-    int gr = (int)((max_cells + kResThreads - 1) / kResThreads);
-    if (gr > 4096 * (kThreads / kResThreads)) gr = 4096 * (kThreads / kResThreads);
-    const size_t cw = (max_cols + kCorrCols - 1) / kCorrCols;  // warps
-    const int gc = (int)((cw + kCorrWarps - 1) / kCorrWarps);
-    vic_solve32_kernel<<<dim3(gs, p.nblock), 32, 0, stream>>>(tab, p);
-    if (p.refine < 0) {  // the FP32 solve: its Woodbury step, no corrections
-      const size_t threads = max_cols * 32;
-      const int gw = (int)((threads + kThreads - 1) / kThreads);
-      vic_woodbury32_kernel<<<dim3(gw, p.nblock), kThreads, 0, stream>>>(tab, p);
-    }
+    const unsigned gt = (unsigned)((max_cols + 31) / 32);  // tiles of columns
+    // (tile, layer) rows, a warp each (the kernel's loop takes what is left)
+    const size_t rows = (max_cells + 31) / 32;
+    int gr = (int)((rows + kThreads / 32 - 1) / (kThreads / 32));
+    if (gr > 8192) gr = 8192;
+    vic_factor32_kernel<<<dim3(gt, p.nblock), 32, 0, stream>>>(tab, p);
     for (int k = 1; k <= p.refine; ++k) {
-      vic_residual_kernel<<<dim3(gr, p.nblock), kResThreads, 0, stream>>>(tab, p, k);
-      vic_correct32_kernel<<<dim3(gc, p.nblock), 32 * kCorrWarps, 0, stream>>>(
-          tab, p, k == p.refine);
+      vic_residual_kernel<<<dim3(gr, p.nblock), kThreads, 0, stream>>>(tab, p, k);
+      vic_correct32_kernel<<<dim3(gt, p.nblock), 32, 0, stream>>>(tab, p, k);
     }
+    vic_accept_kernel<<<dim3(gt, p.nblock), kThreads, 0, stream>>>(tab, p);
     // the columns left to FP64: the partitioned FP64 solve first (a warp
     // per column, four chunks at once), the serial one for what it cannot
     vic_psolve_kernel<true><<<dim3((unsigned)max_cols, p.nblock), 32, 0, stream>>>(tab, p);

@@ -124,14 +124,11 @@ __host__ __device__ inline const double* base_r(const double* b, int nc1) { retu
 // a, b, c (25 each), the solution and the two Woodbury vectors (5 each)
 constexpr int kVicDoublesPerCell = 100;
 // implicit-precision float32 blocks add, after the FP64 part, a part for
-// the refined solve: per interior cell the blocks A, B, C in FP32 (28 each:
-// 25 and a pad), the factors of the FP32 sweep's pivot blocks (32), its C'
-// blocks (28) and the residuals of the three right-hand sides (16: 15 and
-// a pad); per
-// interior column the largest update of each right-hand side in the last
-// pass (3), the largest |x| of each after the first (3) and the direct-solve
-// mask (1 int: 0 accepted, 1 left to the FP64 solve, 2 left by the
-// partitioned FP64 solve to the serial one, 3 solved by the partitioned one)
+// the refined solve (vic_scratch32 lays it out in tiles of 32 columns): at
+// most 160 floats per interior cell, and per interior column 6 floats (the
+// last update, the largest |x|) and the direct-solve mask (1 int: 0 accepted,
+// 1 left to the FP64 solve, 2 left by the partitioned FP64 solve to the
+// serial one, 3 solved by the partitioned one)
 constexpr int kVicFloatsPerCell = 160;
 // the partitioned form of the scheme-9 solve: columns of fewer layers take
 // the serial solve; its region holds two 5x5 blocks per interior cell
