@@ -238,6 +238,7 @@ struct sg_handle {
   std::vector<double*> x1tabs;  // per-block geometry tables (gravity)
   bool has3 = false;            // a 3-D block: the x3 sweep runs
   bool visc3 = false;           // a 3-D block with viscosity: the prep runs
+  int x3_chunk = 1, x3_ctas = 1;  // the x3 sweep's schedule (plan_x3)
   size_t sum_icols = 0;         // implicit columns of all blocks
   int wide = 0;  // enough columns for a thread per column in the finish
   int wide_auto = 0;  // that rule's own answer (finish form 0)
@@ -303,6 +304,39 @@ int choose_tj(const sg_handle* h, const sg_block_desc& d, int nblock) {
     best = tj;
   }
   return best;
+}
+
+// The x3 sweep's chunk.  A thread walks its chunk's faces, one more than its
+// cells, after converting five cells (a quarter of a face's work), and a
+// sub-partition's FP64 pipe is full with one warp, so FP64 time goes as the
+// warps of the fullest sub-partition times a warp's faces; FP32 runs about
+// four warps side by side before that holds.  The chunk with the least of
+// that product is taken.  Measured per launch (us), chunks of 16 / 8 / 5 / 4
+// / 3 / 2: 45 x 37 x 48 FP64 308 / 167 / 114 / 177 / 143 / 168; 64^3 FP32
+// 31 / 20 / 17 / 16 / 24 / 22; four FP32 requests of about 0.8 M cells
+// 157 / 166 / 189 / 200 / 224 / 271 (the rule takes 5, 4 and 16)
+constexpr int kX3F32Warps = 4;
+void plan_x3(sg_handle* h) {
+  int sms = 152;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+  auto warps = [&](const sg_block_desc& d, int c) -> size_t {
+    if (d.nc3 <= 1) return 0;
+    const size_t nx1 = d.nc1 - 2 * d.ng, nx2 = d.nc2 > 1 ? d.nc2 - 2 * d.ng : 1;
+    const size_t lines = d.flux_cov && d.nc1 >= 3 ? ((nx1 + 2) * nx2 + 27) / 30
+                                                  : (nx1 * nx2 + 31) / 32;
+    return lines * ((d.nc3 - 2 * d.ng + c - 1) / c);
+  };
+  const size_t slots = (size_t)sms * 4 * (f64(h) ? 1 : kX3F32Warps);
+  double best = 1e300;
+  for (int c = 2; c <= 16; ++c) {
+    size_t w = 0;
+    for (const sg_block_desc& d : h->descs) w += warps(d, c);
+    const double cost = (double)((w + slots - 1) / slots) * (c + 1.25);
+    if (cost < best) best = cost, h->x3_chunk = c;
+  }
+  size_t w = 1;
+  for (const sg_block_desc& d : h->descs) w = std::max(w, warps(d, h->x3_chunk));
+  h->x3_ctas = (int)std::min<size_t>((w + 3) / 4, 8192);
 }
 
 int upload(sg_handle* h, cudaStream_t s) {
@@ -533,6 +567,8 @@ int sg_autotune(sg_handle* h, int32_t reps, int32_t* tj_out,
     p.psw = h->psw_on;
     p.fallbacks = h->fallbacks;
     p.max_nc1 = h->max_nc1;
+    p.x3_chunk = h->x3_chunk;
+    p.x3_ctas = h->x3_ctas;
     p.visc3 = h->visc3;
     p.vic_kinds = h->vic_kinds;
     p.ref32 = h->ref32;
@@ -887,6 +923,7 @@ int sg_create(const sg_scheme* scheme, const sg_block_desc* blocks,
     }
   }
   h->ntile = tile;
+  if (h->has3) plan_x3(h);
   {
     // a full warp of columns for every SM sub-partition
     int sms = 152;
@@ -1223,6 +1260,8 @@ int sg_stage(sg_handle* h, int32_t stage, const double* dt_dev,
   p.psw = h->psw_on;
   p.fallbacks = h->fallbacks;
   p.max_nc1 = h->max_nc1;
+  p.x3_chunk = h->x3_chunk;
+  p.x3_ctas = h->x3_ctas;
   p.visc3 = h->visc3;
   p.vic_kinds = h->vic_kinds;
   p.ref32 = h->ref32;

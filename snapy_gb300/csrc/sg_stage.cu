@@ -1752,7 +1752,7 @@ __global__ void __launch_bounds__(kThreads)
 
 // the x3 faces of 3-D blocks (CoordinateImpl::divergence's x3 term,
 // src/coord/coordinate.cpp:650-656): one thread per (x1 cell, x2 row, chunk
-// of kX3Chunk x3 cells) walks the chunk's faces with a sliding window of six
+// of p.x3_chunk x3 cells) walks the chunk's faces with a sliding window of six
 // primitives in registers, solves each face once and stores a3 (F3[k+1] -
 // F3[k]) of each cell, which the stage kernel adds to its divergence after
 // the x1 and x2 differences, the reference's order.  With a hydrostatic base the
@@ -1760,7 +1760,14 @@ __global__ void __launch_bounds__(kThreads)
 // covariance row (src/hydro/hydro_forward.cpp:58-231 with dim 3, added to
 // the face flux before the walls, :800-826) is added to the energy row; a
 // reflecting x3 wall zeroes the mass and energy rows of its face.
-constexpr int kX3Chunk = 16;
+//
+// Bound by the FP64 pipe in FP64 (a warp instruction per 64 cycles and
+// sub-partition) and by latency in FP32, so the chunk is sized to fill every
+// sub-partition once (plan_x3) and a CTA is four warps, one for each.  With
+// chunks of 16 cells in CTAs of eight warps and a warp per 30 rows of one x2
+// line, 45 x 37 x 48 cells were 34 CTAs: 781 us per launch, now 114 us; FP32
+// 64^3 61 and 16 us, four served requests of 0.8 M cells 198 and 157 us.
+constexpr int kX3Threads = 128;
 
 // 3-D viscosity's prep (DiffusionImpl::cartesian_fluxes, src/forcing/
 // diffusion.cpp:553-683): on the interior extended by one cell in each
@@ -1815,7 +1822,7 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 template <int RK, bool SHOCK>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kX3Threads)
     x3_kernel(const BlockDev* __restrict__ tab, StageParams p) {
   const BlockDev& B = tab[blockIdx.y];
   if (B.nc3 == 1) return;
@@ -1823,7 +1830,8 @@ __global__ void __launch_bounds__(kThreads)
   const int nx1 = nc1 - 2 * ng, nx2 = nc2 > 1 ? nc2 - 2 * ng : 1,
             nx3 = nc3 - 2 * ng;
   const int o2 = nc2 > 1 ? ng : 0;
-  const int nch = (nx3 + kX3Chunk - 1) / kX3Chunk;
+  const int chunk = p.x3_chunk;
+  const int nch = (nx3 + chunk - 1) / chunk;
   const size_t plane = (size_t)nc1 * nc2 * nc3, kst = (size_t)nc1 * nc2;
   const real* __restrict__ uin = static_cast<const real*>(B.buf[p.in]);
   const real gammad = real(B.gammad);
@@ -1834,15 +1842,16 @@ __global__ void __launch_bounds__(kThreads)
   const bool wlo = B.bc[4] == kBcReflecting, whi = B.bc[5] == kBcReflecting;
   // the covariance row of the x3 faces (_flux_covariance, dim 3) needs each
   // face's mean state on the x1 rows either side: a warp then covers 32
-  // consecutive x1 rows of one (x2, chunk) line -- 30 it owns and a row
-  // either side (an x1 ghost row at the column's ends) -- and trades the
-  // face means by shuffles; every lane of a warp runs the same faces
+  // consecutive entries of the chunk's plane of columns, x1 rows with one
+  // ghost row at either end, x2 after x2 -- 30 it owns and one either side,
+  // which are always an owned row's neighbours -- and trades the face means
+  // by shuffles; every lane of a warp runs the same faces
   const bool cov = B.flux_cov && nc1 >= 3;
   const bool visc = B.nu_iso > 0.;
   const size_t vplane = plane;  // one visc3 plane
-  const int nw = (nx1 + 29) / 30;  // warps per (x2, chunk) line
-  const size_t total = cov ? (size_t)32 * nw * nx2 * nch
-                           : (size_t)nx1 * nx2 * nch;
+  const int ext = nx1 + 2, flat = ext * nx2;  // a plane's entries
+  const int nw = (flat - 2 + 29) / 30;        // warps per chunk
+  const size_t total = cov ? (size_t)32 * nw * nch : (size_t)nx1 * nx2 * nch;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
        e += (size_t)gridDim.x * blockDim.x) {
     int i, j, ch;
@@ -1850,18 +1859,20 @@ __global__ void __launch_bounds__(kThreads)
     if (cov) {
       const int lane = (int)(e & 31);
       const size_t wdx = e >> 5;
-      const int row = ng - 1 + 30 * (int)(wdx % nw) + lane;
-      j = o2 + (int)((wdx / nw) % nx2);
-      ch = (int)(wdx / ((size_t)nw * nx2));
-      own = lane >= 1 && lane <= 30 && row < ng + nx1;
-      i = row < ng + nx1 ? row : ng + nx1;  // past the top ghost row: a copy
+      const int at = 30 * (int)(wdx % nw) + lane;
+      const int q = at < flat ? at : flat - 1;  // past the plane: a copy
+      const int r = q % ext;
+      j = o2 + q / ext;
+      ch = (int)(wdx / nw);
+      own = lane >= 1 && lane <= 30 && at < flat && r >= 1 && r <= nx1;
+      i = ng - 1 + r;
     } else {
       i = ng + (int)(e % nx1);
       j = o2 + (int)((e / nx1) % nx2);
       ch = (int)(e / ((size_t)nx1 * nx2));
     }
-    const int k0 = ng + ch * kX3Chunk;
-    const int k1 = min(k0 + kX3Chunk, ng + nx3);  // cells k0..k1-1
+    const int k0 = ng + ch * chunk;
+    const int k1 = min(k0 + chunk, ng + nx3);  // cells k0..k1-1
     const size_t col = (size_t)j * nc1 + i;
     const real pb = pbc ? real(pbc[i]) : real(0);
     auto load = [&](int k, real* w) {
@@ -2435,11 +2446,7 @@ extern "C" int SG_NAME(sg_launch_x3)(const BlockDev* tab, StageParams p,
     if (gv > 2048) gv = 2048;
     visc3_kernel<<<dim3(gv, p.nblock), kThreads, 0, stream>>>(tab, p);
   }
-  // threads: cells / kX3Chunk per block (bounded by a few waves)
-  size_t work = max_cells / kX3Chunk + 1;
-  int gx = (int)((work + kThreads - 1) / kThreads);
-  if (gx > 2048) gx = 2048;
-  k<<<dim3(gx, p.nblock), kThreads, 0, stream>>>(tab, p);
+  k<<<dim3(p.x3_ctas, p.nblock), kX3Threads, 0, stream>>>(tab, p);
   return (int)cudaGetLastError();
 }
 

@@ -168,6 +168,8 @@ struct StageParams {
                         // staging wait ran out)
   int32_t smem_rows;    // x1 lines held in shared memory per tile
   int32_t max_nc1;
+  int32_t x3_chunk;     // x3 cells a thread of the x3 sweep walks
+  int32_t x3_ctas;      // its CTAs per block
   int32_t visc3;        // some 3-D block has viscosity: visc3_kernel runs
   int32_t asm_kinds;    // implicit blocks: bit 0 some assemble in FP64,
                         // bit 1 some in FP32 (one kernel each)
