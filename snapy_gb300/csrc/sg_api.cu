@@ -239,6 +239,7 @@ struct sg_handle {
   bool has3 = false;            // a 3-D block: the x3 sweep runs
   bool visc3 = false;           // a 3-D block with viscosity: the prep runs
   int x3_chunk = 1, x3_ctas = 1;  // the x3 sweep's schedule (plan_x3)
+  int line_seg = 0, line_ctas = 0;  // line_kernel's (plan_line)
   size_t sum_icols = 0;         // implicit columns of all blocks
   int wide = 0;  // enough columns for a thread per column in the finish
   int wide_auto = 0;  // that rule's own answer (finish form 0)
@@ -339,6 +340,26 @@ void plan_x3(sg_handle* h) {
   h->x3_ctas = (int)std::min<size_t>((w + 3) / 4, 8192);
 }
 
+// The cells a CTA of line_kernel takes: the fewest of 8 to 64 that leave no
+// more CTAs than SMs.  A segment costs its CTA one face's work per thread
+// until the threads are full (12 cells), and each its own halo of six cells
+void plan_line(sg_handle* h) {
+  int sms = 152;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+  auto ctas = [&](int b, int seg) {
+    const BlockDev& B = h->host[b];
+    return B.line ? (B.nc1 - 2 * B.ng + seg - 1) / seg : 0;
+  };
+  for (h->line_seg = 8; h->line_seg < sg::kLineMaxSeg; h->line_seg *= 2) {
+    long n = 0;
+    for (int b = 0; b < h->nblock; ++b) n += ctas(b, h->line_seg);
+    if (n <= sms) break;
+  }
+  h->line_ctas = 0;
+  for (int b = 0; b < h->nblock; ++b)
+    h->line_ctas = std::max(h->line_ctas, ctas(b, h->line_seg));
+}
+
 int upload(sg_handle* h, cudaStream_t s) {
   if (!h->dirty) return 0;
   for (int b = 0; b < h->nblock; ++b) {
@@ -390,7 +411,7 @@ int relayout(sg_handle* h, const int32_t* tj) {
       return fail(SG_ERR_UNSUPPORTED, "block %d: a tile needs %zu B of "
                   "shared memory (limit %d)", b, sm, optin);
     B.tj = t;
-    B.ntile = nx3 * ((nx2 + t - 1) / t);
+    B.ntile = B.line ? 0 : nx3 * ((nx2 + t - 1) / t);
     B.tile0 = tile;
     tile += B.ntile;
     smem = std::max(smem, sm);
@@ -567,6 +588,8 @@ int sg_autotune(sg_handle* h, int32_t reps, int32_t* tj_out,
     p.psw = h->psw_on;
     p.fallbacks = h->fallbacks;
     p.max_nc1 = h->max_nc1;
+    p.line_seg = h->line_seg;
+    p.line_ctas = h->line_ctas;
     p.x3_chunk = h->x3_chunk;
     p.x3_ctas = h->x3_ctas;
     p.visc3 = h->visc3;
@@ -872,7 +895,10 @@ int sg_create(const sg_scheme* scheme, const sg_block_desc* blocks,
     int nx2 = d.nc2 > 1 ? d.nc2 - 2 * d.ng : 1;
     int nx3 = d.nc3 > 1 ? d.nc3 - 2 * d.ng : 1;
     // tiles: tj-wide x2 strips of every interior x3 plane
-    B.ntile = nx3 * ((nx2 + B.tj - 1) / B.tj);
+    // (none where line_kernel takes the block)
+    B.line = d.nc2 == 1 && d.nc3 == 1 && d.grav1 == 0. && !(d.nu_iso > 0.) &&
+             !d.implicit_scheme;
+    B.ntile = B.line ? 0 : nx3 * ((nx2 + B.tj - 1) / B.tj);
     if (d.nc3 > 1) h->has3 = true;
     B.tile0 = tile;
     tile += B.ntile;
@@ -924,6 +950,7 @@ int sg_create(const sg_scheme* scheme, const sg_block_desc* blocks,
   }
   h->ntile = tile;
   if (h->has3) plan_x3(h);
+  plan_line(h);
   {
     // a full warp of columns for every SM sub-partition
     int sms = 152;
@@ -1260,6 +1287,8 @@ int sg_stage(sg_handle* h, int32_t stage, const double* dt_dev,
   p.psw = h->psw_on;
   p.fallbacks = h->fallbacks;
   p.max_nc1 = h->max_nc1;
+  p.line_seg = h->line_seg;
+  p.line_ctas = h->line_ctas;
   p.x3_chunk = h->x3_chunk;
   p.x3_ctas = h->x3_ctas;
   p.visc3 = h->visc3;
@@ -1293,7 +1322,9 @@ int sg_stage(sg_handle* h, int32_t stage, const double* dt_dev,
         h->counts, 0, sizeof(unsigned long long) * sg::kCountSlots * h->nblock, s);
     if (ze != cudaSuccess) return cuda_fail(ze, "sg_stage: monitor counts");
   }
-  int launches = h->ref32 ? 3 : 2;  // (with the base reference's refresh)
+  // the ghosts, the tiles' and the lines' stage, the base reference's refresh
+  int launches = 1 + (h->ntile > 0 ? 1 : 0) + (h->line_ctas > 0 ? 1 : 0) +
+                 (h->ref32 ? 1 : 0);
   if (h->has3) {
     // the x3 faces of the 3-D blocks: their flux differences, which the
     // stage kernel adds to its divergence after x1 and x2

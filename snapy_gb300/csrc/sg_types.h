@@ -28,6 +28,7 @@ struct BlockDev {
   int32_t tj;           // x2 columns per tile
   int32_t ntile;        // tiles of this block
   int32_t tile0;        // first tile index of this block in the batch
+  int32_t line;         // a 1-D block without sources: line_kernel takes it
   int32_t bc[6];        // BcKind per face: x1 in/out, x2 in/out, x3 in/out
   double dx1, dx2, dx3;
   double gammad;
@@ -136,6 +137,9 @@ constexpr int kPswMinLayers = 16;
 constexpr int kPswDoublesPerCell = 50;
 constexpr int kVicFloatsPerColumn = 7;
 
+// the most x1 cells of a line_kernel CTA (its shared memory is sized by it)
+constexpr int kLineMaxSeg = 64;
+
 // the monitor's counts of a step, per block (the RegisterMonitor counters
 // src/hydro/hydro.cpp:175-192 that this path can raise): HLLC faces whose
 // contact pressure was clamped to zero, and columns the implicit solve
@@ -168,6 +172,8 @@ struct StageParams {
                         // staging wait ran out)
   int32_t smem_rows;    // x1 lines held in shared memory per tile
   int32_t max_nc1;
+  int32_t line_seg;     // x1 cells a CTA of line_kernel takes
+  int32_t line_ctas;    // its CTAs per block (0: no such block)
   int32_t x3_chunk;     // x3 cells a thread of the x3 sweep walks
   int32_t x3_ctas;      // its CTAs per block
   int32_t visc3;        // some 3-D block has viscosity: visc3_kernel runs
