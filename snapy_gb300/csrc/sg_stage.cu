@@ -2646,16 +2646,32 @@ extern "C" int SG_NAME(sg_launch_vic)(const BlockDev* tab, StageParams p,
   int gs = (int)((max_cols + kVicCols - 1) / kVicCols);
   if (p.refine) {
     const unsigned gt = (unsigned)((max_cols + 31) / 32);  // tiles of columns
-    // (tile, layer) rows, a warp each (the kernel's loop takes what is left)
-    const size_t rows = (max_cells + 31) / 32;
-    int gr = (int)((rows + kThreads / 32 - 1) / (kThreads / 32));
-    if (gr > 8192) gr = 8192;
-    vic_factor32_kernel<<<dim3(gt, p.nblock), 32, 0, stream>>>(tab, p);
-    for (int k = 1; k <= p.refine; ++k) {
-      vic_residual_kernel<<<dim3(gr, p.nblock), kThreads, 0, stream>>>(tab, p, k);
-      vic_correct32_kernel<<<dim3(gt, p.nblock), 32, 0, stream>>>(tab, p, k);
+    const int lg = (p.max_nc1 - 6 + 7) / 8;  // CTAs of eight layers a tile
+    // the rings' opt-in shared memory, once a device (a handle's first launch
+    // is eager)
+    static bool granted[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 64 || !granted[dev]) {
+      cudaError_t g = cudaFuncSetAttribute(
+          vic_factor32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+          kFacFloats * (int)sizeof(float));
+      if (g == cudaSuccess)
+        g = cudaFuncSetAttribute(vic_correct32_kernel,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kCorFloats * (int)sizeof(float));
+      if (g != cudaSuccess) return (int)g;
+      if (dev < 64) granted[dev] = true;
     }
-    vic_accept_kernel<<<dim3(gt, p.nblock), kThreads, 0, stream>>>(tab, p);
+    vic_factor32_kernel<<<dim3(gt, p.nblock), 64, kFacFloats * sizeof(float),
+                          stream>>>(tab, p);
+    for (int k = 1; k <= p.refine; ++k) {
+      vic_residual_kernel<<<dim3(gt * lg, p.nblock), kThreads, 0, stream>>>(
+          tab, p, k, lg);
+      vic_correct32_kernel<<<dim3(gt, p.nblock), 64, kCorFloats * sizeof(float),
+                             stream>>>(tab, p, k);
+    }
+    vic_sum_kernel<<<dim3(gt * lg, p.nblock), kThreads, 0, stream>>>(tab, p, lg);
     // the columns left to FP64: the partitioned FP64 solve first (a warp
     // per column, four chunks at once), the serial one for what it cannot
     vic_psolve_kernel<true><<<dim3((unsigned)max_cols, p.nblock), 32, 0, stream>>>(tab, p);

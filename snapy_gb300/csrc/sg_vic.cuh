@@ -78,15 +78,14 @@ struct VicTile {
 // (after the FP64 part, 16-byte aligned), in tiles: the blocks A, B, C, the
 // pivot blocks' inverses PI, C' (25 values a cell each), the residuals, then
 // the sweep's y (R, 5) and the first solution X0 (5), at most 156 of the 160
-// floats a cell; then, per column, the largest update of the last pass
-// (stat 0), the largest |x| of the first (stat 3) and the direct-solve mask.
-// The Woodbury vectors, the corrections and each pass's two Woodbury weights
-// a column (Z0, Z1, DK, AL: at most 48 of the 50 floats a cell) take the FP64
-// part's C slots and the FP64 residual (r64, 5 doubles a cell, w to a row, no
-// padding) its B slots, which a refined block uses only for the columns it
-// leaves to the FP64 solve, afterwards
+// floats a cell; then, per column, each pass's largest |d| (stat, 6) and the
+// direct-solve mask.  The corrections and the wall rows' third-point vectors
+// (DK, at most 3 x 8 floats a cell, and E, 10 a column) take
+// the FP64 part's C slots and the FP64 residual (r64, 5 doubles a cell, w to
+// a row, no padding) its B slots, which a refined block uses only for the
+// columns it leaves to the FP64 solve, afterwards
 struct VicScratch32 {
-  float *A, *B, *C, *PI, *CP, *R, *X0, *Z0, *Z1, *DK, *AL, *stat;
+  float *A, *B, *C, *PI, *CP, *R, *X0, *DK, *E, *stat;
   size_t dk;  // the values of one correction's array: correction k at DK + k dk
   double* r64;
   int* mask;
@@ -110,11 +109,9 @@ __device__ __forceinline__ VicScratch32 vic_scratch32(const BlockDev& B,
   t.R = f + 5 * t25;
   t.X0 = t.R + t5;
   float* d = reinterpret_cast<float*>(S.C);
-  t.Z0 = d;
-  t.Z1 = d + t5;
-  t.DK = d + 2 * t5;
+  t.DK = d;
   t.dk = t5;
-  t.AL = d + 5 * t5;
+  t.E = d + 3 * t5;
   t.r64 = S.B;
   t.stat = f + kVicFloatsPerCell * c;
   t.mask = reinterpret_cast<int*>(t.stat + 6 * t.ncol);
