@@ -204,15 +204,15 @@ int sg_kernel_times(sg_handle* h, double* ms, int64_t* launches);
  * this handle's own blocks and current state: every tile width of
  * 1, 2, 3, 4, 6, 8, 12, 16, 24, 32 x2 columns (the same request for every block, each
  * clamped to its x2 extent and halved until its tile fits the shared
- * memory), then, with an implicit solve, its finish as a warp per column
- * and as a thread per column, and keeps the fastest.  The results do not
+ * memory), then, with an implicit solve, its finish with the library's
+ * columns a CTA and with twice as many, and keeps the fastest.  The results do not
  * depend on either choice (same operations, same order).  The trial
  * launches read the current state and write only the rotation's free
  * buffer and the solve's scratch; the step fields and the status bits are
  * left as they were.  Not inside a stream capture; graphs captured before
  * must be captured again.  Outputs (each may be null): tj_out[nblock] the
- * tile widths, *finish_out the finish form (1 warp, 2 thread; 0 when there
- * is no solve), ms_out[2] the best stage and solve milliseconds per launch.
+ * tile widths, *finish_out the finish form (1 the rule's columns a CTA, 2
+ * twice as many; 0 when there is no solve), ms_out[2] the best stage and solve milliseconds per launch.
  * sg_set_schedule applies a stored choice (tj null or 0: the library's
  * rule; finish 0: the library's rule). */
 /* The implicit solve of integration/implicit-precision float32 blocks.  By

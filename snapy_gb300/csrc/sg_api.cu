@@ -32,7 +32,7 @@ using sg::StageParams;
                                      double* const*, size_t,                   \
                                      cudaStream_t);                            \
   extern "C" int sg_launch_vic##sfx(const BlockDev*, StageParams, size_t,     \
-                                    size_t, int, int*, cudaStream_t,           \
+                                    size_t, int*, cudaStream_t,                \
                                     cudaEvent_t*);                             \
   extern "C" int sg_launch_x3##sfx(const BlockDev*, StageParams, size_t,      \
                                    cudaStream_t);                              \
@@ -240,9 +240,7 @@ struct sg_handle {
   bool visc3 = false;           // a 3-D block with viscosity: the prep runs
   int x3_chunk = 1, x3_ctas = 1;  // the x3 sweep's schedule (plan_x3)
   int line_seg = 0, line_ctas = 0;  // line_kernel's (plan_line)
-  size_t sum_icols = 0;         // implicit columns of all blocks
-  int wide = 0;  // enough columns for a thread per column in the finish
-  int wide_auto = 0;  // that rule's own answer (finish form 0)
+  int fin_len = 0, fin_ctas = 0;  // the finish's schedule (plan_finish)
   bool implicit = false;
   int vic_kinds = 0;  // bit 0: a block with the full 5x5 matrix, bit 1: 3x3
   bool ref32 = false;  // an FP32 block under gravity: base_ref_kernel runs
@@ -260,7 +258,8 @@ struct sg_handle {
   int any_f32 = 0;  // a block assembles its implicit blocks in FP32
   size_t max_icells = 0, max_icols = 0;
   std::vector<sg_block_desc> descs;   // as created (tile re-layout)
-  int32_t finish = 0;  // implicit finish form: 0 auto, 1 warp, 2 thread
+  int32_t finish = 0;  // implicit finish form: 0 and 1 the rule's columns a
+                       // CTA, 2 twice as many
   std::vector<size_t> scratch_bytes;  // per block: vic_bytes + the x3 part
   std::vector<size_t> vic_bytes;
   std::vector<size_t> dv3_bytes;  // per block: the x3 part of the scratch
@@ -338,6 +337,43 @@ void plan_x3(sg_handle* h) {
   size_t w = 1;
   for (const sg_block_desc& d : h->descs) w = std::max(w, warps(d, h->x3_chunk));
   h->x3_ctas = (int)std::min<size_t>((w + 3) / 4, 8192);
+}
+
+// The columns a CTA of the implicit solve's finish takes (as the length of
+// its shared arrays): the fewest that leave at most two CTAs an SM, up to
+// kFinLen; form 2 takes twice as many.  The serial passes cost a CTA the same
+// for one column or 32, and with one CTA's worth of warps on an SM nothing
+// hides them.  Measured per launch (us) with 1 / 2 / 4 / 8 / 16 / 32 columns:
+// 512 columns of 128, FP64: 73 / 44 / 45 / 61 / 91 / -; 301 of 75: 26 / 25 /
+// 32 / 40 / 56 / 94; 1,665 of 48: 106 / 58 / 49 / 37 / 39 / 63; 4,096 of 64,
+// FP32: 313 / 168 / 113 / 84 / 67 / 90.  kFinLen of 516 / 1032 / 1376 / 2064
+// / 4128: 64-member ensemble 525 / 399 / 311 / 346 / 515, four served requests
+// 1155 / 864 / 667 / 736 / 1122 (larger ones leave an SM two CTAs or one)
+void plan_finish(sg_handle* h) {
+  int sms = 152;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+  size_t ctas = 0, most = 0;
+  auto count = [&](int len) {
+    ctas = most = 0;
+    for (int b = 0; b < h->nblock; ++b) {
+      const BlockDev& B = h->host[b];
+      if (!B.implicit) continue;
+      const size_t c = sg::fin_cols(B.nc1 - 2 * B.ng, len);
+      const size_t n = ((size_t)(B.nc2 > 1 ? B.nc2 - 2 * B.ng : 1) *
+                            (B.nc3 > 1 ? B.nc3 - 2 * B.ng : 1) + c - 1) / c;
+      ctas += n;
+      most = std::max(most, n);
+    }
+  };
+  const int one = sg::fin_pitch(h->max_nc1 - 6);
+  const int top = std::max(one, sg::kFinLen);
+  int len = one;
+  for (count(len); ctas > 2 * (size_t)sms && len < top; count(len))
+    len = std::min(len + len / 8 + 1, top);
+  if (h->finish == 2) len = std::min(2 * len, top);
+  count(len);
+  h->fin_len = len;
+  h->fin_ctas = (int)most;
 }
 
 // The cells a CTA of line_kernel takes: the fewest of 8 to 64 that leave no
@@ -525,7 +561,7 @@ int sg_set_schedule(sg_handle* h, const int32_t* tj, int32_t finish) {
   int rc = relayout(h, tj);
   if (rc) return rc;
   h->finish = finish;
-  h->wide = finish == 0 ? h->wide_auto : (finish == 2 ? 1 : 0);
+  plan_finish(h);
   return 0;
 }
 
@@ -588,6 +624,8 @@ int sg_autotune(sg_handle* h, int32_t reps, int32_t* tj_out,
     p.psw = h->psw_on;
     p.fallbacks = h->fallbacks;
     p.max_nc1 = h->max_nc1;
+    p.fin_len = h->fin_len;
+    p.fin_ctas = h->fin_ctas;
     p.line_seg = h->line_seg;
     p.line_ctas = h->line_ctas;
     p.x3_chunk = h->x3_chunk;
@@ -609,9 +647,9 @@ int sg_autotune(sg_handle* h, int32_t reps, int32_t* tj_out,
     };
     auto vic = [&]() -> int {
       int r = f64(h) ? sg_launch_vic_f64(h->dev, p, h->max_icells, h->max_icols,
-                                         h->wide, h->status, s, nullptr)
+                                         h->status, s, nullptr)
                      : sg_launch_vic_f32(h->dev, p, h->max_icells, h->max_icols,
-                                         h->wide, h->status, s, nullptr);
+                                         h->status, s, nullptr);
       return r ? cuda_fail((cudaError_t)r, "sg_autotune: trial solve") : 0;
     };
     auto timed = [&](auto&& launch, double* ms) -> int {
@@ -652,8 +690,8 @@ int sg_autotune(sg_handle* h, int32_t reps, int32_t* tj_out,
     }
     if (!rc) rc = relayout(h, best_tj.data());
     if (!rc) rc = upload(h, s);
-    // (2) the implicit solve's finish: a warp per column or a thread per
-    // column (the stage's explicit tendency is in the scratch first), and
+    // (2) the implicit solve's finish: the rule's columns a CTA or twice as
+    // many (the stage's explicit tendency is in the scratch first), and
     // with sg_set_sweep mode 2 its solve serial or partitioned
     if (!rc && h->implicit) {
       rc = stage();
@@ -669,7 +707,10 @@ int sg_autotune(sg_handle* h, int32_t reps, int32_t* tj_out,
         }
         for (int form : {1, 2}) {
           if (rc) break;
-          h->wide = form == 2;
+          h->finish = form;
+          plan_finish(h);
+          p.fin_len = h->fin_len;
+          p.fin_ctas = h->fin_ctas;
           double ms = 0.;
           rc = timed(vic, &ms);
           if (!rc && ms < best) {
@@ -681,7 +722,7 @@ int sg_autotune(sg_handle* h, int32_t reps, int32_t* tj_out,
         }
       }
       h->finish = best_finish;
-      h->wide = best_finish == 2;
+      plan_finish(h);
       if (both) {
         psw_apply(h, best_sweep);
         if (!rc) rc = upload(h, s);
@@ -945,19 +986,12 @@ int sg_create(const sg_scheme* scheme, const sg_block_desc* blocks,
     if (d.implicit_scheme) {
       h->max_icells = std::max(h->max_icells, icells);
       h->max_icols = std::max(h->max_icols, icols);
-      h->sum_icols += icols;
     }
   }
   h->ntile = tile;
   if (h->has3) plan_x3(h);
   plan_line(h);
-  {
-    // a full warp of columns for every SM sub-partition
-    int sms = 152;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
-    h->wide_auto = h->sum_icols >= (size_t)32 * 4 * sms;
-    h->wide = h->wide_auto;
-  }
+  if (h->implicit) plan_finish(h);
   cudaError_t e = cudaMalloc(&h->dev, sizeof(BlockDev) * nblock);
   if (e == cudaSuccess)
     e = cudaMalloc(&h->red, sizeof(unsigned long long) * 4 * nblock);
@@ -1287,6 +1321,8 @@ int sg_stage(sg_handle* h, int32_t stage, const double* dt_dev,
   p.psw = h->psw_on;
   p.fallbacks = h->fallbacks;
   p.max_nc1 = h->max_nc1;
+  p.fin_len = h->fin_len;
+  p.fin_ctas = h->fin_ctas;
   p.line_seg = h->line_seg;
   p.line_ctas = h->line_ctas;
   p.x3_chunk = h->x3_chunk;
@@ -1340,18 +1376,17 @@ int sg_stage(sg_handle* h, int32_t stage, const double* dt_dev,
   if (timed) cudaEventRecord(ev[1], s);
   if (h->implicit) {
     rc = f64(h) ? sg_launch_vic_f64(h->dev, p, h->max_icells, h->max_icols,
-                                    h->wide, h->status, s,
+                                    h->status, s,
                                     timed ? ev + 2 : nullptr)
                 : sg_launch_vic_f32(h->dev, p, h->max_icells, h->max_icols,
-                                    h->wide, h->status, s,
+                                    h->status, s,
                                     timed ? ev + 2 : nullptr);
     if (rc) return cuda_fail((cudaError_t)rc, "sg_stage: implicit solve");
     if (timed) cudaEventRecord(ev[4], s);
     // assembly, solve, finish; the refined solve adds its FP32 sweep, a
     // residual and a sweep per correction, the acceptance and the left-over
     // columns' solve
-    // (a wide batch's finish is three launches)
-    launches += 3 + (h->wide ? 2 : 0) + (h->vic_kinds == 3 ? 1 : 0) +
+    launches += 3 + (h->vic_kinds == 3 ? 1 : 0) +
                 (h->asm_kinds == 3 ? 1 : 0) +
                 (h->refine ? 3 + 2 * std::max(h->refine, 0) : 0) +
                 (h->psw_on ? 1 : 0);

@@ -2627,7 +2627,7 @@ extern "C" int SG_NAME(sg_launch_init)(const BlockDev* tab, int nblock,
 // explicit tendency of the implicit blocks)
 extern "C" int SG_NAME(sg_launch_vic)(const BlockDev* tab, StageParams p,
                                       size_t max_cells, size_t max_cols,
-                                      int wide, int* status,
+                                      int* status,
                                       cudaStream_t stream, cudaEvent_t* ev) {
   int ga = (int)((max_cells + kThreads - 1) / kThreads);
   if (ga > 4096) ga = 4096;
@@ -2700,18 +2700,18 @@ extern "C" int SG_NAME(sg_launch_vic)(const BlockDev* tab, StageParams p,
   e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   if (ev) cudaEventRecord(ev[1], stream);
-  if (wide) {
-    // three passes: per cell, the serial scans per column, per cell
-    int gt = (int)((max_cols + kFinishBThreads - 1) / kFinishBThreads);
-    int gc = (int)((max_cells + kThreads - 1) / kThreads);
-    if (gc > 8192) gc = 8192;
-    vic_finish_a_kernel<<<dim3(gc, p.nblock), kThreads, 0, stream>>>(tab, p);
-    vic_finish_b_kernel<<<dim3(gt, p.nblock), kFinishBThreads, 0, stream>>>(tab, p);
-    vic_finish_c_kernel<<<dim3(gc, p.nblock), kThreads, 0, stream>>>(tab, p);
-  } else {
-    int gc = (int)((max_cols + kVicWarps - 1) / kVicWarps);
-    vic_finish_kernel<32><<<dim3(gc, p.nblock), 32 * kVicWarps, 0, stream>>>(tab, p);
+  const size_t fin = (size_t)p.fin_len * sizeof(double) *
+                     (kFinArrays + ((p.vic_kinds & 2) ? kFinPartial : 0));
+  static size_t fin_granted[64] = {};
+  int fin_dev = 0;
+  cudaGetDevice(&fin_dev);
+  if (fin_dev >= 64 || fin > fin_granted[fin_dev]) {
+    e = cudaFuncSetAttribute(vic_finish_kernel,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fin);
+    if (e != cudaSuccess) return (int)e;
+    if (fin_dev < 64) fin_granted[fin_dev] = fin;
   }
+  vic_finish_kernel<<<dim3(p.fin_ctas, p.nblock), kFinThreads, fin, stream>>>(tab, p);
   return (int)cudaGetLastError();
 }
 

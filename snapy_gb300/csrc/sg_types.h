@@ -140,6 +140,17 @@ constexpr int kVicFloatsPerColumn = 7;
 // the most x1 cells of a line_kernel CTA (its shared memory is sized by it)
 constexpr int kLineMaxSeg = 64;
 
+// the implicit solve's finish keeps kFinArrays arrays of `len` doubles a CTA
+// (kFinPartial more for the partial matrix): a column's pitch in them (n + 1
+// values, odd), and the columns that fit (sg_create gives len at least one)
+constexpr int kFinArrays = 5, kFinPartial = 2;
+constexpr int kFinLen = 1376;  // the largest len of a CTA of several columns
+__host__ __device__ inline int fin_pitch(int n) { return (n + 1) | 1; }
+__host__ __device__ inline int fin_cols(int n, int len) {
+  const int c = len / fin_pitch(n);
+  return c < 32 ? c : 32;
+}
+
 // the monitor's counts of a step, per block (the RegisterMonitor counters
 // src/hydro/hydro.cpp:175-192 that this path can raise): HLLC faces whose
 // contact pressure was clamped to zero, and columns the implicit solve
@@ -172,6 +183,8 @@ struct StageParams {
                         // staging wait ran out)
   int32_t smem_rows;    // x1 lines held in shared memory per tile
   int32_t max_nc1;
+  int32_t fin_len;      // doubles of a finish CTA's array
+  int32_t fin_ctas;     // its CTAs per block
   int32_t line_seg;     // x1 cells a CTA of line_kernel takes
   int32_t line_ctas;    // its CTAs per block (0: no such block)
   int32_t x3_chunk;     // x3 cells a thread of the x3 sweep walks

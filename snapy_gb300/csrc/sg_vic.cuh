@@ -21,9 +21,8 @@
 // column: the 5x5 block products run one entry per lane through warp
 // shuffles, the 8 right-hand sides of the LU back-solve one per lane, the
 // factorisation on the warp's shared-memory tile), and the column's
-// redistribution, remainder and RK combine (vic_finish_kernel, one warp per
-// column, or one thread per column when the batch has columns enough to
-// fill every SM sub-partition).  Every product is summed in index order, so the results are bit
+// redistribution, remainder and RK combine (vic_finish_kernel, a CTA per few
+// columns).  Every product is summed in index order, so the results are bit
 // for bit the CPU oracle's.
 #pragma once
 
@@ -631,15 +630,6 @@ __device__ __forceinline__ double vshfl(double v, int src) {
 __device__ __forceinline__ unsigned long long vbits(double x) {
   return static_cast<unsigned long long>(__double_as_longlong(x));
 }
-
-// a column's work array in the finish: element i at p[i s]
-struct VCol {
-  double* p;
-  size_t s;
-  __device__ __forceinline__ double& operator[](int i) const {
-    return p[(size_t)i * s];
-  }
-};
 
 // finite, tested on the exponent bits (integer pipes, not the FP64 one)
 __device__ __forceinline__ bool vfinite(double x) {
@@ -1285,194 +1275,178 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-constexpr int kVicWarps = 4;  // columns per CTA of the finish (a warp each)
+// (3) redistribution, the gravity-work remainder and the RK combine, a CTA
+// per fin_cols columns with the columns' work in shared memory.  What a cell
+// needs of its own runs a thread per cell; the constituent column's serial
+// passes (the sums R and S, the face-mass prefix M with the availability
+// clamp) run a lane per column and keep only their chain: three additions
+// and two comparisons a layer, the comparisons on the bit patterns, so the
+// FP64 pipe (a warp instruction per 64 cycles) sees the additions alone.
+//
+// Bound by the FP64 pipe: about 55 instructions a cell, and 4 a layer for
+// the passes of a CTA's columns.  Measured per launch (us), before (a warp
+// per column, its passes on lane 0; wide batches three launches, a thread per
+// column for the passes) and now: 512 columns of 128 FP64 138 and 45, 301 of
+// 75 85 and 25, 384 of 100 FP32 106 and 35, 4,096 of 64 113 and 65, nine FP64
+// members 153 and 59, 64 members 477 and 313, four served requests 829 and
+// 670.
+constexpr int kFinThreads = 256;
 
-// (3) redistribution, the gravity-work remainder and the RK combine of each
-// column, one warp per column: the serial passes of the constituent column
-// (sums, face-mass prefix, availability clamp) on lane 0, the per-layer maps
-// on every lane
-template <int NL>
-__device__ __forceinline__ void vsync() {
-  if (NL > 1) __syncwarp();
+// a > b and a < 0 from the bit patterns: the order of the doubles, without
+// the FP64 pipe (no NaN comes here: a column with one has failed)
+__device__ __forceinline__ bool dgt(double a, double b) {
+  long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+  x ^= (x >> 63) & 0x7fffffffffffffffll;
+  y ^= (y >> 63) & 0x7fffffffffffffffll;
+  return x > y;
+}
+__device__ __forceinline__ bool dneg(double a) {
+  const long long x = __double_as_longlong(a);
+  return x < 0 && (x << 1) != 0;
 }
 
-// NL lanes per column: 32 (a warp per column, kVicWarps per CTA: the serial
-// passes on lane 0, the per-layer maps on every lane) or 1 (a thread per
-// column, for batches with enough columns to fill the GPU: every FP64
-// instruction of the serial passes then serves 32 columns).  The operations
-// and their order are the same in both.
-template <int NL>
-__global__ void __launch_bounds__(NL == 32 ? 32 * kVicWarps : kThreads)
+__global__ void __launch_bounds__(kFinThreads, 3)
     vic_finish_kernel(const BlockDev* __restrict__ tab, StageParams p) {
+  extern __shared__ __align__(16) unsigned char fin_smem[];
+  __shared__ double sR[32], sS[32], sRS[32];
+  __shared__ int sok[32];
   const BlockDev& B = tab[blockIdx.y];
   if (!B.implicit) return;
-  const int lane = NL == 32 ? (threadIdx.x & 31) : 0;
   const VicScratch S = vic_scratch(B);
   const int ng = B.ng, nc1 = B.nc1, n = nc1 - 2 * ng;
-  const size_t ncol = S.cells / n;
-  const size_t col = NL == 32 ? (size_t)blockIdx.x * kVicWarps + (threadIdx.x >> 5)
-                              : (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= ncol) return;  // whole warps leave together when NL = 32
+  const int cols = fin_cols(n, p.fin_len);
+  const size_t ncol = S.cells / n, col0 = (size_t)blockIdx.x * cols;
+  if (col0 >= ncol) return;
+  const int nc = ncol - col0 < (size_t)cols ? (int)(ncol - col0) : cols;
+  const int tid = threadIdx.x, lane = tid & 31, wq = tid >> 5;
   const size_t plane = (size_t)nc1 * B.nc2 * B.nc3;
   const real* uin = static_cast<const real*>(B.buf[p.in]);
   const real* u0 = static_cast<const real*>(B.buf[p.u0]);
   real* uout = static_cast<real*>(B.buf[p.out]);
-  const size_t jrow = vic_row(B, col);
-  const size_t base = jrow * nc1 + ng;
-  const double grav = B.grav1;
   const double vol = B.dx3 * (B.dx2 * B.dx1);
   const double rvol = 1. / vol;  // the quotients by vol divide by it (vdiv)
-  const double* x1v = B.x1v + ng;
-  const double* x1f = B.x1f + ng;
-  const double* D = S.D + col * n * 5;
-  double* du = S.du + col * n;      // row v at du[v * cells + i]
-  const double* du0 = S.du0 + col * n;
   const size_t cs = S.cells;
-  const bool ok = vfinite(D[0]);
   const bool wood = n >= 3;
-  // work arrays of the column, in the (now free) Woodbury scratch
-  // the warp form keeps a column's arrays contiguous; the thread form
-  // interleaves the columns (index i at i ncol + col), so a warp's 32
-  // columns read and write consecutive doubles
-  const size_t ws = NL == 32 ? 1 : ncol;
-  double* const w0p = NL == 32 ? S.Z0 + col * n * 5 : S.Z0 + col;
-  const VCol mM{w0p, ws};                                  // n + 1: the face mass below layer i
-  const VCol mq{w0p + (size_t)(n + 1) * ws, ws};           // n + 1: the moved total mass
-  const VCol mdn{w0p + (size_t)(2 * n + 2) * ws, ws};      // n: the dry-gas increment
-  const VCol rho{w0p + (size_t)(3 * n + 2) * ws, ws};      // n: the density of each layer
-  // the partial matrix (implicit-scheme 1): the tangential velocities of
-  // layers 0..n (n: the ghost above), in the (free) second Woodbury vector
   const bool partial = B.implicit == 1;
-  double* const w1p = NL == 32 ? S.Z1 + col * n * 5 : S.Z1 + col;
-  const VCol vt2{w1p, ws}, vt3{w1p + (size_t)(n + 1) * ws, ws};
-  if (ok) {
-    for (int i = lane; i < n; i += NL) {
-      double w[5];
-      vic_prim(uin, plane, base + i, B.gammad, w, B.base, nc1);
-      rho[i] = w[0];
-      mdn[i] = 0.;
-      mq[i] = (D[i * 5] - du[i]) * vol;  // staged: phi of layer i
-      if (partial) {
-        vt2[i] = w[2];
-        vt3[i] = w[3];
+  const int pitch = fin_pitch(n);
+  const int len = p.fin_len;
+  double* aM = reinterpret_cast<double*>(fin_smem);  // phi, X, then M
+  double* aR = aM + len;  // the density, the available mass, the IDN row
+  double* aQ = aR + len;  // rho V, then the moved mass q
+  double* aV = aQ + len;  // q / V
+  double* aW = aV + len;  // D_rho - du0_rho
+  double* aT2 = aW + len;  // partial: the tangential velocities, 0 .. n
+  double* aT3 = aT2 + len;
+  if (tid < nc) sok[tid] = vfinite(S.D[(col0 + tid) * n * 5]);
+  __syncthreads();
+
+  // per cell: the density, phi = (D_rho - du_rho) V
+  const int cells = nc * n;
+  for (int e = tid; e < cells; e += kFinThreads) {
+    const int c = e / n, i = e - c * n;
+    if (!sok[c]) continue;
+    const size_t col = col0 + c, g = col * n + i;
+    const size_t base = vic_row(B, col) * nc1 + ng;
+    const int o = c * pitch + i;
+    double w[5];
+    vic_prim(uin, plane, base + i, B.gammad, w, B.base, nc1);
+    aR[o] = w[0];
+    aQ[o] = w[0] * vol;
+    const double d = S.D[g * 5];
+    aM[o] = (d - S.du[g]) * vol;
+    aW[o] = d - S.du0[g];
+    if (partial) {
+      aT2[o] = w[2];
+      aT3[o] = w[3];
+      if (i == n - 1) {  // the ghost above, the donor of the top face
+        vic_prim(uin, plane, base + n, B.gammad, w, B.base, nc1);
+        aT2[o + 1] = w[2];
+        aT3[o + 1] = w[3];
       }
     }
-    if (partial && lane == 0) {
-      double w[5];
-      vic_prim(uin, plane, base + n, B.gammad, w, B.base, nc1);
-      vt2[n] = w[2];
-      vt3[n] = w[3];
-    }
-    vsync<NL>();
-    if (lane == 0) {
-      double R = 0, Ssum = 0;
-      for (int i = 0; i < n; ++i) {
-        R += mq[i];
-        Ssum += rho[i] * vol;
-      }
-      double M = 0;
-      const double rss = 1. / Ssum;
-      for (int i = 0; i < n; ++i) {
-        mM[i] = M;
-        M -= mq[i] - R * vdiv(rho[i] * vol, Ssum, rss);
-      }
-      mM[n] = 0.;
-      for (int i = 0; i <= n; ++i) mq[i] = 0.;
-      double avail = (rho[0] * 1. + du[0]) * vol;
-      if (avail < 0) avail = 0;
-      for (int i = 0; i + 1 < n; ++i) {
-        double avail_up = (rho[i + 1] * 1. + du[i + 1]) * vol;
-        if (avail_up < 0) avail_up = 0;
-        double Mf = mM[i + 1];
-        double q = Mf > 0 ? Mf * 1. : Mf * 1.;
-        if (q > avail) q = avail;
-        if (q < -avail_up) q = -avail_up;
-        const double qv = vdiv(q, vol, rvol);
-        mdn[i] -= qv;
-        mdn[i + 1] += qv;
-        mq[i + 1] = q;
-        avail = avail_up + q;
-      }
-    }
-    vsync<NL>();
-    for (int i = lane; i < n; i += NL) {
-      du[i] += mdn[i];
-      du[cs + i] = D[i * 5 + 1];
-      if (!partial) {  // the partial matrix keeps the explicit m_t rows
-        du[2 * cs + i] = D[i * 5 + 2];
-        du[3 * cs + i] = D[i * 5 + 3];
-      }
-      double e = D[i * 5 + 4];
-      double projected = vdiv(mM[i] - mM[i + 1], vol, rvol);
-      double ph = -grav * x1v[i];
-      double pw = ph * (D[i * 5] - du0[i] - projected);
-      double dp_lo = -grav * (x1f[i] - x1v[i]);
-      double dp_hi = -grav * (x1f[i + 1] - x1v[i]);
-      double mv_lo = mq[i] - mM[i], mv_hi = mq[i + 1] - mM[i + 1];
-      double cw = vdiv(-(dp_hi * mv_hi - dp_lo * mv_lo), vol, rvol);
-      du[4 * cs + i] = e + (pw + cw);
-    }
-    vsync<NL>();
-    if (partial && lane == 0) {
-      // vic_tangential_momentum_column (src/implicit/vic_redistribute_impl.h
-      // :178-200): each face's moved total mass carries the donor (upwind)
-      // cell's tangential velocity; a zero transfer leaves du as it is
-      for (int i = 0; i + 1 < n; ++i) {
-        const double q = mq[i + 1];
-        const int donor = q > 0 ? i : i + 1;
-        const double pm[2] = {q * vt2[donor], q * vt3[donor]};
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          if (pm[t] == 0) continue;
-          du[(2 + t) * cs + i] -= vdiv(pm[t], vol, rvol);
-          du[(2 + t) * cs + i + 1] += vdiv(pm[t], vol, rvol);
-        }
-      }
-    }
-    vsync<NL>();
-    if (wood) {
-      // the remainder g1 sigma^2 s[du - du0] - K (raw - du0) of each layer,
-      // from the final IDN row of its neighbours
-      // staged in mdn (free again): every layer's work reads the IDN row
-      // only, so the IPR row is written after all of them
-      for (int i = lane; i < n; i += NL) {
-        double wt[3];
-        int i0;
-        vic_slope_tab(B, n, i, wt, &i0);
-        VicK K = vic_krows(B, n, i);
-        double mv0 = du[i0] - du0[i0], mv1 = du[i0 + 1] - du0[i0 + 1],
-               mv2 = du[i0 + 2] - du0[i0 + 2];
-        double sl = wt[0] * mv0;
-        sl += wt[1] * mv1;
-        sl += wt[2] * mv2;
-        double wk = K.gv * sl;
-        auto rw = [&](int k) { return D[k * 5] - du0[k]; };
-        double s = K.mid * rw(i);
-        if (i >= 1) s += K.lo * rw(i - 1);
-        if (i <= n - 2) s += K.hi * rw(i + 1);
-        if (i == 0) s += K.t0 * rw(2);
-        if (i == n - 1) s += K.t1 * rw(n - 3);
-        wk -= s;
-        mdn[i] = wk;
-      }
-      vsync<NL>();
-      for (int i = lane; i < n; i += NL) du[4 * cs + i] += mdn[i];
-    }
-    vsync<NL>();
   }
+  __syncthreads();
+  // per column: R = sum phi on one warp, S = sum rho V on another
+  if (wq < 2 && lane < nc && sok[lane]) {
+    const double* a = (wq ? aQ : aM) + lane * pitch;
+    double s = 0;
+#pragma unroll 4
+    for (int i = 0; i < n; ++i) s += a[i];
+    if (wq) {
+      sS[lane] = s;
+      sRS[lane] = 1. / s;
+    } else {
+      sR[lane] = s;
+    }
+  }
+  __syncthreads();
+  // per cell: what M loses over the layer, and the mass it can give
+  for (int e = tid; e < cells; e += kFinThreads) {
+    const int c = e / n, i = e - c * n;
+    if (!sok[c]) continue;
+    const int o = c * pitch + i;
+    aM[o] = aM[o] - sR[c] * vdiv(aQ[o], sS[c], sRS[c]);
+    double avail = (aR[o] * 1. + S.du[(col0 + c) * n + i]) * vol;
+    if (dneg(avail)) avail = 0;
+    aR[o] = avail;
+  }
+  __syncthreads();
+  // per column: the face-mass prefix and the availability clamp
+  if (wq == 0 && lane < nc && sok[lane]) {
+    double* m = aM + lane * pitch;
+    double* q = aQ + lane * pitch;
+    const double* av = aR + lane * pitch;
+    double M = 0, avail = av[0];
+    q[0] = 0.;
+#pragma unroll 4
+    for (int i = 0; i + 1 < n; ++i) {
+      const double x = m[i], up = av[i + 1];
+      m[i] = M;
+      M -= x;
+      double f = M;
+      if (dgt(f, avail)) f = avail;
+      if (dgt(-up, f)) f = -up;
+      q[i + 1] = f;
+      avail = up + f;
+    }
+    m[n - 1] = M;
+    m[n] = 0.;
+    q[n] = 0.;
+  }
+  __syncthreads();
+  // per face: q / V
+  for (int e = tid; e < cells; e += kFinThreads) {
+    const int c = e / n, i = e - c * n, o = c * pitch + i;
+    if (sok[c]) aV[o] = vdiv(aQ[o], vol, rvol);
+  }
+  __syncthreads();
+  // per cell: the IDN row with its dry increment (the faces in order, the
+  // lower one's first)
+  for (int e = tid; e < cells; e += kFinThreads) {
+    const int c = e / n, i = e - c * n, o = c * pitch + i;
+    if (!sok[c]) continue;
+    double dn = i > 0 ? 0. + aV[o] : 0.;
+    if (i + 1 < n) dn = dn - aV[o + 1];
+    aR[o] = S.du[(col0 + c) * n + i] + dn;
+  }
+  __syncthreads();
+
   // passive scalars: the clamped dry transfer of each x1 face (zero for a
   // failed column), for their share of it
   if (B.nscalar > 0)
-    for (int f = lane; f <= n; f += NL)
-      B.vicq[jrow * nc1 + ng + f] = ok ? (double)mq[f] : 0.;
+    for (int e = tid; e < nc * (n + 1); e += kFinThreads) {
+      const int c = e / (n + 1), f = e - c * (n + 1);
+      B.vicq[vic_row(B, col0 + c) * nc1 + ng + f] = sok[c] ? aQ[c * pitch + f] : 0.;
+    }
   // the x1 step field of an implicit block (FluxRegister::end_stage after
   // ImplicitHydroImpl::post_, src/implicit/implicit_hydro.cpp:625-673): the
   // stage's T_1 plus the solve's face transfers per unit area and time,
   // "vic.mass_dry" q / (dt A) on row IDN and "vic.momentum_t"
   // -sum_{k < f} (du - du0)_k V / (dt A) on rows IVY and IVZ (the prefix from
-  // the bottom wall, top face included), then the prescribed wall faces.  A
-  // failed column posts nothing.  Each face's adds run in the reference's
-  // order, +0 posts included (a -0 total becomes +0)
+  // the bottom wall, top face included; the partial matrix posts the donor
+  // transfer q w_t of each face, :520-530,662-666), then the prescribed wall
+  // faces.  A failed column posts nothing.  Each face's adds run in the
+  // reference's order, +0 posts included (a -0 total becomes +0)
   if (double* S1 = B.step[0]) {
     const double dt = p.dt[blockIdx.y];
     const double kdt = dt * (B.dx3 * B.dx2), rkdt = 1. / kdt;
@@ -1481,27 +1455,35 @@ __global__ void __launch_bounds__(NL == 32 ? 32 * kVicWarps : kThreads)
     const int nf = n + 1;
     const double* T = B.t1;
     const bool wlo = B.bc[0] == kBcReflecting, whi = B.bc[1] == kBcReflecting;
-    auto tot = [&](int v, int f) { return T[((size_t)v * ncol + col) * nf + f]; };
-    auto at = [&](int v, int f) { return S1 + v * plane + jrow * nc1 + ng + f; };
-    for (int f = lane; f < nf; f += NL) {
-      double t0 = tot(IDN, f), t1 = tot(IVX, f), t4 = tot(IPR, f);
-      if (ok) t0 = t0 + vdiv(mq[f], kdt, rkdt);
+    auto tot = [&](size_t col, int v, int f) {
+      return T[((size_t)v * ncol + col) * nf + f];
+    };
+    auto at = [&](size_t col, int v, int f) {
+      return S1 + v * plane + vic_row(B, col) * nc1 + ng + f;
+    };
+    for (int e = tid; e < nc * nf; e += kFinThreads) {
+      const int c = e / nf, f = e - c * nf;
+      const size_t col = col0 + c;
+      double t0 = tot(col, IDN, f), t1 = tot(col, IVX, f), t4 = tot(col, IPR, f);
+      if (sok[c]) t0 = t0 + vdiv(aQ[c * pitch + f], kdt, rkdt);
       if ((f == 0 && wlo) || (f == n && whi)) t0 = t4 = 0.;
-      step_set(at(IDN, f), t0, w1s, w2dt, first);
-      step_set(at(IVX, f), t1, w1s, w2dt, first);
-      step_set(at(IPR, f), t4, w1s, w2dt, first);
+      step_set(at(col, IDN, f), t0, w1s, w2dt, first);
+      step_set(at(col, IVX, f), t1, w1s, w2dt, first);
+      step_set(at(col, IPR, f), t4, w1s, w2dt, first);
     }
-    if (lane == 0) {
+    if (tid < nc) {
+      const size_t col = col0 + tid;
+      const bool ok = sok[tid] != 0;
+      const double *D = S.D + col * n * 5, *du0 = S.du0 + col * n;
+      const int o = tid * pitch;
       double sy = 0., sz = 0.;
       for (int f = 0; f < nf; ++f) {
-        double ty = tot(IVY, f), tz = tot(IVZ, f);
+        double ty = tot(col, IVY, f), tz = tot(col, IVZ, f);
         if (ok && partial) {
-          // the partial matrix posts the donor transfer q w_t of each face
-          // (src/implicit/implicit_hydro.cpp:520-530,662-666)
-          const double q = mq[f];
+          const double q = aQ[o + f];
           const int donor = q > 0. ? f - 1 : f;
-          ty = ty + vdiv(q * vt2[donor], kdt, rkdt);
-          tz = tz + vdiv(q * vt3[donor], kdt, rkdt);
+          ty = ty + vdiv(q * aT2[o + donor], kdt, rkdt);
+          tz = tz + vdiv(q * aT3[o + donor], kdt, rkdt);
         } else if (ok) {
           double py = 0., pz = 0.;
           if (f > 0) {
@@ -1513,287 +1495,86 @@ __global__ void __launch_bounds__(NL == 32 ? 32 * kVicWarps : kThreads)
           ty = ty + vdiv(py, kdt, rkdt);
           tz = tz + vdiv(pz, kdt, rkdt);
         }
-        step_set(at(IVY, f), ty, w1s, w2dt, first);
-        step_set(at(IVZ, f), tz, w1s, w2dt, first);
+        step_set(at(col, IVY, f), ty, w1s, w2dt, first);
+        step_set(at(col, IVZ, f), tz, w1s, w2dt, first);
       }
     }
   }
-  // the RK combine of the column (a failed column keeps the explicit du)
-  const double* dsel = ok ? S.du + col * n : du0;
+
+  // per cell: the map of the solution, the partial matrix's tangential
+  // transfers, the gravity-work remainder and the RK combine (a failed
+  // column keeps the explicit du)
   const real w0 = real(p.w0), w1 = real(p.w1), w2 = real(p.w2);
-  for (int i = lane; i < n; i += NL) {
-    const size_t c = base + i;
-#pragma unroll
-    for (int v = 0; v < NHYDRO; ++v) {
-      const size_t q = v * plane + c;
-      uout[q] = w0 * u0[q] + w1 * uin[q] + w2 * real(dsel[v * cs + i]);
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// (3w) the finish of wide batches in three launches.  A thread per column
-// walks every layer serially and, with a few warps per SM, waits on memory
-// at each one; here only the constituent column's serial scans keep a
-// thread per column, and the per-layer work runs a thread per cell:
-//   vic_finish_a_kernel  per cell: the layer's density (and, for the partial
-//                        matrix, its tangential velocities) and phi =
-//                        (D_rho - du_rho) V
-//   vic_finish_b_kernel  per column: the sums R and S, the face-mass prefix
-//                        M, the availability clamp (q, the dry increment),
-//                        the scalars' face transfers and the x1 step field
-//   vic_finish_c_kernel  per cell: the map of the solution, the partial
-//                        matrix's tangential transfers, the gravity-work
-//                        remainder and the RK combine, from the inputs only
-//                        (no cell writes what another reads)
-// Every value takes the operations of vic_finish_kernel in its order, so
-// the results are the same bit for bit.  A column's work arrays stay in its
-// (free) Woodbury scratch, column-contiguous:
-//   Z0: mM [n + 1] | mq [n + 1] | mdn [n] | rho [n]
-//   Z1: vt2 [n + 1] | vt3 [n + 1] | phi [n]
-struct FinishCol {
-  double *mM, *mq, *mdn, *rho, *vt2, *vt3, *phi;
-};
-
-__device__ __forceinline__ FinishCol finish_col(const VicScratch& S,
-                                                size_t col, int n) {
-  double* z0 = S.Z0 + col * n * 5;
-  double* z1 = S.Z1 + col * n * 5;
-  return FinishCol{z0, z0 + (n + 1), z0 + (2 * n + 2), z0 + (3 * n + 2),
-                   z1, z1 + (n + 1), z1 + (2 * n + 2)};
-}
-
-__global__ void __launch_bounds__(kThreads)
-    vic_finish_a_kernel(const BlockDev* __restrict__ tab, StageParams p) {
-  const BlockDev& B = tab[blockIdx.y];
-  if (!B.implicit) return;
-  const VicScratch S = vic_scratch(B);
-  const int ng = B.ng, nc1 = B.nc1, n = nc1 - 2 * ng;
-  const size_t plane = (size_t)nc1 * B.nc2 * B.nc3;
-  const real* uin = static_cast<const real*>(B.buf[p.in]);
-  const double vol = B.dx3 * (B.dx2 * B.dx1);
-  const bool partial = B.implicit == 1;
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < S.cells;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const size_t col = e / n;
-    const int i = (int)(e - col * n);
-    const double* D = S.D + col * n * 5;
-    if (!vfinite(D[0])) continue;
-    const size_t base = vic_row(B, col) * nc1 + ng;
-    const FinishCol F = finish_col(S, col, n);
-    double w[5];
-    vic_prim(uin, plane, base + i, B.gammad, w, B.base, nc1);
-    F.rho[i] = w[0];
-    F.phi[i] = (D[i * 5] - S.du[e]) * vol;
-    if (partial) {
-      F.vt2[i] = w[2];
-      F.vt3[i] = w[3];
-      if (i == n - 1) {  // the ghost above, the donor of the top face
-        vic_prim(uin, plane, base + n, B.gammad, w, B.base, nc1);
-        F.vt2[n] = w[2];
-        F.vt3[n] = w[3];
-      }
-    }
-  }
-}
-
-// a thread per column: small CTAs spread a batch's few columns (21,120 for
-// the 64-member ensemble) over every SM (one box, the ensemble's finish:
-// 514 us per stage with 256 threads, 472 with 64, 463 with 32)
-#ifndef SG_FINISH_B_THREADS
-#define SG_FINISH_B_THREADS 32
-#endif
-constexpr int kFinishBThreads = SG_FINISH_B_THREADS;
-__global__ void __launch_bounds__(kFinishBThreads)
-    vic_finish_b_kernel(const BlockDev* __restrict__ tab, StageParams p) {
-  const BlockDev& B = tab[blockIdx.y];
-  if (!B.implicit) return;
-  const VicScratch S = vic_scratch(B);
-  const int ng = B.ng, nc1 = B.nc1, n = nc1 - 2 * ng;
-  const size_t ncol = S.cells / n;
-  const size_t col = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= ncol) return;
-  const size_t plane = (size_t)nc1 * B.nc2 * B.nc3;
-  const size_t jrow = vic_row(B, col);
-  const double vol = B.dx3 * (B.dx2 * B.dx1);
-  const double rvol = 1. / vol;
-  const double* D = S.D + col * n * 5;
-  const double* du = S.du + col * n;
-  const double* du0 = S.du0 + col * n;
-  const size_t cs = S.cells;
-  const bool ok = vfinite(D[0]);
-  const bool partial = B.implicit == 1;
-  const FinishCol F = finish_col(S, col, n);
-  if (ok) {
-    double R = 0, Ssum = 0;
-    for (int i = 0; i < n; ++i) {
-      R += F.phi[i];
-      Ssum += F.rho[i] * vol;
-    }
-    double M = 0;
-    const double rss = 1. / Ssum;
-    for (int i = 0; i < n; ++i) {
-      F.mM[i] = M;
-      M -= F.phi[i] - R * vdiv(F.rho[i] * vol, Ssum, rss);
-    }
-    F.mM[n] = 0.;
-    F.mq[0] = 0.;
-    double avail = (F.rho[0] * 1. + du[0]) * vol;
-    if (avail < 0) avail = 0;
-    double dn = 0.;  // the dry increment of layer i, carried up
-    for (int i = 0; i + 1 < n; ++i) {
-      double avail_up = (F.rho[i + 1] * 1. + du[i + 1]) * vol;
-      if (avail_up < 0) avail_up = 0;
-      double Mf = F.mM[i + 1];
-      double q = Mf > 0 ? Mf * 1. : Mf * 1.;
-      if (q > avail) q = avail;
-      if (q < -avail_up) q = -avail_up;
-      const double qv = vdiv(q, vol, rvol);
-      F.mdn[i] = dn - qv;
-      dn = 0. + qv;
-      F.mq[i + 1] = q;
-      avail = avail_up + q;
-    }
-    F.mdn[n - 1] = dn;
-    F.mq[n] = 0.;
-  }
-  if (B.nscalar > 0)
-    for (int f = 0; f <= n; ++f)
-      B.vicq[jrow * nc1 + ng + f] = ok ? F.mq[f] : 0.;
-  // the x1 step field, as in vic_finish_kernel
-  if (double* S1 = B.step[0]) {
-    const double dt = p.dt[blockIdx.y];
-    const double kdt = dt * (B.dx3 * B.dx2), rkdt = 1. / kdt;
-    const double w1s = p.w1, w2dt = p.w2 * dt;
-    const bool first = p.first != 0;
-    const int nf = n + 1;
-    const double* T = B.t1;
-    const bool wlo = B.bc[0] == kBcReflecting, whi = B.bc[1] == kBcReflecting;
-    auto tot = [&](int v, int f) { return T[((size_t)v * ncol + col) * nf + f]; };
-    auto at = [&](int v, int f) { return S1 + v * plane + jrow * nc1 + ng + f; };
-    double sy = 0., sz = 0.;
-    for (int f = 0; f < nf; ++f) {
-      double t0 = tot(IDN, f), t1 = tot(IVX, f), t4 = tot(IPR, f);
-      if (ok) t0 = t0 + vdiv(F.mq[f], kdt, rkdt);
-      if ((f == 0 && wlo) || (f == n && whi)) t0 = t4 = 0.;
-      step_set(at(IDN, f), t0, w1s, w2dt, first);
-      step_set(at(IVX, f), t1, w1s, w2dt, first);
-      step_set(at(IPR, f), t4, w1s, w2dt, first);
-      double ty = tot(IVY, f), tz = tot(IVZ, f);
-      if (ok && partial) {
-        const double q = F.mq[f];
-        const int donor = q > 0. ? f - 1 : f;
-        ty = ty + vdiv(q * F.vt2[donor], kdt, rkdt);
-        tz = tz + vdiv(q * F.vt3[donor], kdt, rkdt);
-      } else if (ok) {
-        double py = 0., pz = 0.;
-        if (f > 0) {
-          sy = sy + (D[(f - 1) * 5 + 2] - du0[2 * cs + f - 1]) * vol;
-          sz = sz + (D[(f - 1) * 5 + 3] - du0[3 * cs + f - 1]) * vol;
-          py = -sy;
-          pz = -sz;
-        }
-        ty = ty + vdiv(py, kdt, rkdt);
-        tz = tz + vdiv(pz, kdt, rkdt);
-      }
-      step_set(at(IVY, f), ty, w1s, w2dt, first);
-      step_set(at(IVZ, f), tz, w1s, w2dt, first);
-    }
-  }
-}
-
-__global__ void __launch_bounds__(kThreads)
-    vic_finish_c_kernel(const BlockDev* __restrict__ tab, StageParams p) {
-  const BlockDev& B = tab[blockIdx.y];
-  if (!B.implicit) return;
-  const VicScratch S = vic_scratch(B);
-  const int ng = B.ng, nc1 = B.nc1, n = nc1 - 2 * ng;
-  const size_t plane = (size_t)nc1 * B.nc2 * B.nc3;
-  const real* uin = static_cast<const real*>(B.buf[p.in]);
-  const real* u0 = static_cast<const real*>(B.buf[p.u0]);
-  real* uout = static_cast<real*>(B.buf[p.out]);
-  const double grav = B.grav1;
-  const double vol = B.dx3 * (B.dx2 * B.dx1);
-  const double rvol = 1. / vol;
-  const double* x1v = B.x1v + ng;
-  const double* x1f = B.x1f + ng;
-  const size_t cs = S.cells;
-  const bool wood = n >= 3;
-  const bool partial = B.implicit == 1;
-  const real w0 = real(p.w0), w1 = real(p.w1), w2 = real(p.w2);
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < S.cells;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const size_t col = e / n;
-    const int i = (int)(e - col * n);
-    const double* D = S.D + col * n * 5;
-    const double* du = S.du + col * n;
-    const double* du0 = S.du0 + col * n;
-    const bool ok = vfinite(D[0]);
+  for (int e = tid; e < cells; e += kFinThreads) {
+    const int c = e / n, i = e - c * n, o = c * pitch + i;
+    const size_t col = col0 + c, g = col * n + i;
+    const double* du0 = S.du0 + g;
     double d[5];
-    if (ok) {
-      const FinishCol F = finish_col(S, col, n);
-      d[0] = du[i] + F.mdn[i];
-      d[1] = D[i * 5 + 1];
+    if (sok[c]) {
+      const double* D = S.D + g * 5;
+      d[0] = aR[o];
+      d[1] = D[1];
       if (!partial) {
-        d[2] = D[i * 5 + 2];
-        d[3] = D[i * 5 + 3];
+        d[2] = D[2];
+        d[3] = D[3];
       } else {
-        // vic_tangential_momentum_column: the face below adds its transfer,
-        // then the face above takes its own (a zero transfer is skipped)
-        const double* vt[2] = {F.vt2, F.vt3};
+        // vic_tangential_momentum_column (src/implicit/
+        // vic_redistribute_impl.h:178-200): each face's moved total mass
+        // carries the donor (upwind) cell's tangential velocity, the face
+        // below first; a zero transfer leaves du as it is
+        const double* vt[2] = {aT2 + o, aT3 + o};
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
-          double a = du[(2 + t) * cs + i];
+          double a = S.du[(2 + t) * cs + g];
           if (i > 0) {
-            const double q = F.mq[i];
-            const double pm = q * vt[t][q > 0 ? i - 1 : i];
+            const double q = aQ[o];
+            const double pm = q * vt[t][q > 0 ? -1 : 0];
             if (pm != 0) a += vdiv(pm, vol, rvol);
           }
           if (i + 1 < n) {
-            const double q = F.mq[i + 1];
-            const double pm = q * vt[t][q > 0 ? i : i + 1];
+            const double q = aQ[o + 1];
+            const double pm = q * vt[t][q > 0 ? 0 : 1];
             if (pm != 0) a -= vdiv(pm, vol, rvol);
           }
           d[2 + t] = a;
         }
       }
-      const double projected = vdiv(F.mM[i] - F.mM[i + 1], vol, rvol);
-      const double ph = -grav * x1v[i];
-      const double pw = ph * (D[i * 5] - du0[i] - projected);
-      const double dp_lo = -grav * (x1f[i] - x1v[i]);
-      const double dp_hi = -grav * (x1f[i + 1] - x1v[i]);
-      const double mv_lo = F.mq[i] - F.mM[i], mv_hi = F.mq[i + 1] - F.mM[i + 1];
-      const double cw = vdiv(-(dp_hi * mv_hi - dp_lo * mv_lo), vol, rvol);
-      double e4 = D[i * 5 + 4] + (pw + cw);
+      const double* gt = B.x1tab + 6 * i;  // [4], [5]: g dz above, below
+      const double projected = vdiv(aM[o] - aM[o + 1], vol, rvol);
+      const double ph = -B.grav1 * B.x1v[ng + i];
+      const double pw = ph * (aW[o] - projected);
+      const double mv_lo = aQ[o] - aM[o], mv_hi = aQ[o + 1] - aM[o + 1];
+      const double cw = vdiv(-(-gt[4] * mv_hi - -gt[5] * mv_lo), vol, rvol);
+      double e4 = D[4] + (pw + cw);
       if (wood) {
+        // the remainder g1 sigma^2 s[du - du0] - K (raw - du0)
         double wt[3];
         int i0;
         vic_slope_tab(B, n, i, wt, &i0);
-        VicK K = vic_krows(B, n, i);
-        auto mv = [&](int k) { return (du[k] + F.mdn[k]) - du0[k]; };
-        double sl = wt[0] * mv(i0);
-        sl += wt[1] * mv(i0 + 1);
-        sl += wt[2] * mv(i0 + 2);
+        const VicK K = vic_krows(B, n, i);
+        const int s0 = i0 - i;
+        double sl = wt[0] * (aR[o + s0] - du0[s0]);
+        sl += wt[1] * (aR[o + s0 + 1] - du0[s0 + 1]);
+        sl += wt[2] * (aR[o + s0 + 2] - du0[s0 + 2]);
         double wk = K.gv * sl;
-        auto rw = [&](int k) { return D[k * 5] - du0[k]; };
-        double s = K.mid * rw(i);
-        if (i >= 1) s += K.lo * rw(i - 1);
-        if (i <= n - 2) s += K.hi * rw(i + 1);
-        if (i == 0) s += K.t0 * rw(2);
-        if (i == n - 1) s += K.t1 * rw(n - 3);
+        double s = K.mid * aW[o];
+        if (i >= 1) s += K.lo * aW[o - 1];
+        if (i <= n - 2) s += K.hi * aW[o + 1];
+        if (i == 0) s += K.t0 * aW[o + 2];
+        if (i == n - 1) s += K.t1 * aW[o - 2];
         wk -= s;
         e4 += wk;
       }
       d[4] = e4;
     } else {
 #pragma unroll
-      for (int v = 0; v < 5; ++v) d[v] = du0[v * cs + i];
+      for (int v = 0; v < 5; ++v) d[v] = du0[v * cs];
     }
-    const size_t c = vic_row(B, col) * nc1 + ng + i;
+    const size_t cell = vic_row(B, col) * nc1 + ng + i;
 #pragma unroll
     for (int v = 0; v < NHYDRO; ++v) {
-      const size_t q = v * plane + c;
-      uout[q] = w0 * u0[q] + w1 * uin[q] + w2 * real(d[v]);
+      const size_t q = v * plane + cell;
+      uout[q] = w0 * u0[q] + w1 * uin[q] + w2 * as_real<real>(d[v]);
     }
   }
 }
