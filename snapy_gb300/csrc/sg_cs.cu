@@ -3,9 +3,10 @@
 // (6, 4, nc, nc): Phi, the radial and the two covariant tangential momenta.
 //
 // A stage is five launches, each over all six panels:
-//   cs_flux_kernel       every x2 and x3 face of the panels' interiors: the
-//                        primitives of its six-cell stencil (U/Phi, momenta
-//                        raised by the cell cosine), weno5 for Phi and cp5
+//   cs_prim_kernel       the primitives of every cell with a halo of three
+//                        (U/Phi, momenta raised by the cell cosine)
+//   cs_flux_kernel       every x2 and x3 face of the panels' interiors:
+//                        weno5 for Phi and cp5
 //                        for the velocities, the face-frame rotation, the
 //                        shallow-roe flux (dir yz) and its rotation back to
 //                        covariant components
@@ -13,14 +14,13 @@
 //                        src/coord/gnomonic_equiangle.cpp:357-463,
 //                        src/riemann/riemann_kernels.h:447-495)
 //                        (a seam face keeps its interior-side state)
-//   cs_seam_face_kernel  the seam faces again, each with its exterior-side
+//   cs_seam_kernel       the seam faces again, each with its exterior-side
 //                        state the neighbour panel's own interior-side
 //                        state, mapped into this panel's frame at the
 //                        shared face (the cross-panel face-state sync,
-//                        src/hydro/hydro_forward.cpp:719-757)
-//   cs_seam_flux_kernel  the seam faces of the non-owning panels take the
-//                        owner's flux through the Cartesian frame
-//                        (src/layout/seam_register.cpp:35)
+//                        src/hydro/hydro_forward.cpp:719-757); a face of a
+//                        non-owning panel takes the owner's flux through the
+//                        Cartesian frame (src/layout/seam_register.cpp:35)
 //   cs_update_kernel     (A2 dF2 + A3 dF3) / V minus the metric sources,
 //                        du = -dt div, and the RK combine
 //                        (src/coord/coordinate.cpp:618-662,
@@ -31,7 +31,18 @@
 //                        (src/layout/cubed_sphere_layout.cpp:563-803,
 //                        src/coord/gnomonic_equiangle.cpp:536-609)
 // All the seam geometry is in three tables built once on the host; the
-// kernels only gather.  This file is compiled twice: as the host API with
+// kernels only gather.
+//
+// FP64 is bound by the FP64 pipe (a warp instruction per 64 cycles and
+// sub-partition, however many lanes it carries), FP32 by latency.  So a cell's
+// primitives are formed once, not by each of the twelve faces that read it,
+// the square roots of the faces' geometry are a table, quotients with one
+// divisor share its reciprocal (vdiv), and the small seam and halo kernels
+// are single warps, spread over the SMs.  Measured per launch (us), before and
+// now: 6 x 45^2 FP64 HLLC: flux 70 / 26 (and 3 for the primitives), seams
+// 19 + 9 / 13, update 15 / 6, halo 14 / 6; a step 387 / 172.  6 x 96^2 FP32:
+// flux 27 / 6.4 (2.8), seams 3.6 + 3.9 / 4.0, update 7.6 / 3.9, halo 6.7 /
+// 3.7; a step 87 / 65.
 // the FP64 kernels, built with -fmad=false (the oracle's operations in its
 // order), and with SG_CS_F32_UNIT defined as the FP32 kernels alone, with
 // contraction allowed (the FP32 path is held to a tolerance, not to the
@@ -60,6 +71,10 @@ struct CsParams {
   const void* stab;
   int nseam;
   const void* sst;  // the seam face-state table (4 sides x n per panel)
+  const int* srow;  // a seam face's row in stab (-1: its panel owns it)
+  void* w;          // the primitives of `in`, laid out like a state
+  const void* fgeo;  // of each face g = 1 / sin^2: sqrt(g), 1 / sqrt(g) of
+                     // the x2 faces, then of the x3 faces
   void* sbuf;       // the seam faces' interior-side states (24 n x 4)
   const void* in;
   const void* u0;
@@ -92,8 +107,11 @@ using sg::IVX;
 using sg::IVY;
 using sg::IVZ;
 using sg::as_f64;
+using sg::vdiv;
 
 constexpr int kThreads = 256;
+constexpr int kSmall = 128;  // the stage's cell and face kernels: a warp for
+                             // each sub-partition
 constexpr int kNg = 3;
 constexpr int kGhostStride = 24;
 constexpr int kSeamStride = 18;
@@ -134,18 +152,29 @@ using sgcs::CsParams;
 // U -> W of one cell: v = m / Phi, the tangential pair raised by cos.
 // With phi0 > 0 (the FP32 state) the stored Phi row is the anomaly
 // Phi - phi0: w[IDN] stays the anomaly (what the reconstruction reads) and
-// the velocities divide by the total
-template <typename T>
+// the velocities divide by the total.  SHARED: the quotients by Phi and by
+// 1 - cos^2 divide through the reciprocals (vdiv: the same quotients while
+// Phi is not zero; the time step keeps the divisions, whose infinities it
+// reads)
+template <typename T, bool SHARED = true>
 __device__ __forceinline__ void sw_prim(const T* q, size_t pst, size_t c,
                                         T cs, T* w, T phi0 = T(0)) {
   const T phi = phi0 > T(0) ? phi0 + q[c] : q[c];
   w[IDN] = q[c];
-  const T v1 = q[pst + c] / phi, v2 = q[2 * pst + c] / phi,
-          v3 = q[3 * pst + c] / phi;
-  const T sth2 = T(1.) - cs * cs;
-  w[IVX] = v1;
-  w[IVY] = v2 / sth2 - v3 * cs / sth2;
-  w[IVZ] = -v2 * cs / sth2 + v3 / sth2;
+  if (!SHARED) {
+    const T sth2 = T(1.) - cs * cs;
+    const T v2 = q[2 * pst + c] / phi, v3 = q[3 * pst + c] / phi;
+    w[IVX] = q[pst + c] / phi;
+    w[IVY] = v2 / sth2 - v3 * cs / sth2;
+    w[IVZ] = -v2 * cs / sth2 + v3 / sth2;
+    return;
+  }
+  const T rp = T(1.) / phi;
+  const T v2 = vdiv(q[2 * pst + c], phi, rp), v3 = vdiv(q[3 * pst + c], phi, rp);
+  const T sth2 = T(1.) - cs * cs, rs = T(1.) / sth2;
+  w[IVX] = vdiv(q[pst + c], phi, rp);
+  w[IVY] = vdiv(v2, sth2, rs) - vdiv(v3 * cs, sth2, rs);
+  w[IVZ] = vdiv(-v2 * cs, sth2, rs) + vdiv(v3, sth2, rs);
 }
 
 // shallow_roe_impl with dir yz: DIM 2 (x2 faces, normal IVY) or 1 (x3).
@@ -262,22 +291,22 @@ __device__ __forceinline__ void hllc_sw(const T* L, const T* R, T* F, T phi0) {
 template <typename T, bool HLLC, bool SEAM>
 __device__ __forceinline__ void cs_face(const CsParams& P, const Geo<T>& G,
                                         int p, bool x2, int k, int j,
-                                        int side, int along) {
+                                        int side, int along, T (&F)[4]) {
   const int n = P.n, nc = P.nc;
   const size_t pst = (size_t)nc * nc;  // one variable of a panel
   const T phi0 = T(P.phi0);
-  const T* U = static_cast<const T*>(P.in);
   T* SB = static_cast<T*>(P.sbuf);  // 4 values per seam face
   {
-    T wl[4], wr[4], F[4];
+    T wl[4], wr[4];
     if (!SEAM) {
-      const T* q = U + (size_t)p * 4 * pst;
+      const T* q = static_cast<const T*>(P.w) + (size_t)p * 4 * pst;
       T st[6][4];
 #pragma unroll
       for (int m = 0; m < 6; ++m) {
         const int kk = x2 ? k : k - 3 + m, jj = x2 ? j - 3 + m : j;
         const size_t c = (size_t)kk * nc + jj;
-        sw_prim<T>(q, pst, c, T(G.cos_c[c]), st[m], phi0);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) st[m][v] = q[v * pst + c];
       }
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
@@ -315,22 +344,19 @@ __device__ __forceinline__ void cs_face(const CsParams& P, const Geo<T>& G,
                        M[3 * a + 2] * we[IVZ];
     }
     const size_t fidx = x2 ? (size_t)k * (nc + 1) + j : (size_t)k * nc + j;
-    const T cs = T(x2 ? G.cos_f2[fidx] : G.cos_f3[fidx]);
-    const T sn = T(x2 ? G.sin_f2[fidx] : G.sin_f3[fidx]);
-    const T gi = T(1.0) / (sn * sn);
+    const size_t fst = (size_t)nc * (nc + 1);  // one variable of a panel's faces
+    const T cs = x2 ? G.cos_f2[fidx] : G.cos_f3[fidx];
+    const T* fg = static_cast<const T*>(P.fgeo) + (x2 ? 0 : 2 * fst) + fidx;
+    const T rg = fg[0], ig = fg[fst];
     // to the face-local orthonormal frame (prim2local2_ / 3_)
     auto to_face = [&](T* w) {
       const T uu2 = w[IVY], uu3 = w[IVZ];
       if (x2) {
-        const T T22 = T(1.0) / sqrt(gi), T32 = cs / sqrt(T(1.0)),
-                T33 = sqrt(T(1.0));
-        w[IVZ] = T32 * uu2 + T33 * uu3;
-        w[IVY] = T22 * uu2;
+        w[IVZ] = cs * uu2 + uu3;
+        w[IVY] = ig * uu2;
       } else {
-        const T T22 = sqrt(T(1.0)), T23 = cs / sqrt(T(1.0)),
-                T33 = T(1.0) / sqrt(gi);
-        w[IVY] = T22 * uu2 + T23 * uu3;
-        w[IVZ] = T33 * uu3;
+        w[IVY] = uu2 + cs * uu3;
+        w[IVZ] = ig * uu3;
       }
     };
     to_face(wl);
@@ -349,23 +375,48 @@ __device__ __forceinline__ void cs_face(const CsParams& P, const Geo<T>& G,
     // back to covariant fluxes (flux2global2_ / 3_)
     const T txy = F[IVY], txz = F[IVZ];
     if (x2) {
-      const T T22 = sqrt(gi), T32 = -sqrt(gi) * cs / T(1.0),
-              T33 = T(1.0) / sqrt(T(1.0));
-      F[IVZ] = T32 * txy + T33 * txz;
-      F[IVY] = T22 * txy;
+      F[IVZ] = -rg * cs * txy + txz;
+      F[IVY] = rg * txy;
     } else {
-      const T T22 = T(1.0) / sqrt(T(1.0)), T23 = -cs / T(1.0) * sqrt(gi),
-              T33 = sqrt(gi);
-      F[IVY] = T22 * txy + T23 * txz;
-      F[IVZ] = T33 * txz;
+      F[IVY] = txy + -cs * rg * txz;
+      F[IVZ] = rg * txz;
     }
     const T ty = F[IVY], tz = F[IVZ];
     F[IVY] = ty + tz * cs;
     F[IVZ] = tz + ty * cs;
-    T* out = static_cast<T*>(x2 ? P.f2 : P.f3);
-    const size_t fst = (size_t)nc * (nc + 1);  // one variable of a panel's faces
+  }
+}
+
+// the flux F of that face to its place
+template <typename T>
+__device__ __forceinline__ void cs_put(const CsParams& P, int p, bool x2, int k,
+                                       int j, const T (&F)[4]) {
+  const int nc = P.nc;
+  const size_t fst = (size_t)nc * (nc + 1);
+  T* out = static_cast<T*>(x2 ? P.f2 : P.f3) + (size_t)p * 4 * fst +
+           (x2 ? (size_t)k * (nc + 1) + j : (size_t)k * nc + j);
 #pragma unroll
-    for (int v = 0; v < 4; ++v) out[((size_t)p * 4 + v) * fst + fidx] = F[v];
+  for (int v = 0; v < 4; ++v) out[v * fst] = F[v];
+}
+
+// the primitives of every cell but the halo's corners, which no face reads
+template <typename T>
+__global__ void __launch_bounds__(kSmall)
+    cs_prim_kernel(const __grid_constant__ CsParams P) {
+  const int n = P.n, nc = P.nc;
+  const size_t pst = (size_t)nc * nc, total = 6 * pst;
+  const Geo<T> G = geo_of<T>(P.geo, nc);
+  const T phi0 = T(P.phi0);
+  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
+       e += (size_t)gridDim.x * blockDim.x) {
+    const int j = (int)(e % nc), k = (int)((e / nc) % nc);
+    const size_t p = e / pst, c = e - p * pst;
+    if ((j < kNg || j >= kNg + n) && (k < kNg || k >= kNg + n)) continue;
+    T w[4];
+    sw_prim<T>(static_cast<const T*>(P.in) + p * 4 * pst, pst, c, G.cos_c[c], w, phi0);
+    T* W = static_cast<T*>(P.w) + p * 4 * pst + c;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) W[v * pst] = w[v];
   }
 }
 
@@ -373,7 +424,7 @@ __device__ __forceinline__ void cs_face(const CsParams& P, const Geo<T>& G,
 // rest x3 faces (panel, face k, column j), each from its own panel's
 // stencils; a seam face keeps its interior-side state for the seam pass
 template <typename T, bool HLLC>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kSmall)
     cs_flux_kernel(const __grid_constant__ CsParams P) {
   const int n = P.n;
   const Geo<T> G = geo_of<T>(P.geo, P.nc);
@@ -394,64 +445,65 @@ __global__ void __launch_bounds__(kThreads)
       p = (int)(r / ((size_t)n * (n + 1)));
       if (k == kNg || k == kNg + n) side = k == kNg ? 2 : 3, along = j - kNg;
     }
-    cs_face<T, HLLC, false>(P, G, p, x2, k, j, side, along);
+    T F[4];
+    cs_face<T, HLLC, false>(P, G, p, x2, k, j, side, along, F);
+    cs_put<T>(P, p, x2, k, j, F);
   }
 }
 
 // the 24 n seam faces again from the seam buffer (thread e: panel e / 4n,
 // side (e / n) % 4 in L R B T, along e % n): the Riemann problem of the
-// face's own interior side and the neighbour's
+// face's own interior side and the neighbour's.  A face that takes the
+// owner's flux solves the owner's problem itself (the same operations, the
+// same flux): the covariant pair raised at the owner's face and projected on
+// this face's tangents, signed
 template <typename T, bool HLLC>
-__global__ void __launch_bounds__(kThreads)
-    cs_seam_face_kernel(const __grid_constant__ CsParams P) {
-  const int n = P.n;
-  const Geo<T> G = geo_of<T>(P.geo, P.nc);
+__global__ void __launch_bounds__(32)
+    cs_seam_kernel(const __grid_constant__ CsParams P) {
+  const int n = P.n, nc = P.nc;
+  const Geo<T> G = geo_of<T>(P.geo, nc);
+  const size_t fst = (size_t)nc * (nc + 1);
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < 24 * n;
        e += gridDim.x * blockDim.x) {
     const int along = e % n, side = (e / n) % 4, p = e / (4 * n);
     const bool x2 = side < 2;
     const int edge = (side & 1) ? kNg + n : kNg;
     const int k = x2 ? kNg + along : edge, j = x2 ? edge : kNg + along;
-    cs_face<T, HLLC, true>(P, G, p, x2, k, j, side, along);
-  }
-}
-
-// the owner's covariant flux pair raised at its face and projected on the
-// destination face's tangents, signed
-template <typename T>
-__global__ void __launch_bounds__(kThreads) cs_seam_flux_kernel(CsParams P) {
-  const int nc = P.nc;
-  const size_t fst = (size_t)nc * (nc + 1);
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < P.nseam;
-       e += gridDim.x * blockDim.x) {
-    const T* r = static_cast<const T*>(P.stab) + (size_t)e * kSeamStride;
-    T* dst = static_cast<T*>((int)r[0] == 2 ? P.f2 : P.f3);
-    const T* src = static_cast<const T*>((int)r[2] == 2 ? P.f2 : P.f3);
-    const size_t di = (size_t)r[1], si = (size_t)r[3];
-    const size_t dp = di / fst, dc = di % fst, sp = si / fst, sc = si % fst;
-    auto at = [&](const T* a, size_t pn, int v, size_t c) {
-      return a[(pn * 4 + v) * fst + c];
-    };
-    const T sign = T(r[4]), c = T(r[5]);
-    const T m2 = at(src, sp, IVY, sc), m3 = at(src, sp, IVZ, sc);
-    const T s2 = T(1.) - c * c;
-    const T v2 = m2 / s2 - m3 * c / s2;
-    const T v3 = -m2 * c / s2 + m3 / s2;
-    T V[3];
+    const int row = P.srow[e];
+    T F[4];
+    if (row < 0) {
+      cs_face<T, HLLC, true>(P, G, p, x2, k, j, side, along, F);
+    } else {
+      const T* r = static_cast<const T*>(P.stab) + (size_t)row * kSeamStride;
+      const bool sx2 = (int)r[2] == 2;
+      const size_t si = (size_t)r[3];
+      const int sp = (int)(si / fst), sc = (int)(si % fst);
+      const int sk = sx2 ? sc / (nc + 1) : sc / nc;
+      const int sj = sx2 ? sc % (nc + 1) : sc % nc;
+      const int sside = sx2 ? (sj == kNg ? 0 : 1) : (sk == kNg ? 2 : 3);
+      T f[4];
+      cs_face<T, HLLC, true>(P, G, sp, sx2, sk, sj, sside, (sx2 ? sk : sj) - kNg, f);
+      const T sign = r[4], c = r[5];
+      const T m2 = f[IVY], m3 = f[IVZ];
+      const T s2 = T(1.) - c * c, rs = T(1.) / s2;
+      const T v2 = vdiv(m2, s2, rs) - vdiv(m3 * c, s2, rs);
+      const T v3 = vdiv(-m2 * c, s2, rs) + vdiv(m3, s2, rs);
+      T V[3];
 #pragma unroll
-    for (int q = 0; q < 3; ++q) V[q] = T(r[6 + q]) * v2 + T(r[9 + q]) * v3;
-    const T fd = at(src, sp, IDN, sc), fr = at(src, sp, IVX, sc);
-    const T y = (V[0] * T(r[12]) + V[1] * T(r[13])) + V[2] * T(r[14]);
-    const T z = (V[0] * T(r[15]) + V[1] * T(r[16])) + V[2] * T(r[17]);
-    dst[(dp * 4 + IDN) * fst + dc] = sign * fd;
-    dst[(dp * 4 + IVX) * fst + dc] = sign * fr;
-    dst[(dp * 4 + IVY) * fst + dc] = sign * y;
-    dst[(dp * 4 + IVZ) * fst + dc] = sign * z;
+      for (int q = 0; q < 3; ++q) V[q] = r[6 + q] * v2 + r[9 + q] * v3;
+      const T y = (V[0] * r[12] + V[1] * r[13]) + V[2] * r[14];
+      const T z = (V[0] * r[15] + V[1] * r[16]) + V[2] * r[17];
+      F[IDN] = sign * f[IDN];
+      F[IVX] = sign * f[IVX];
+      F[IVY] = sign * y;
+      F[IVZ] = sign * z;
+    }
+    cs_put<T>(P, p, x2, k, j, F);
   }
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads) cs_update_kernel(CsParams P) {
+__global__ void __launch_bounds__(kSmall) cs_update_kernel(CsParams P) {
   const int n = P.n, nc = P.nc;
   const size_t pst = (size_t)nc * nc, f2st = (size_t)nc * (nc + 1),
                f3st = (size_t)(nc + 1) * nc;
@@ -471,13 +523,14 @@ __global__ void __launch_bounds__(kThreads) cs_update_kernel(CsParams P) {
     const int k = kNg + (int)((e / n) % n);
     const int p = (int)(e / ((size_t)n * n));
     const size_t c = (size_t)k * nc + j;
-    const T* q = U + (size_t)p * 4 * pst;
+    const T* q = static_cast<const T*>(P.w) + (size_t)p * 4 * pst + c;
     T w[4];
-    sw_prim<T>(q, pst, c, T(G.cos_c[c]), w, phi0);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) w[v] = q[v * pst];
     const size_t i2 = (size_t)k * (nc + 1) + j, i3 = (size_t)k * nc + j;
     const T a2lo = T(G.a2[i2]), a2hi = T(G.a2[i2 + 1]);
     const T a3lo = T(G.a3[i3]), a3hi = T(G.a3[i3 + nc]);
-    const T vol = T(G.vol[c]);
+    const T vol = T(G.vol[c]), rvol = T(1.) / vol;
     T div[4];
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
@@ -485,7 +538,7 @@ __global__ void __launch_bounds__(kThreads) cs_update_kernel(CsParams P) {
       const T* f3 = F3 + ((size_t)p * 4 + v) * f3st;
       const T d2 = a2hi * f2[i2 + 1] - a2lo * f2[i2];
       const T d3 = a3hi * f3[i3 + nc] - a3lo * f3[i3];
-      div[v] = (d2 + d3) / vol;
+      div[v] = vdiv(d2 + d3, vol, rvol);
     }
     // Phi and p = Phi^2 / 2; with phi0 > 0, the stored anomaly Phi' and
     // the pressure anomaly phi0 Phi' + Phi'^2 / 2 (see shallow_roe)
@@ -509,7 +562,7 @@ __global__ void __launch_bounds__(kThreads) cs_update_kernel(CsParams P) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads) cs_ghost_kernel(CsParams P, void* buf) {
+__global__ void __launch_bounds__(32) cs_ghost_kernel(CsParams P, void* buf) {
   const int nc = P.nc;
   const size_t pst = (size_t)nc * nc;
   T* Q = static_cast<T*>(buf);
@@ -535,9 +588,9 @@ __global__ void __launch_bounds__(kThreads) cs_ghost_kernel(CsParams P, void* bu
       const T* g = r + 4 + 7 * s;
       const T c = T(g[0]);
       const T m2 = Q[at(src[s], IVY)], m3 = Q[at(src[s], IVZ)];
-      const T s2 = T(1.) - c * c;
-      const T v2 = m2 / s2 - m3 * c / s2;
-      const T v3 = -m2 * c / s2 + m3 / s2;
+      const T s2 = T(1.) - c * c, rs = T(1.) / s2;
+      const T v2 = vdiv(m2, s2, rs) - vdiv(m3 * c, s2, rs);
+      const T v3 = vdiv(-m2 * c, s2, rs) + vdiv(m3, s2, rs);
 #pragma unroll
       for (int qq = 0; qq < 3; ++qq) Vs[s][qq] = T(g[1 + qq]) * v2 + T(g[4 + qq]) * v3;
     }
@@ -580,7 +633,7 @@ __global__ void __launch_bounds__(kThreads) cs_dt_kernel(CsParams P, const void*
     const int p = (int)(e / ((size_t)n * n));
     const size_t c = (size_t)k * nc + j;
     T w[4];
-    sw_prim<T>(U + (size_t)p * 4 * pst, pst, c, T(G.cos_c[c]), w, phi0);
+    sw_prim<T, false>(U + (size_t)p * 4 * pst, pst, c, T(G.cos_c[c]), w, phi0);
     const T cs = sqrt(phi0 > T(0) ? phi0 + w[IDN] : w[IDN]);
     const T d2 = T(G.w2[c]) / (fabs(w[IVY]) + cs);
     const T d3 = T(G.w3[c]) / (fabs(w[IVZ]) + cs);
@@ -656,9 +709,9 @@ int cs_fail(int code, const char* fmt, ...) {
   return sg_fail_message(code, buf);
 }
 
-int grid_for(size_t work) {
-  size_t g = (work + kThreads - 1) / kThreads;
-  if (g > 4096) g = 4096;
+int grid_for(size_t work, int threads = kThreads) {
+  size_t g = (work + threads - 1) / threads;
+  if (g > 8192) g = 8192;
   return (int)(g ? g : 1);
 }
 
@@ -707,21 +760,21 @@ __global__ void __launch_bounds__(kThreads) cs_step_kernel(CsParams P) {
 // the five launches of a stage, the seam halo and the dt reduction in T
 template <typename T>
 int launch_stage(const CsParams& P, size_t faces, size_t cells, cudaStream_t s) {
+  cs_prim_kernel<T><<<grid_for((size_t)6 * P.nc * P.nc, kSmall), kSmall, 0, s>>>(P);
   (P.hllc ? cs_flux_kernel<T, true> : cs_flux_kernel<T, false>)
-      <<<grid_for(faces), kThreads, 0, s>>>(P);
-  (P.hllc ? cs_seam_face_kernel<T, true> : cs_seam_face_kernel<T, false>)
-      <<<grid_for(24 * (size_t)P.n), kThreads, 0, s>>>(P);
-  cs_seam_flux_kernel<T><<<grid_for(P.nseam), kThreads, 0, s>>>(P);
+      <<<grid_for(faces, kSmall), kSmall, 0, s>>>(P);
+  (P.hllc ? cs_seam_kernel<T, true> : cs_seam_kernel<T, false>)
+      <<<grid_for(24 * (size_t)P.n, 32), 32, 0, s>>>(P);
   if (P.s2 && P.s3)
     cs_step_kernel<T><<<grid_for(2 * (size_t)24 * P.n * (P.n + 1)), kThreads, 0, s>>>(P);
-  cs_update_kernel<T><<<grid_for(cells), kThreads, 0, s>>>(P);
-  cs_ghost_kernel<T><<<grid_for(P.nghost), kThreads, 0, s>>>(P, P.out);
+  cs_update_kernel<T><<<grid_for(cells, kSmall), kSmall, 0, s>>>(P);
+  cs_ghost_kernel<T><<<grid_for(P.nghost, 32), 32, 0, s>>>(P, P.out);
   return (int)cudaGetLastError();
 }
 
 template <typename T>
 int launch_ghost(const CsParams& P, void* buf, cudaStream_t s) {
-  cs_ghost_kernel<T><<<grid_for(P.nghost), kThreads, 0, s>>>(P, buf);
+  cs_ghost_kernel<T><<<grid_for(P.nghost, 32), 32, 0, s>>>(P, buf);
   return (int)cudaGetLastError();
 }
 
@@ -755,8 +808,43 @@ __global__ void to_f32(const double* src, float* dst, size_t n) {
     dst[i] = (float)src[i];
 }
 
+// the faces' sqrt(g) and 1 / sqrt(g), g = 1 / sin^2, in the state's type
+template <typename T>
+__global__ void cs_face_geo(const T* geo, T* out, int nc) {
+  const Geo<T> G = geo_of<T>(geo, nc);
+  const size_t fst = (size_t)nc * (nc + 1);
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < 2 * fst;
+       i += (size_t)gridDim.x * blockDim.x) {
+    const bool x2 = i < fst;
+    const size_t f = x2 ? i : i - fst;
+    const T sn = x2 ? G.sin_f2[f] : G.sin_f3[f];
+    const T rg = sqrt(T(1.0) / (sn * sn));
+    T* o = out + (x2 ? 0 : 2 * fst) + f;
+    o[0] = rg;
+    o[fst] = T(1.0) / rg;
+  }
+}
+
+// the row of the seam table that sets each seam face (set to -1 before)
+__global__ void cs_seam_rows(const double* tab, int nseam, int n, int nc, int* row) {
+  const size_t fst = (size_t)nc * (nc + 1);
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nseam;
+       e += gridDim.x * blockDim.x) {
+    const double* r = tab + (size_t)e * kSeamStride;
+    const bool x2 = (int)r[0] == 2;
+    const size_t di = (size_t)r[1];
+    const int p = (int)(di / fst), c = (int)(di % fst);
+    const int k = x2 ? c / (nc + 1) : c / nc, j = x2 ? c % (nc + 1) : c % nc;
+    const int side = x2 ? (j == kNg ? 0 : 1) : (k == kNg ? 2 : 3);
+    row[(p * 4 + side) * n + (x2 ? k : j) - kNg] = e;
+  }
+}
+
 struct sg_cs_handle {
   sg_cs_desc d;
+  void* w = nullptr;     // the primitives
+  void* fgeo = nullptr;  // the faces' derived geometry
+  int* srow = nullptr;   // the seam faces' rows
   // SG_F32: FP32 copies of the geometry and of the two seam tables
   float* geo32 = nullptr;
   float* gtab32 = nullptr;
@@ -796,13 +884,28 @@ int sg_cs_create(const sg_cs_desc* d, sg_cs_handle** out) {
     const unsigned long long init[2] = {kKeyInf, 0};
     e = cudaMemcpy(h->key, init, sizeof(init), cudaMemcpyHostToDevice);
   }
+  const size_t esz = d->dtype == SG_F64 ? 8 : 4;
+  const size_t ncp = (size_t)d->n + 2 * kNg, srows = (size_t)24 * d->n;
+  if (e == cudaSuccess) e = cudaMalloc(&h->w, 6 * 4 * ncp * ncp * esz);
+  if (e == cudaSuccess) e = cudaMalloc(&h->fgeo, 4 * ncp * (ncp + 1) * esz);
+  if (e == cudaSuccess) e = cudaMalloc(&h->srow, srows * sizeof(int));
+  if (e == cudaSuccess) e = cudaMemset(h->srow, 0xff, srows * sizeof(int));
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();  // the tables are written
+  if (e == cudaSuccess) {
+    cs_seam_rows<<<grid_for(d->nseam), kThreads>>>(d->seam_tab, d->nseam, d->n,
+                                                   (int)ncp, h->srow);
+    if (d->dtype == SG_F64)
+      cs_face_geo<double><<<grid_for(2 * ncp * (ncp + 1)), kThreads>>>(
+          d->geo, static_cast<double*>(h->fgeo), (int)ncp);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  }
   if (e == cudaSuccess && d->dtype == SG_F32) {
     // the FP32 kernels read FP32 copies; the tables' flat indices (cells,
     // and faces up to 6 nc (nc + 1)) stay exact in FP32 below 2^24
     const size_t nc = (size_t)d->n + 2 * kNg;
     if (6 * nc * (nc + 1) >= (size_t)1 << 24) {
-      cudaFree(h->key);
-      delete h;
+      sg_cs_destroy(h);
       return cs_fail(SG_ERR_UNSUPPORTED, "sg_cs_create: FP32 needs fewer than "
                      "2^24 faces in the six panels (n %d)", d->n);
     }
@@ -819,17 +922,14 @@ int sg_cs_create(const sg_cs_desc* d, sg_cs_handle** out) {
       to_f32<<<grid_for(nt), kThreads>>>(d->ghost_tab, h->gtab32, nt);
       to_f32<<<grid_for(ns), kThreads>>>(d->seam_tab, h->stab32, ns);
       to_f32<<<grid_for(nss), kThreads>>>(d->seam_state_tab, h->sst32, nss);
+      cs_face_geo<float><<<grid_for(2 * ncp * (ncp + 1)), kThreads>>>(
+          h->geo32, static_cast<float*>(h->fgeo), (int)ncp);
       e = cudaGetLastError();
       if (e == cudaSuccess) e = cudaDeviceSynchronize();
     }
   }
   if (e != cudaSuccess) {
-    if (h->key) cudaFree(h->key);
-    cudaFree(h->geo32);
-    cudaFree(h->gtab32);
-    cudaFree(h->stab32);
-    cudaFree(h->sst32);
-    delete h;
+    sg_cs_destroy(h);
     return cs_fail(SG_ERR_CUDA, "sg_cs_create: %s", cudaGetErrorString(e));
   }
   *out = h;
@@ -839,6 +939,9 @@ int sg_cs_create(const sg_cs_desc* d, sg_cs_handle** out) {
 int sg_cs_destroy(sg_cs_handle* h) {
   if (!h) return 0;
   if (h->key) cudaFree(h->key);
+  cudaFree(h->w);
+  cudaFree(h->fgeo);
+  cudaFree(h->srow);
   cudaFree(h->geo32);
   cudaFree(h->gtab32);
   cudaFree(h->stab32);
@@ -921,6 +1024,9 @@ static CsParams cs_params(const sg_cs_handle* h) {
   P.nseam = h->d.nseam;
   P.sst = f32 ? (const void*)h->sst32 : (const void*)h->d.seam_state_tab;
   P.phi0 = h->d.dtype == SG_F32 ? h->d.phi_ref : 0.;
+  P.srow = h->srow;
+  P.w = h->w;
+  P.fgeo = h->fgeo;
   P.hllc = h->d.riemann == SG_CS_HLLC;
   const size_t nc = P.nc;
   const size_t s = h->d.dtype == SG_F64 ? 8 : 4;
