@@ -241,6 +241,7 @@ struct sg_handle {
   int x3_chunk = 1, x3_ctas = 1;  // the x3 sweep's schedule (plan_x3)
   int line_seg = 0, line_ctas = 0;  // line_kernel's (plan_line)
   int fin_len = 0, fin_ctas = 0;  // the finish's schedule (plan_finish)
+  int solve_ctas = 0;             // the direct solve's (plan_solve)
   bool implicit = false;
   int vic_kinds = 0;  // bit 0: a block with the full 5x5 matrix, bit 1: 3x3
   bool ref32 = false;  // an FP32 block under gravity: base_ref_kernel runs
@@ -376,6 +377,55 @@ void plan_finish(sg_handle* h) {
   h->fin_ctas = (int)most;
 }
 
+// The form of the direct solve of each block: a warp per column for the
+// blocks of more than some number of layers, four columns a warp for the
+// rest.  The time is the longest column's chain (thousands of cycles a layer,
+// alone on a sub-partition) or the FP64 pipe's work (thousands of cycles a
+// layer and warp) on the fullest sub-partition, which holds about 1.7 times
+// the mean; the number of layers with the least of that is taken.  Measured
+// per launch (us), four columns / a warp each: 512 columns of 128 layers 1360
+// / 783, 1,665 of 48 525 / 621; nine members of 27 to 103 layers 1202 / 1142,
+// and 959 with the warp form from 93 layers up (the rule's choice), 1238 from
+// 69 up
+constexpr double kSolveWarpChain = 11., kSolveFourChain = 20.;
+constexpr double kSolveWarpPipe = 9., kSolveFourPipe = 13.5;
+void plan_solve(sg_handle* h) {
+  int sms = 152;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+  auto direct = [](const BlockDev& B) { return B.implicit == 9 && !B.implicit_f32; };
+  auto cols = [](const BlockDev& B) {
+    return (size_t)(B.nc2 > 1 ? B.nc2 - 2 * B.ng : 1) * (B.nc3 > 1 ? B.nc3 - 2 * B.ng : 1);
+  };
+  // the time if blocks of more than `most` layers take the warp form
+  auto cost = [&](int most) {
+    double chain = 0., pipe = 0.;
+    for (const BlockDev& B : h->host) {
+      if (!direct(B)) continue;
+      const double n = B.nc1 - 2 * B.ng;
+      const bool one = n > most;
+      chain = std::max(chain, n * (one ? kSolveWarpChain : kSolveFourChain));
+      pipe += n * (one ? (double)cols(B) * kSolveWarpPipe
+                       : (double)((cols(B) + 3) / 4) * kSolveFourPipe);
+    }
+    return std::max(chain, 1.7 * pipe / (4. * sms));
+  };
+  int most = 1 << 30;
+  double best = cost(most);
+  for (const BlockDev& B : h->host) {
+    if (!direct(B)) continue;
+    const int m = B.nc1 - 2 * B.ng - 1;  // this block and longer ones
+    const double t = cost(m);
+    if (t < best) best = t, most = m;
+  }
+  size_t ctas = 1;
+  for (BlockDev& B : h->host) {
+    B.wsolve = direct(B) && B.nc1 - 2 * B.ng > most;
+    if (B.implicit == 9)
+      ctas = std::max(ctas, B.wsolve && !B.psw ? cols(B) : (cols(B) + 3) / 4);
+  }
+  h->solve_ctas = (int)ctas;
+}
+
 // The cells a CTA of line_kernel takes: the fewest of 8 to 64 that leave no
 // more CTAs than SMs.  A segment costs its CTA one face's work per thread
 // until the threads are full (12 cells), and each its own halo of six cells
@@ -486,6 +536,7 @@ void psw_apply(sg_handle* h, int on) {
   for (int b = 0; b < h->nblock; ++b)
     h->host[b].psw = on && psw_block(h, b) ? h->psw_mem + h->psw_off[b] : nullptr;
   h->psw_on = on;
+  plan_solve(h);
   h->dirty = true;
 }
 }  // namespace
@@ -624,6 +675,7 @@ int sg_autotune(sg_handle* h, int32_t reps, int32_t* tj_out,
     p.psw = h->psw_on;
     p.fallbacks = h->fallbacks;
     p.max_nc1 = h->max_nc1;
+    p.solve_ctas = h->solve_ctas;
     p.fin_len = h->fin_len;
     p.fin_ctas = h->fin_ctas;
     p.line_seg = h->line_seg;
@@ -704,6 +756,7 @@ int sg_autotune(sg_handle* h, int32_t reps, int32_t* tj_out,
           psw_apply(h, sweep);
           if (!rc) rc = upload(h, s);
           p.psw = sweep;
+          p.solve_ctas = h->solve_ctas;
         }
         for (int form : {1, 2}) {
           if (rc) break;
@@ -991,7 +1044,10 @@ int sg_create(const sg_scheme* scheme, const sg_block_desc* blocks,
   h->ntile = tile;
   if (h->has3) plan_x3(h);
   plan_line(h);
-  if (h->implicit) plan_finish(h);
+  if (h->implicit) {
+    plan_finish(h);
+    plan_solve(h);
+  }
   cudaError_t e = cudaMalloc(&h->dev, sizeof(BlockDev) * nblock);
   if (e == cudaSuccess)
     e = cudaMalloc(&h->red, sizeof(unsigned long long) * 4 * nblock);
@@ -1321,6 +1377,7 @@ int sg_stage(sg_handle* h, int32_t stage, const double* dt_dev,
   p.psw = h->psw_on;
   p.fallbacks = h->fallbacks;
   p.max_nc1 = h->max_nc1;
+  p.solve_ctas = h->solve_ctas;
   p.fin_len = h->fin_len;
   p.fin_ctas = h->fin_ctas;
   p.line_seg = h->line_seg;

@@ -43,6 +43,8 @@
 // 19 + 9 / 13, update 15 / 6, halo 14 / 6; a step 387 / 172.  6 x 96^2 FP32:
 // flux 27 / 6.4 (2.8), seams 3.6 + 3.9 / 4.0, update 7.6 / 3.9, halo 6.7 /
 // 3.7; a step 87 / 65.
+//
+// This file is compiled twice: as the host API with
 // the FP64 kernels, built with -fmad=false (the oracle's operations in its
 // order), and with SG_CS_F32_UNIT defined as the FP32 kernels alone, with
 // contraction allowed (the FP32 path is held to a tolerance, not to the

@@ -2691,7 +2691,7 @@ extern "C" int SG_NAME(sg_launch_vic)(const BlockDev* tab, StageParams p,
     if (p.refine)
       vic_solve_kernel<true><<<dim3(gs, p.nblock), 32, 0, stream>>>(tab, p, status);
     else
-      vic_solve_kernel<false><<<dim3(gs, p.nblock), 32, 0, stream>>>(tab, p, status);
+      vic_solve_kernel<false><<<dim3(p.solve_ctas, p.nblock), 32, 0, stream>>>(tab, p, status);
   }
   if (p.vic_kinds & 2) {
     const int g3 = (int)((max_cols + kThreads - 1) / kThreads);

@@ -51,6 +51,7 @@ struct BlockDev {
   int32_t implicit;
   int32_t implicit_f32;  // implicit-precision float32: FP32 block assembly
   double* vic;
+  int32_t wsolve;  // the direct solve takes a warp per column (plan_solve)
   // the layer-parallel (partitioned) form of the scheme-9 solve of an
   // FP64-assembled block (sg_set_sweep): its region, per interior cell the
   // E and F blocks (25 doubles each), then one int per interior column
@@ -183,6 +184,7 @@ struct StageParams {
                         // staging wait ran out)
   int32_t smem_rows;    // x1 lines held in shared memory per tile
   int32_t max_nc1;
+  int32_t solve_ctas;   // the direct solve's CTAs per block
   int32_t fin_len;      // doubles of a finish CTA's array
   int32_t fin_ctas;     // its CTAs per block
   int32_t line_seg;     // x1 cells a CTA of line_kernel takes

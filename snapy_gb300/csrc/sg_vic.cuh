@@ -703,6 +703,270 @@ struct VicSolveSmem {
   double rd[kVicCols][5];          // 1 / the diagonal of each factorisation
 };
 
+// The same sweep with a warp for one column (a block's wsolve), for batches
+// whose columns leave sub-partitions idle: the elimination and the
+// factorisation a lane per entry (lane 5 c + r: row r of column c, the
+// right-hand side the sixth column), the back-solve four lanes per
+// right-hand-side column (lane 4 q + h: row h + 1; row 0 rides on the lane
+// of row 4 once that row is solved).  A layer is then about 130 FP64
+// instructions in sequence where four columns share a warp in 210, with an
+// eighth of the other instructions (a lane holds an entry, not a column), and
+// its row exchanges are real branches.  Every value takes the operations of
+// the four-column form in its order (each entry its subtractions k ascending,
+// the same quotients), so the solution is the same bit for bit.  512 columns
+// of 128 layers: 1360 us per launch with four columns a warp, 783 with one.
+struct VicWarpSmem {
+  double b[25], c[25], lu[25];  // the layer's b, c and factors, row-major
+  double s[40];     // the previous solution: column q's row k at 5 q + k
+  double dv[5], z[5], rd[5];    // rhs rows, the diagonal's reciprocals
+  double v[2][15];  // back substitution: d, z0, z1 of a layer
+  int perm[5];      // the factorisation's row of each row
+};
+
+__device__ __forceinline__ void vic_column_warp(const BlockDev& Bk,
+                                                const VicScratch& S, size_t col,
+                                                int n, double dtc,
+                                                VicWarpSmem& w, int* status) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x;
+  const int c = lane / 5, r = lane - 5 * c;
+  const bool in25 = lane < 25, ind = lane >= 25 && lane < 30;
+  const double rdtc = 1.0 / dtc;
+  const bool wood = n >= 3;
+  double* A = S.A + col * n * 25;
+  const double* Bm = S.B + col * n * 25;
+  const double* C = S.C + col * n * 25;
+  double* D = S.D + col * n * 5;
+  double* Z0 = S.Z0 + col * n * 5;
+  double* Z1 = S.Z1 + col * n * 5;
+  const double* du = S.du + col * n;  // row v at du[v * cells + i]
+  auto from = [&](double v, int src) { return __shfl_sync(full, v, src); };
+
+  // the input screen: du of every layer finite
+  bool fin = true;
+  for (int e = lane; e < 5 * n; e += 32)
+    fin = fin && vfinite(du[(size_t)(e / n) * S.cells + (e % n)]);
+  bool ok = __all_sync(full, fin);
+
+  // a layer's entries arrive one layer ahead
+  const int at = r * 5 + c;
+  double na = 0., nb = 0., nc = 0., nd = 0.;
+  auto fetch = [&](int i) {
+    if (in25) {
+      na = A[i * 25 + at];
+      nb = Bm[i * 25 + at];
+      nc = C[i * 25 + at];
+    } else if (ind) {
+      nd = du[(size_t)r * S.cells + i];
+    }
+  };
+  fetch(0);
+  const int q = lane >> 2, h = lane & 3, row = h + 1, g0 = lane & ~3;
+  for (int i = 0; i < n && ok; ++i) {
+    double x = na;
+    const double bv = nb, cv = nc;
+    const double dq = div_rcp(nd, dtc, rdtc);
+    if (ind) x = dq;
+    if (i + 1 < n) fetch(i + 1);
+    if (in25) {
+      w.b[at] = bv;
+      w.c[at] = cv;
+    }
+    __syncwarp();
+    // x -= b s'  (a[i] - b[i] a'[i-1] and rhs - b[i] d'[i-1]), k in order;
+    // z0's five rows from the products of 25 lanes
+    double z = i == 0 && lane == 4 ? 1. : 0.;
+    if (i > 0) {
+      if (lane < 30) {
+        double t = w.b[r * 5] * w.s[c * 5];
+#pragma unroll
+        for (int k = 1; k < 5; ++k) t = t + w.b[r * 5 + k] * w.s[c * 5 + k];
+        x = x - t;
+      }
+      const double pz = in25 ? bv * w.s[30 + c] : 0.;
+      double t = from(pz, r);
+#pragma unroll
+      for (int k = 1; k < 5; ++k) t = t + from(pz, 5 * k + r);
+      z = z - t;
+    }
+
+    // ---- the factorisation, the right-hand side's forward sweep with it ----
+    bool good = !in25 || vfinite(x);
+    unsigned long long ab = in25 ? vbits(fabs(x)) : 0ull, mx = 0ull;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      const unsigned long long o = __shfl_sync(full, ab, 5 * k + r);
+      mx = o > mx ? o : mx;
+    }
+    double big = __longlong_as_double(static_cast<long long>(mx));
+    double vv = 1.0 / big;
+    good = good && mx != 0ull && vfinite(vv);
+    int perm = r;
+    double rd = 0.;
+#pragma unroll
+    for (int J = 0; J < 5; ++J) {
+      const double dum = vv * fabs(x);
+      if (c == J && r >= J) good = good && vfinite(dum);
+      unsigned long long best = 0ull;
+      int imax = J;
+#pragma unroll
+      for (int k = J; k < 5; ++k) {
+        const unsigned long long o = __shfl_sync(full, vbits(dum), 5 * J + k);
+        if (o >= best) {
+          best = o;
+          imax = k;
+        }
+      }
+      if (imax != J) {  // the whole warp
+        const int src = r == J ? imax : (r == imax ? J : r);
+        const int sl = lane < 30 ? 5 * c + src : lane;
+        x = from(x, sl);
+        vv = from(vv, sl);
+        big = from(big, sl);
+        perm = __shfl_sync(full, perm, sl);
+      }
+      const double dinv = 1.0 / from(x, 6 * J);
+      if (c == J && r == J) rd = dinv;
+      if (J < 4) {
+        if (in25 && c == J && r > J) x = x * dinv;
+        const double l = from(x, 5 * J + r);
+        const double u = from(x, lane < 30 ? 5 * c + J : lane);
+        if (lane < 30 && c > J && r > J) x = x - l * u;
+      }
+    }
+    if (in25) {
+      good = good && vfinite(x);
+      // the pivot tolerance on the final diagonal and scale
+      if (c == r)
+        good = good && !(div_rcp(fabs(x), big, vv) <= 8. * 5 * 2.220446049250313e-16);
+    }
+    ok = __all_sync(full, good);
+    if (in25) {
+      w.lu[at] = x;
+      if (c == r) w.rd[r] = rd;
+    } else if (ind) {
+      w.dv[r] = x;
+    }
+    if (lane < 5) {
+      w.z[lane] = z;
+      w.perm[lane] = perm;
+    }
+    __syncwarp();
+
+    // ---- lubksb: columns 0-4 of c, d (forward done), z0, z1 ----
+    const int p0 = w.perm[0], pr = w.perm[row];
+    double y0, y;
+    if (q < 5) {
+      y0 = w.c[p0 * 5 + q];
+      y = w.c[pr * 5 + q];
+    } else if (q == 5) {
+      y0 = w.dv[0];
+      y = w.dv[row];
+    } else if (q == 6) {
+      y0 = w.z[p0];
+      y = w.z[pr];
+    } else {
+      y0 = i == n - 1 && p0 == 4 ? 1. : 0.;
+      y = i == n - 1 && pr == 4 ? 1. : 0.;
+    }
+    const double* lr = w.lu + row * 5;
+    if (q != 5) y = y - lr[0] * y0;
+#pragma unroll
+    for (int jj = 1; jj < 4; ++jj) {
+      const double v = from(y, g0 + jj - 1);
+      if (q != 5 && row > jj) y = y - lr[jj] * v;
+    }
+    const double* ur = h == 3 ? w.lu : lr;  // the products of row 0 or its own
+    const double x4 = from(div_rcp(y, w.lu[24], w.rd[4]), g0 + 3);
+    const double m4 = ur[4] * x4;
+    const double x3 = from(div_rcp(y - m4, w.lu[18], w.rd[3]), g0 + 2);
+    const double m3 = ur[3] * x3;
+    const double x2 = from(div_rcp((y - m3) - m4, w.lu[12], w.rd[2]), g0 + 1);
+    const double m2 = ur[2] * x2;
+    const double x1 = from(div_rcp(((y - m2) - m3) - m4, w.lu[6], w.rd[1]), g0);
+    const double m1 = ur[1] * x1;
+    const double x0 =
+        from(div_rcp((((y0 - m1) - m2) - m3) - m4, w.lu[0], w.rd[0]), g0 + 3);
+    const double xs = h == 0 ? x1 : (h == 1 ? x2 : (h == 2 ? x3 : x4));
+    ok = __all_sync(full, (q >= 6 && !wood) || (vfinite(xs) && vfinite(x0))) && ok;
+    if (q < 5) {
+      double* a = A + i * 25 + q;
+      a[row * 5] = xs;
+      if (h == 0) a[0] = x0;
+    } else {
+      double* o = (q == 5 ? D : (q == 6 ? Z0 : Z1)) + i * 5;
+      o[row] = xs;
+      if (h == 0) o[0] = x0;
+    }
+    w.s[5 * q + row] = xs;
+    if (h == 0) w.s[5 * q] = x0;
+    __syncwarp();
+  }
+
+  // ---- back substitution: x[i] -= a'[i] x[i+1] for d, z0, z1 ----
+  if (ok) {
+    const int v = lane / 5;
+    const bool on = lane < 15;
+    double* vec = v == 0 ? D : (v == 1 ? Z0 : Z1);
+    if (on) w.v[0][lane] = w.s[25 + lane];
+    double ar[5] = {0., 0., 0., 0., 0.}, cur = 0.;
+    auto load = [&](int i) {
+      if (!on) return;
+#pragma unroll
+      for (int k = 0; k < 5; ++k) ar[k] = A[i * 25 + r * 5 + k];
+      cur = vec[i * 5 + r];
+    };
+    load(n - 2);
+    __syncwarp();
+    int at2 = 0;
+    for (int i = n - 2; i >= 0; --i) {
+      const double a0 = ar[0], a1 = ar[1], a2 = ar[2], a3 = ar[3], a4 = ar[4];
+      const double now = cur;
+      if (i > 0) load(i - 1);
+      if (on) {
+        const double* xn = w.v[at2] + v * 5;
+        double t = a0 * xn[0];
+        t = t + a1 * xn[1];
+        t = t + a2 * xn[2];
+        t = t + a3 * xn[3];
+        t = t + a4 * xn[4];
+        const double val = now - t;
+        vec[i * 5 + r] = val;
+        w.v[at2 ^ 1][lane] = val;
+      }
+      __syncwarp();
+      at2 ^= 1;
+    }
+    if (wood) {
+      VicK K0 = vic_krows(Bk, n, 0), K1 = vic_krows(Bk, n, n - 1);
+      const double k0 = -K0.t0 / dtc, k1 = -K1.t1 / dtc;
+      const int a0 = 2, a1 = n - 3;
+      double m00 = 1. + k0 * Z0[a0 * 5], m01 = k0 * Z1[a0 * 5];
+      double m10 = k1 * Z0[a1 * 5], m11 = 1. + k1 * Z1[a1 * 5];
+      double r0 = k0 * D[a0 * 5], r1 = k1 * D[a1 * 5];
+      double det = m00 * m11 - m01 * m10;
+      double al0 = (m11 * r0 - m01 * r1) / det;
+      double al1 = (m00 * r1 - m10 * r0) / det;
+      __syncwarp();  // read before any lane updates D
+      for (int e = lane; e < 5 * n; e += 32) {
+        double d = D[e];
+        d -= Z0[e] * al0;
+        d -= Z1[e] * al1;
+        D[e] = d;
+        ok = ok && vfinite(d);
+      }
+    } else {
+      for (int e = lane; e < 5 * n; e += 32) ok = ok && vfinite(D[e]);
+    }
+    ok = __all_sync(full, ok);
+  }
+  // a failed column is marked in its solution: the finish keeps du0
+  if (!ok && lane == 0) {
+    D[0] = __longlong_as_double(0x7ff8000000000000ll);
+    atomicOr(&status[blockIdx.y], kVicFailed);
+  }
+}
+
 // BLK32: the refined solve's masked columns, whose blocks are the FP32 ones
 // (a separate instantiation, so the direct solve's block loads carry no
 // select)
@@ -710,12 +974,21 @@ template <bool BLK32>
 __global__ void __launch_bounds__(32)
     vic_solve_kernel(const BlockDev* __restrict__ tab, StageParams p,
                      int* status) {
-  __shared__ VicSolveSmem sm;
+  __shared__ union {
+    VicSolveSmem four;
+    VicWarpSmem one;
+  } smem;
+  VicSolveSmem& sm = smem.four;
   const BlockDev& Bk = tab[blockIdx.y];
   if (!Bk.implicit || Bk.implicit == 1) return;  // scheme 1: vic_solve3
   const VicScratch S = vic_scratch(Bk);
   const int n = Bk.nc1 - 2 * Bk.ng;
   const size_t ncol = S.cells / n;
+  if (!BLK32 && Bk.wsolve && !Bk.psw) {
+    if (blockIdx.x < ncol)
+      vic_column_warp(Bk, S, blockIdx.x, n, p.w2 * p.dt[blockIdx.y], smem.one, status);
+    return;
+  }
   if ((size_t)blockIdx.x * kVicCols >= ncol) return;  // the whole warp
   const int lane = threadIdx.x, g = lane / kVicLanes, q = lane % kVicLanes;
   const size_t col = (size_t)blockIdx.x * kVicCols + g;

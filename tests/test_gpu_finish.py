@@ -64,3 +64,21 @@ def test_members_of_different_lengths(oracle, cuda):
         for s in range(3):
             ob.stage(u, dt, s)
         close(ens.state(k).cpu().numpy(), u)
+
+
+@pytest.mark.parametrize("sizes", [[(100, 30), (30, 900)], [(7, 3), (6, 2600)],
+                                   [(64, 607)], [(64, 900)]])
+def test_both_forms_of_the_direct_solve(oracle, cuda, sizes):
+    """Few long columns (a warp each) and many short ones (four a warp), in
+    one launch and alone, few columns and past a warp's share."""
+    members = [options(a, b) for a, b in sizes]
+    ens = Ensemble([o for o, _ in members], device=cuda)
+    ens.initialize([w.to(cuda) for _, w in members], autotune=False)
+    dts = ens.max_time_step().clone()
+    ens.step(dts)
+    for k, ((o, w), dt) in enumerate(zip(members, dts.cpu().tolist())):
+        ob = oracle.block_from_options(o)
+        u = ob.initialize(w.numpy())
+        for s in range(3):
+            ob.stage(u, dt, s)
+        close(ens.state(k).cpu().numpy(), u)
