@@ -242,6 +242,7 @@ struct sg_handle {
   int line_seg = 0, line_ctas = 0;  // line_kernel's (plan_line)
   int fin_len = 0, fin_ctas = 0;  // the finish's schedule (plan_finish)
   int solve_ctas = 0;             // the direct solve's (plan_solve)
+  int asm_ctas[2] = {0, 0};       // the assembly's, FP64 and FP32
   bool implicit = false;
   int vic_kinds = 0;  // bit 0: a block with the full 5x5 matrix, bit 1: 3x3
   bool ref32 = false;  // an FP32 block under gravity: base_ref_kernel runs
@@ -675,6 +676,8 @@ int sg_autotune(sg_handle* h, int32_t reps, int32_t* tj_out,
     p.psw = h->psw_on;
     p.fallbacks = h->fallbacks;
     p.max_nc1 = h->max_nc1;
+    p.asm_ctas[0] = h->asm_ctas[0];
+    p.asm_ctas[1] = h->asm_ctas[1];
     p.solve_ctas = h->solve_ctas;
     p.fin_len = h->fin_len;
     p.fin_ctas = h->fin_ctas;
@@ -1037,6 +1040,20 @@ int sg_create(const sg_scheme* scheme, const sg_block_desc* blocks,
     h->dv3_bytes.push_back(dv3_bytes);
     h->scratch_bytes.push_back(vic_bytes + dv3_bytes + sc_bytes);
     if (d.implicit_scheme) {
+      // the assembly's CTAs: runs of padded layers, two of each lent
+      const int cw = B.implicit_f32 ? sg::kAsmCols32 : 1;
+      const int rows = B.implicit_f32 ? sg::kAsmThreads32 / sg::kAsmCols32
+                                      : sg::kAsmThreads64;
+      const size_t run = ((icols + cw - 1) / cw) * (size_t)(d.nc1 - 2 * d.ng + 2);
+      int& ctas = h->asm_ctas[B.implicit_f32 ? 1 : 0];
+      ctas = std::max(ctas, (int)((run - 2 + rows - 3) / (rows - 2)));
+      const double gm1 = d.gammad - 1., gm1r = 0.5 * (d.gammad + d.gammad) - 1.;
+      B.asmc[0] = d.dx3 * (d.dx2 * d.dx1);
+      B.asmc[1] = 0.5 / B.asmc[0];
+      B.asmc[2] = 1. / B.asmc[0];
+      B.asmc[3] = (gm1 + 1.) / gm1;
+      B.asmc[4] = 1. / gm1r;
+      B.asmc[5] = 1. / (gm1r + 1.);
       h->max_icells = std::max(h->max_icells, icells);
       h->max_icols = std::max(h->max_icols, icols);
     }
@@ -1377,6 +1394,8 @@ int sg_stage(sg_handle* h, int32_t stage, const double* dt_dev,
   p.psw = h->psw_on;
   p.fallbacks = h->fallbacks;
   p.max_nc1 = h->max_nc1;
+  p.asm_ctas[0] = h->asm_ctas[0];
+  p.asm_ctas[1] = h->asm_ctas[1];
   p.solve_ctas = h->solve_ctas;
   p.fin_len = h->fin_len;
   p.fin_ctas = h->fin_ctas;

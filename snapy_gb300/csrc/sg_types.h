@@ -51,6 +51,10 @@ struct BlockDev {
   int32_t implicit;
   int32_t implicit_f32;  // implicit-precision float32: FP32 block assembly
   double* vic;
+  // the FP64 assembly's constants: V, 1 / 2V, 1 / V, gamma / (gamma - 1) from
+  // gm1 = gamma - 1 as (gm1 + 1) / gm1, and with gm1 the Roe average's the
+  // reciprocals of gm1 and gm1 + 1
+  double asmc[6];
   int32_t wsolve;  // the direct solve takes a warp per column (plan_solve)
   // the layer-parallel (partitioned) form of the scheme-9 solve of an
   // FP64-assembled block (sg_set_sweep): its region, per interior cell the
@@ -141,6 +145,10 @@ constexpr int kVicFloatsPerColumn = 7;
 // the most x1 cells of a line_kernel CTA (its shared memory is sized by it)
 constexpr int kLineMaxSeg = 64;
 
+// the implicit solve's assembly: padded cells of a CTA (FP64: of one column
+// after another; FP32: of kAsmCols32 columns side by side)
+constexpr int kAsmThreads64 = 128, kAsmThreads32 = 256, kAsmCols32 = 8;
+
 // the implicit solve's finish keeps kFinArrays arrays of `len` doubles a CTA
 // (kFinPartial more for the partial matrix): a column's pitch in them (n + 1
 // values, odd), and the columns that fit (sg_create gives len at least one)
@@ -184,6 +192,7 @@ struct StageParams {
                         // staging wait ran out)
   int32_t smem_rows;    // x1 lines held in shared memory per tile
   int32_t max_nc1;
+  int32_t asm_ctas[2];  // the assembly's CTAs per block: FP64, FP32
   int32_t solve_ctas;   // the direct solve's CTAs per block
   int32_t fin_len;      // doubles of a finish CTA's array
   int32_t fin_ctas;     // its CTAs per block

@@ -151,45 +151,37 @@ __device__ __forceinline__ void count_fp64_column(const StageParams& p, int b) {
   if (p.counts) atomicAdd(&p.counts[b * kCountSlots + kCountFp64Columns], 1ull);
 }
 
+// the flux Jacobian's entries that are not 0, 1, a velocity or gamma - 1:
+// (1,0) (1,1) (1,2) (1,3) (2,0) (3,0) (4,0) .. (4,4); gq = (gm1 + 1) / gm1
+constexpr int kJac = 11;
 template <typename T>
-__device__ __forceinline__ void vmat_mul(const T* a, const T* b,
-                                         T* out) {
-#pragma unroll
-  for (int r = 0; r < 5; ++r)
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-      T s = a[r * 5] * b[c];
-#pragma unroll
-      for (int k = 1; k < 5; ++k) s += a[r * 5 + k] * b[k * 5 + c];
-      out[r * 5 + c] = s;
-    }
-}
-
-template <typename T>
-__device__ __forceinline__ void vflux_jacobian(T* J, T gm1,
+__device__ __forceinline__ void vflux_jacobian(T (&J)[kJac], T gm1, T gq,
                                                const T* w) {
   T v1 = w[1], v2 = w[2], v3 = w[3], rho = w[0], pres = w[4];
   T s2 = v1 * v1 + v2 * v2 + v3 * v3;
-  T c1 = ((gm1 - 1) * s2 / 2 - (gm1 + 1) / gm1 * pres / rho) * v1;
-  T c2 = (gm1 + 1) / gm1 * pres / rho + s2 / 2 - gm1 * v1 * v1;
-  J[0] = 0; J[1] = T(1.); J[2] = T(0.); J[3] = T(0.); J[4] = T(0.);
-  J[5] = gm1 * s2 / 2 - v1 * v1; J[6] = (T(2.) - gm1) * v1; J[7] = -gm1 * v2;
-  J[8] = -gm1 * v3; J[9] = gm1;
-  J[10] = -v1 * v2; J[11] = v2; J[12] = v1; J[13] = T(0.); J[14] = T(0.);
-  J[15] = -v1 * v3; J[16] = v3; J[17] = T(0.); J[18] = v1; J[19] = T(0.);
-  J[20] = c1; J[21] = c2; J[22] = -gm1 * v2 * v1; J[23] = -gm1 * v3 * v1;
-  J[24] = (gm1 + 1) * v1;
+  const T e = gq * pres / rho;
+  J[0] = gm1 * s2 / 2 - v1 * v1;
+  J[1] = (T(2.) - gm1) * v1;
+  J[2] = -gm1 * v2;
+  J[3] = -gm1 * v3;
+  J[4] = -v1 * v2;
+  J[5] = -v1 * v3;
+  J[6] = ((gm1 - 1) * s2 / 2 - e) * v1;
+  J[7] = e + s2 / 2 - gm1 * v1 * v1;
+  J[8] = -gm1 * v2 * v1;
+  J[9] = -gm1 * v3 * v1;
+  J[10] = (gm1 + 1) * v1;
 }
 
 // |A| = R |Lambda| R^-1 at the face between wl and wr (Roe average)
 template <typename T>
-__device__ __forceinline__ void vabs_jacobian(T* A, T gm1,
-                                              const T* wl,
+__device__ __forceinline__ void vabs_jacobian(T (&A)[25], T gm1, T rgm1,
+                                              T rgp1, const T* wl,
                                               const T* wr) {
   // every quotient as written below; those sharing a divisor divide by
-  // its reciprocal (vdiv: the same bits), and 1 / (2 hp), -1 / hp are the
-  // reciprocals themselves
-  const T gp1 = gm1 + T(1.), rgm1 = T(1.) / gm1, rgp1 = T(1.) / gp1;
+  // its reciprocal (vdiv: the same bits; rgm1 = 1 / gm1, rgp1 = 1 / (gm1 +
+  // 1)), and 1 / (2 hp), -1 / hp are the reciprocals themselves
+  const T gp1 = gm1 + T(1.);
   T sqrtdl = sqrt(wl[0]), sqrtdr = sqrt(wr[0]);
   T isdlpdr = T(1.0) / (sqrtdl + sqrtdr);
   T pr[5];
@@ -213,34 +205,40 @@ __device__ __forceinline__ void vabs_jacobian(T* A, T gm1,
   T h = hp + ke;
   const T d1 = T(2.) * cs * hp, d2 = T(2.) * hp;
   const T r1 = T(1.) / d1, r2 = T(1.) / d2, rh = T(1.) / hp;
-  const T R[25] = {T(1.),         T(1.), T(1.),         T(0.), T(0.),  //
-                        u - cs,     u,  u + cs,     T(0.), T(0.),  //
-                        v,          v,  v,          T(1.), T(0.),  //
-                        w,          w,  w,          T(0.), T(1.),  //
-                        h - u * cs, ke, h + u * cs, v,  w};
-  const T Ri[25] = {vdiv(cs * ke + u * hp, d1, r1),
-                         vdiv(-hp - cs * u, d1, r1),
-                         vdiv(-v, d2, r2),
-                         vdiv(-w, d2, r2),
-                         r2,
-                         vdiv(hp - ke, hp, rh),
-                         vdiv(u, hp, rh),
-                         vdiv(v, hp, rh),
-                         vdiv(w, hp, rh),
-                         -rh,
-                         vdiv(cs * ke - u * hp, d1, r1),
-                         vdiv(hp - cs * u, d1, r1),
-                         vdiv(-v, d2, r2),
-                         vdiv(-w, d2, r2),
-                         r2,
-                         -v, T(0.), T(1.), T(0.), T(0.),
-                         -w, T(0.), T(0.), T(1.), T(0.)};
-  T RL[25];
+  // A = (R Lambda) R^-1 with the products of R's and R^-1's zeros left out
+  // (each sum's other terms in their order: R's first three columns are full,
+  // its fourth holds 1 and v in the last three rows, its fifth 1 and w; the
+  // last two rows of R^-1 are (-v, 0, 1, 0, 0) and (-w, 0, 0, 1, 0))
+  const T Ri[3][5] = {
+      {vdiv(cs * ke + u * hp, d1, r1), vdiv(-hp - cs * u, d1, r1),
+       vdiv(-v, d2, r2), vdiv(-w, d2, r2), r2},
+      {vdiv(hp - ke, hp, rh), vdiv(u, hp, rh), vdiv(v, hp, rh),
+       vdiv(w, hp, rh), -rh},
+      {vdiv(cs * ke - u * hp, d1, r1), vdiv(hp - cs * u, d1, r1),
+       vdiv(-v, d2, r2), vdiv(-w, d2, r2), r2}};
+  const T R[5][3] = {{lam[0], lam[1], lam[2]},
+                     {(u - cs) * lam[0], u * lam[1], (u + cs) * lam[2]},
+                     {v * lam[0], v * lam[1], v * lam[2]},
+                     {w * lam[0], w * lam[1], w * lam[2]},
+                     {(h - u * cs) * lam[0], ke * lam[1], (h + u * cs) * lam[2]}};
 #pragma unroll
   for (int i = 0; i < 5; ++i)
 #pragma unroll
-    for (int k = 0; k < 5; ++k) RL[i * 5 + k] = R[i * 5 + k] * lam[k];
-  vmat_mul(RL, Ri, A);
+    for (int c = 0; c < 5; ++c) {
+      T s = R[i][0] * Ri[0][c];
+      s += R[i][1] * Ri[1][c];
+      s += R[i][2] * Ri[2][c];
+      A[i * 5 + c] = s;
+    }
+  const T l3 = lam[3], vl = v * lam[3], wl4 = w * lam[4];
+  A[10] += l3 * -v;
+  A[12] += l3;
+  A[15] += lam[4] * -w;
+  A[18] += lam[4];
+  A[20] += vl * -v;
+  A[20] += wl4 * -w;
+  A[22] += vl;
+  A[23] += wl4;
 }
 
 // the primitives of a cell (u of the storage type -> FP64 W); an FP32
@@ -323,108 +321,129 @@ __device__ __forceinline__ VicK vic_krows(const BlockDev& B, int n, int k) {
 // state's blocks, exact in FP32 and in the FP64 copies the residuals of the
 // refined solve read).  The FP64 instantiation performs the reference's
 // operations in its order.
-// a block's constants of the assembly in the compute type, formed once per
-// launch (the cell loop reloads what it reads from the block table)
+#ifndef SG_ASM32_CTAS
+#define SG_ASM32_CTAS 3
+#endif
+#ifndef SG_ASM64_CTAS
+#define SG_ASM64_CTAS 3
+#endif
+// the assembly's CTA: columns side by side, threads, CTAs an SM (the register
+// budget it is held to), and its shared arrays
+template <typename T>
+struct AsmShape {
+  static constexpr bool f32 = sizeof(T) == sizeof(float);
+  static constexpr int cw = f32 ? kAsmCols32 : 1;
+  static constexpr int threads = f32 ? kAsmThreads32 : kAsmThreads64;
+  static constexpr int ctas = f32 ? SG_ASM32_CTAS : SG_ASM64_CTAS;
+};
+template <typename T>
+struct AsmSmem {
+  T W[5][AsmShape<T>::threads], J[kJac][AsmShape<T>::threads],
+      A[25][AsmShape<T>::threads];
+};
+
+// a block's constants of the assembly in the compute type (in FP64 those
+// without dt come from the table, BlockDev::asmc)
 template <typename T>
 struct AsmConst {
-  T grav, gm1, gm1r, area, vol, half_inv_vol, rvol, rdt, dtc, gammad;
-  __device__ AsmConst(const BlockDev& B, double dtc_) {
-    gammad = T(B.gammad);
+  T grav, gm1, gm1r, area, vol, half_inv_vol, rvol, rdt, dtc, gq, rgm1, rgp1;
+  __device__ AsmConst(const BlockDev& B, double dtc_, double rdtc) {
     grav = T(B.grav1);
     gm1 = T(B.gammad - 1.);
     gm1r = T(0.5 * (B.gammad + B.gammad) - 1.);
     area = T(B.dx3 * B.dx2);
-    vol = T(B.dx3 * (B.dx2 * B.dx1));
-    half_inv_vol = T(0.5) / vol;
-    rvol = T(1.) / vol;
+    vol = T(B.asmc[0]);
     dtc = T(dtc_);
-    rdt = T(1.) / dtc;
+    if constexpr (sizeof(T) == sizeof(float)) {
+      half_inv_vol = T(0.5) / vol;
+      rvol = T(1.) / vol;
+      rdt = T(1.) / dtc;
+      gq = (gm1 + T(1.)) / gm1;
+      rgm1 = T(1.) / gm1r;
+      rgp1 = T(1.) / (gm1r + T(1.));
+    } else {
+      half_inv_vol = B.asmc[1];
+      rvol = B.asmc[2];
+      rdt = rdtc;
+      gq = B.asmc[3];
+      rgm1 = B.asmc[4];
+      rgp1 = B.asmc[5];
+    }
   }
 };
 
 template <typename T>
-__device__ __forceinline__ void vic_assemble_cell(const BlockDev& B,
-                                                  const VicScratch& S,
-                                                  const real* uin,
-                                                  double dtc, double rdtc,
-                                                  size_t e, bool f32copy,
-                                                  const AsmConst<T>& kc) {
-  const int ng = B.ng, nc1 = B.nc1, n = nc1 - 2 * ng;
-  const size_t plane = (size_t)nc1 * B.nc2 * B.nc3;
+__device__ __forceinline__ void vic_assemble_cell(
+    const BlockDev& B, const VicScratch& S, double dtc, double rdtc, size_t col,
+    int i, bool f32copy, const AsmConst<T>& kc, const AsmSmem<T>& sm, int t) {
+  constexpr int cw = AsmShape<T>::cw;
+  const int ng = B.ng, n = B.nc1 - 2 * ng;
   const T grav = kc.grav, gm1 = kc.gm1;
   const T area = kc.area, vol = kc.vol;
   const double* x1v = B.x1v + ng;
   const double* x1f = B.x1f + ng;
   const bool wood = n >= 3;
-  const int i = (int)(e % n);
-  const size_t col = e / n;
-  const size_t jrow = vic_row(B, col);
-  const size_t base = jrow * nc1 + ng;  // padded cell of layer 0
-  T wl[5], wr[5], wn[5];
-  if constexpr (sizeof(T) == sizeof(float)) {
-    // FP32 assembly: the primitives in FP32 from the FP32 state and the
-    // base rounded to FP32 (the blocks are FP32 either way)
-    vic_prim32(uin, plane, base + i - 1, kc.gammad, wl, B.base, nc1);
-    vic_prim32(uin, plane, base + i, kc.gammad, wr, B.base, nc1);
-    vic_prim32(uin, plane, base + i + 1, kc.gammad, wn, B.base, nc1);
-  } else {
-    double wd[3][5];
-    vic_prim(uin, plane, base + i - 1, B.gammad, wd[0], B.base, nc1);
-    vic_prim(uin, plane, base + i, B.gammad, wd[1], B.base, nc1);
-    vic_prim(uin, plane, base + i + 1, B.gammad, wd[2], B.base, nc1);
-#pragma unroll
-    for (int v = 0; v < 5; ++v) {
-      wl[v] = T(wd[0][v]);
-      wr[v] = T(wd[1][v]);
-      wn[v] = T(wd[2][v]);
-    }
-  }
-  T Jp[25], Jc[25], Jn[25], Am[25], Ap[25];
-  const T gm1r = kc.gm1r;
-  vflux_jacobian(Jp, gm1, wl);
-  vflux_jacobian(Jc, gm1, wr);
-  vabs_jacobian(Am, gm1r, wl, wr);
-  vflux_jacobian(Jn, gm1, wn);
-  vabs_jacobian(Ap, gm1r, wr, wn);
   const T half_inv_vol = kc.half_inv_vol;
   const T rvol = kc.rvol;
   const T lower = vdiv(T(0.5) * area * as_real<T>(x1v[i] - x1f[i]), vol, rvol);
   const T upper = vdiv(T(0.5) * area * as_real<T>(x1f[i + 1] - x1v[i]), vol, rvol);
-  T a[25], b[25], c_[25];
-#pragma unroll
-  for (int r = 0; r < 5; ++r)
-#pragma unroll
-    for (int q = 0; q < 5; ++q) {
-      const int k = r * 5 + q;
-      T phi = (r == 1 && q == 0) || (r == 4 && q == 1) ? grav : T(0.);
-      a[k] = (Am[k] * area + Ap[k] * area + (area - area) * Jc[k]) *
-                 half_inv_vol - phi;
-      b[k] = -(Am[k] + Jp[k]) * area * half_inv_vol;
-      c_[k] = -(Ap[k] - Jn[k]) * area * half_inv_vol;
-    }
-  const T rdt = kc.rdt;
-#pragma unroll
-  for (int r = 0; r < 5; ++r) a[r * 5 + r] += rdt;
-#pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    a[20 + k] -= grav * (upper * Ap[k] - lower * Am[k]);
-    b[20 + k] -= grav * lower * Am[k];
-    c_[20 + k] += grav * upper * Ap[k];
+  const int tl = t - cw, th = t + cw;
+  const T rdt = kc.rdt, gl = grav * lower, gu = grav * upper;
+  const bool partial = B.implicit == 1;
+  // the K rows over dt_corr (the partial matrix adds its own below)
+  T kmid = T(0.), klo = T(0.), khi = T(0.);
+  const VicK K = wood ? vic_krows(B, n, i) : VicK{};
+  if (wood && !partial) {
+    kmid = vdiv(as_real<T>(K.mid), kc.dtc, rdt);
+    klo = vdiv(as_real<T>(K.lo), kc.dtc, rdt);
+    khi = vdiv(as_real<T>(K.hi), kc.dtc, rdt);
   }
-  a[21] += grav * (T(1.) - lower - upper);
-  b[21] -= grav * lower;
-  c_[21] -= grav * upper;
-  const T bnd[5] = {T(1.), T(-1.), T(1.), T(1.), T(1.)};
-  if (i == 0)
-#pragma unroll
-    for (int r = 0; r < 5; ++r)
-#pragma unroll
-      for (int q = 0; q < 5; ++q) a[r * 5 + q] += b[r * 5 + q] * bnd[q];
-  if (i == n - 1)
-#pragma unroll
-    for (int r = 0; r < 5; ++r)
-#pragma unroll
-      for (int q = 0; q < 5; ++q) a[r * 5 + q] += c_[r * 5 + q] * bnd[q];
+  // entry k (a compile-time constant where these are called): the |A| of the
+  // faces below and above, and what the flux Jacobian of the cell at x adds
+  // (its zeros left out)
+  auto am = [&](int k) -> T { return sm.A[k][tl]; };
+  auto ap = [&](int k) -> T { return sm.A[k][t]; };
+  auto jac = [&](int k, int x, T v, T sign) -> T {
+    if (k == 1) return v + sign;
+    if (k >= 5 && k <= 8) return v + sign * sm.J[k - 5][x];
+    if (k == 9) return v + sign * gm1;
+    if (k == 10) return v + sign * sm.J[4][x];
+    if (k == 11) return v + sign * sm.W[2][x];
+    if (k == 12 || k == 18) return v + sign * sm.W[1][x];
+    if (k == 15) return v + sign * sm.J[5][x];
+    if (k == 16) return v + sign * sm.W[3][x];
+    if (k >= 20) return v + sign * sm.J[k - 14][x];
+    return v;
+  };
+  // b = -(|A-| + J-) A / 2V, c = -(|A+| - J+) A / 2V, and a = (|A-| + |A+|)
+  // A / 2V - Phi + 1 / dt, with the energy row's face work, the walls' mirror
+  // (m1 flips) and the K rows
+  auto bval = [&](int k) -> T {
+    T v = -jac(k, tl, am(k), T(1.)) * area * half_inv_vol;
+    if (k >= 20) v -= gl * am(k - 20);
+    if (k == 21) v -= gl;
+    if (k == 20) v -= klo;
+    return v;
+  };
+  auto cval = [&](int k) -> T {
+    T v = -jac(k, th, ap(k), T(-1.)) * area * half_inv_vol;
+    if (k >= 20) v += gu * ap(k - 20);
+    if (k == 21) v -= gu;
+    if (k == 20) v -= khi;
+    return v;
+  };
+  auto aval = [&](int k, T bw, T cw_) -> T {  // bw, cw_: b and c
+    T v = (am(k) * area + ap(k) * area) * half_inv_vol;
+    if (k == 5 || k == 21) v -= grav;
+    if (k % 6 == 0) v += rdt;
+    if (k >= 20) v -= grav * (upper * ap(k - 20) - lower * am(k - 20));
+    if (k == 21) v += grav * (T(1.) - lower - upper);
+    const T flip = k % 5 == 1 ? T(-1.) : T(1.);
+    if (i == 0) v += bw * flip;
+    if (i == n - 1) v += cw_ * flip;
+    if (k == 20) v -= kmid;
+    return v;
+  };
   const size_t cell = col * n + i;
   double du0[5];
 #pragma unroll
@@ -441,56 +460,7 @@ __device__ __forceinline__ void vic_assemble_cell(const BlockDev& B,
   // and into the right-hand side at the frozen remainder
   // q_t = du[m_t] - v_t du[rho] (src/implicit/vic_assemble_impl.h:152-214);
   // the neighbours' folds are skipped at the merged walls
-  const bool partial = B.implicit == 1;
-  T a3[9], b3[9], c3[9], rc[3] = {T(0.), T(0.), T(0.)};
-  if (partial) {
-    const int rows[3] = {0, 1, 4};
-    T aT[6], bT[6], cT[6];
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        a3[r * 3 + q] = a[rows[r] * 5 + rows[q]];
-        b3[r * 3 + q] = b[rows[r] * 5 + rows[q]];
-        c3[r * 3 + q] = c_[rows[r] * 5 + rows[q]];
-      }
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        aT[r * 2 + k] = a[rows[r] * 5 + 2 + k];
-        bT[r * 2 + k] = b[rows[r] * 5 + 2 + k];
-        cT[r * 2 + k] = c_[rows[r] * 5 + 2 + k];
-      }
-    }
-    auto fold = [&](T* blk, const T* tb, int j, const T* wj) {
-      const double* dj = S.du + col * n + j;  // row v at dj[v * cells]
-      const T drho = T(dj[0]);
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const T v = wj[2 + k];
-        const T qt = T(dj[(size_t)(2 + k) * S.cells]) - v * drho;
-        if (v != T(0.))
-#pragma unroll
-          for (int r = 0; r < 3; ++r) blk[r * 3] = blk[r * 3] + tb[r * 2 + k] * v;
-        if (qt != T(0.))
-#pragma unroll
-          for (int r = 0; r < 3; ++r) rc[r] = rc[r] + tb[r * 2 + k] * qt;
-      }
-    };
-    fold(a3, aT, i, wr);
-    if (i > 0) fold(b3, bT, i - 1, wl);
-    if (i < n - 1) fold(c3, cT, i + 1, wn);
-  }
   if (wood) {
-    VicK K = vic_krows(B, n, i);
-    if (partial) {
-      a3[6] -= vdiv(as_real<T>(K.mid), kc.dtc, rdt);
-      b3[6] -= vdiv(as_real<T>(K.lo), kc.dtc, rdt);
-      c3[6] -= vdiv(as_real<T>(K.hi), kc.dtc, rdt);
-    } else {
-      a[20] -= vdiv(as_real<T>(K.mid), kc.dtc, rdt);
-      b[20] -= vdiv(as_real<T>(K.lo), kc.dtc, rdt);
-      c_[20] -= vdiv(as_real<T>(K.hi), kc.dtc, rdt);
-    }
     // du[IPR] -= (K du0[IDN])_i : the IDN row is read only (FP64 always)
     const double* dn = S.du + col * n;
     double s = K.mid * dn[i];
@@ -502,6 +472,48 @@ __device__ __forceinline__ void vic_assemble_cell(const BlockDev& B,
     S.du[4 * S.cells + cell] = du4;
   }
   if (partial) {
+    const int rows[3] = {0, 1, 4};
+    T a3[9], b3[9], c3[9], rc[3] = {T(0.), T(0.), T(0.)}, aT[6], bT[6], cT[6];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const int k = rows[r] * 5 + rows[q];
+        b3[r * 3 + q] = bval(k);
+        c3[r * 3 + q] = cval(k);
+        a3[r * 3 + q] = aval(k, b3[r * 3 + q], c3[r * 3 + q]);
+      }
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int e = rows[r] * 5 + 2 + k;
+        bT[r * 2 + k] = bval(e);
+        cT[r * 2 + k] = cval(e);
+        aT[r * 2 + k] = aval(e, bT[r * 2 + k], cT[r * 2 + k]);
+      }
+    }
+    auto fold = [&](T* blk, const T* tb, int j, int x) {
+      const double* dj = S.du + col * n + j;  // row v at dj[v * cells]
+      const T drho = T(dj[0]);
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const T v = sm.W[2 + k][x];
+        const T qt = T(dj[(size_t)(2 + k) * S.cells]) - v * drho;
+        if (v != T(0.))
+#pragma unroll
+          for (int r = 0; r < 3; ++r) blk[r * 3] = blk[r * 3] + tb[r * 2 + k] * v;
+        if (qt != T(0.))
+#pragma unroll
+          for (int r = 0; r < 3; ++r) rc[r] = rc[r] + tb[r * 2 + k] * qt;
+      }
+    };
+    fold(a3, aT, i, t);
+    if (i > 0) fold(b3, bT, i - 1, tl);
+    if (i < n - 1) fold(c3, cT, i + 1, th);
+    if (wood) {
+      a3[6] -= vdiv(as_real<T>(K.mid), kc.dtc, rdt);
+      b3[6] -= vdiv(as_real<T>(K.lo), kc.dtc, rdt);
+      c3[6] -= vdiv(as_real<T>(K.hi), kc.dtc, rdt);
+    }
     // a cell's row of 25: the 3x3 block, row-major, then (A only) the
     // right-hand-side term of the fold
 #pragma unroll
@@ -514,19 +526,17 @@ __device__ __forceinline__ void vic_assemble_cell(const BlockDev& B,
     for (int r = 0; r < 3; ++r) S.A[cell * 25 + 9 + r] = (double)rc[r];
     return;
   }
-  // the FP64 blocks, unless the refined solve reads the FP32 ones (exact:
-  // its residuals and the masked columns' direct solve widen them)
-  if (!(sizeof(T) == sizeof(float) && f32copy)) {
+  T a[25], b[25], c_[25];
 #pragma unroll
-    for (int k = 0; k < 25; ++k) {
-      S.A[cell * 25 + k] = (double)a[k];
-      S.B[cell * 25 + k] = (double)b[k];
-      S.C[cell * 25 + k] = (double)c_[k];
-    }
+  for (int k = 0; k < 25; ++k) {
+    b[k] = bval(k);
+    c_[k] = cval(k);
+    a[k] = aval(k, b[k], c_[k]);
   }
   if (sizeof(T) == sizeof(float) && f32copy) {
-    // the refined solve's tiles: the blocks, and the right-hand side du /
-    // dt_corr in FP64 (its residuals') and in FP32 (its first sweep's)
+    // the refined solve's tiles: the blocks in FP32 (exact: its residuals and
+    // the masked columns' direct solve widen them), and the right-hand side du
+    // / dt_corr in FP64 (its residuals') and in FP32 (its first sweep's)
     const VicScratch32 F = vic_scratch32(B, S, n);
     const size_t tile = col >> 5, c = col & 31;
     const int w = VicTile::width(F.ncol, tile);
@@ -546,48 +556,86 @@ __device__ __forceinline__ void vic_assemble_cell(const BlockDev& B,
       pd[(size_t)v * w] = q;
       pr[(size_t)v * w] = narrow_exact(q);
     }
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < 25; ++k) {
+    S.A[cell * 25 + k] = (double)a[k];
+    S.B[cell * 25 + k] = (double)b[k];
+    S.C[cell * 25 + k] = (double)c_[k];
   }
 }
 
-// CTAs of the FP32 assembly resident per SM (the register budget it is held
-// to: 65536 / (256 kAsm32Ctas))
-#ifndef SG_ASM32_CTAS
-#define SG_ASM32_CTAS 2
-#endif
-constexpr int kAsm32Ctas = SG_ASM32_CTAS;
-
-// the assembly in the compute type T: the FP64 and FP32 forms are separate
-// kernels, so the FP32 one is not held to the FP64 one's register count
+// The assembly, a CTA per run of padded layers of the columns taken one
+// after the other (each with the ghost below it and the one above), a thread
+// per padded cell: its primitives and Jacobian once, then the |A| of its upper
+// face once, then the blocks of its cell from its own and its neighbours'
+// values in shared memory.  A CTA's first and last layers are the next ones'
+// too (they lend their values), so no column length leaves threads idle.  FP64
+// runs take one column, 128 cells; FP32 runs take eight columns by 32 layers,
+// so a warp's stores to the refined solve's tiles fill 32-byte sectors.
+//
+// Bound by the FP64 pipe in FP64 (about 700 instructions a cell; a thread
+// that assembled its cell alone took 1280: three cells' primitives, two
+// Jacobians, both faces' |A|, the zeros' products), by its loads and stores
+// in FP32.  Measured per launch (us), before and now: 512 x 128 FP64 212 / 125,
+// 45 x 37 x 48 319 / 151, 301 x 75 108 / 64, nine members 330 / 210; FP32 64
+// members 418 / 305, four served requests 738 / 690 (two CTAs an SM: 374 and
+// 874; a branch per store to either layout: 488 and 1155).
 template <typename T>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == sizeof(float) ? kAsm32Ctas : 1)
+__global__ void __launch_bounds__(AsmShape<T>::threads, AsmShape<T>::ctas)
     vic_assemble_kernel(const BlockDev* __restrict__ tab, StageParams p) {
+  constexpr int cw = AsmShape<T>::cw, rows = AsmShape<T>::threads / cw;
+  __shared__ AsmSmem<T> sm;
   const BlockDev& B = tab[blockIdx.y];
   if (!B.implicit || (B.implicit_f32 != 0) != (sizeof(T) == sizeof(float)))
     return;
+  const int nc1 = B.nc1, n = nc1 - 2 * B.ng;
   const VicScratch S = vic_scratch(B);
-  const real* uin = static_cast<const real*>(B.buf[p.in]);
+  const size_t ncol = S.cells / n, run = ((ncol + cw - 1) / cw) * (n + 2);
+  const size_t first = (size_t)blockIdx.x * (rows - 2);
+  if (first + 2 >= run) return;
+  const int t = threadIdx.x, row = t / cw;
+  const size_t at = first + row, g = at / (n + 2);
+  const int i = (int)(at - g * (n + 2)) - 1;  // -1: the ghost below, n: above
+  const size_t col = g * cw + t % cw;
+  const bool on = at < run && col < ncol;
   const double dtc = p.w2 * p.dt[blockIdx.y];
   const double rdtc = 1. / dtc;
-  const AsmConst<T> kc(B, dtc);
-  const int n = B.nc1 - 2 * B.ng;
-  if (sizeof(T) == sizeof(float) && p.refine != 0 && B.implicit == 9) {
-    // the refined solve's tiles: a CTA takes 32 columns by 8 layers, a warp
-    // 8 columns by 4 layers, so a store fills 32-byte sectors of a tile's
-    // row (8 columns) and a load of the state reads 4 consecutive layers
-    const size_t ncol = S.cells / n;
-    const size_t lg = (n + 7) / 8, units = ((ncol + 31) / 32) * lg;
-    const int wq = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (size_t q = blockIdx.x; q < units; q += gridDim.x) {
-      const size_t col = 32 * (q / lg) + 8 * (wq & 3) + (lane & 7);
-      const int i = 8 * (int)(q % lg) + 4 * (wq >> 2) + (lane >> 3);
-      if (col < ncol && i < n)
-        vic_assemble_cell<T>(B, S, uin, dtc, rdtc, col * n + i, true, kc);
+  const AsmConst<T> kc(B, dtc, rdtc);
+  T w[5];
+  if (on) {
+    const real* uin = static_cast<const real*>(B.buf[p.in]);
+    const size_t plane = (size_t)nc1 * B.nc2 * B.nc3;
+    const size_t cell = vic_row(B, col) * nc1 + B.ng + i;
+    if constexpr (sizeof(T) == sizeof(float)) {
+      // FP32 assembly: the primitives in FP32 from the FP32 state and the
+      // base rounded to FP32 (the blocks are FP32 either way)
+      vic_prim32(uin, plane, cell, (float)B.gammad, w, B.base, nc1);
+    } else {
+      vic_prim(uin, plane, cell, B.gammad, w, B.base, nc1);
     }
-    return;
+    T J[kJac];
+    vflux_jacobian(J, kc.gm1, kc.gq, w);
+#pragma unroll
+    for (int k = 0; k < 5; ++k) sm.W[k][t] = w[k];
+#pragma unroll
+    for (int k = 0; k < kJac; ++k) sm.J[k][t] = J[k];
   }
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < S.cells;
-       e += (size_t)gridDim.x * blockDim.x)
-    vic_assemble_cell<T>(B, S, uin, dtc, rdtc, e, false, kc);
+  __syncthreads();
+  if (on && i < n && row < rows - 1) {
+    T A[25], wn[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) wn[k] = sm.W[k][t + cw];
+    vabs_jacobian(A, kc.gm1r, kc.rgm1, kc.rgp1, w, wn);
+#pragma unroll
+    for (int k = 0; k < 25; ++k) sm.A[k][t] = A[k];
+  }
+  __syncthreads();
+  if (on && i >= 0 && i < n && row > 0 && row < rows - 1)
+    vic_assemble_cell<T>(B, S, dtc, rdtc, col, i,
+                         sizeof(T) == sizeof(float) && p.refine != 0 && B.implicit == 9,
+                         kc, sm, t);
 }
 
 // ludcmp<double, 5, Implicit> on a row-major 5x5 in shared memory
