@@ -22,6 +22,8 @@ using sg::StageParams;
 #define SG_DECLARE(sfx)                                                        \
   extern "C" size_t sg_stage_smem##sfx(int nc1, int tj, int has2, int wb,      \
                                        int cov, int visc);                     \
+  extern "C" size_t sg_stage_bound##sfx(int nc1, int tj, int has2, int wb,     \
+                                        int cov, int visc);                    \
   extern "C" int sg_launch_stage##sfx(const BlockDev*, StageParams, size_t,    \
                                       cudaStream_t);                           \
   extern "C" int sg_launch_ghost##sfx(const BlockDev*, int, int, size_t,       \
@@ -284,11 +286,13 @@ namespace {
 
 bool f64(const sg_handle* h) { return h->scheme.dtype == SG_F64; }
 
-size_t stage_smem(const sg_handle* h, const sg_block_desc& d, int tj) {
+size_t stage_smem(const sg_handle* h, const sg_block_desc& d, int tj,
+                  bool bound = false) {
   int has2 = d.nc2 > 1, wb = d.grav1 != 0., cov = d.flux_cov && d.nc1 >= 3;
   int visc = d.nu_iso > 0.;
-  return f64(h) ? sg_stage_smem_f64(d.nc1, tj, has2, wb, cov, visc)
-                : sg_stage_smem_f32(d.nc1, tj, has2, wb, cov, visc);
+  auto f = f64(h) ? (bound ? sg_stage_bound_f64 : sg_stage_smem_f64)
+                  : (bound ? sg_stage_bound_f32 : sg_stage_smem_f32);
+  return f(d.nc1, tj, has2, wb, cov, visc);
 }
 
 // tile width: enough CTAs to cover the SMs, shared memory within one CTA's
@@ -1000,13 +1004,15 @@ int sg_create(const sg_scheme* scheme, const sg_block_desc* blocks,
     if (d.nc3 > 1) h->has3 = true;
     B.tile0 = tile;
     tile += B.ntile;
-    size_t sm = stage_smem(h, d, B.tj);
+    // (a tile is refused by the size of its regions laid apart)
+    size_t sm = stage_smem(h, d, B.tj, true);
     if ((long)sm > optin) {
       sg_destroy(h);
       return fail(SG_ERR_UNSUPPORTED,
                   "block %d: a tile needs %zu B of shared memory (limit %d)",
                   b, sm, optin);
     }
+    sm = stage_smem(h, d, B.tj);
     h->smem = std::max(h->smem, sm);
     size_t plane = (size_t)d.nc1 * d.nc2 * d.nc3;
     h->max_plane = std::max(h->max_plane, plane);

@@ -160,11 +160,17 @@ __device__ __forceinline__ void riemann(const real* wl, const real* wr,
 
 // smem layout of a tile (counts in `real`), shared by the kernel and the
 // host-side size query
+// (what is read last before another region is first written shares its
+// place, so more CTAs fit an SM: a tile of 4 columns of 128 in FP32 109 KB
+// apart and 78 KB so, of 3 columns 82 and 64.  With the FP64 scan cut to its
+// additions, per launch (us): 64 members FP32 449 and 372, four served requests
+// 824 and 722; FP64 512 x 128 277 and 261, 301 x 75 111 and 101)
 struct TileLayout {
   int R, ntj, nc1, nx1;
   bool has2, wb, cov, visc;
   int w, f1, f2, ref, pert, cov_arr, divv, vf1, vf2;  // offsets
   int total;
+  int bound;  // what sg_create holds against the limit: the regions apart
   __host__ __device__ TileLayout(int ntj_, int nc1_, int ng, bool has2_,
                                  bool wb_, bool cov_, bool visc_)
       : ntj(ntj_), nc1(nc1_), has2(has2_), wb(wb_), cov(cov_ && has2_),
@@ -179,23 +185,36 @@ struct TileLayout {
     o += NHYDRO * ntj * (nx1 + 1);
     f2 = o;
     o += has2 ? NHYDRO * (ntj + 1) * nx1 : 0;
-    // psf_lo, psf_hi, pref, dref, dsf_l, dsf_r, rho/p per tile row, FP64 in
-    // both builds (the FP32 build keeps the hydrostatic reference in FP64)
     constexpr int kDw = (int)(sizeof(double) / sizeof(real));
-    o += (o % kDw) ? kDw - (o % kDw) : 0;
+    int b = o + ((o % kDw) ? kDw - (o % kDw) : 0) + (wb ? 7 * ntj * nc1 * kDw : 0);
+    // per tile column the face pressures [nc1 + 1], pref, dref, dsf_l, dsf_r
+    // and rho/p (FP32: each [nc1 + 1], the anomaly form)
     ref = o;
-    o += wb ? 7 * ntj * nc1 * kDw : 0;
+    o += wb ? ntj * (sizeof(real) == sizeof(double) ? 6 * nc1 + 1 : 6 * (nc1 + 1)) : 0;
     pert = o;  // the reconstructed perturbations of p and rho per cell
     o += wb ? 2 * ntj * nc1 : 0;
+    const int refend = o;
     cov_arr = o;  // rho, h, un of the x2 face means, x1 rows 0..nc1-1
     o += cov ? 3 * (ntj + 1) * nc1 : 0;
     divv = o;  // div v on tile rows -1..ntj, all x1 cells
     o += visc ? (ntj + 2) * nc1 : 0;
-    vf1 = o;  // viscous momentum fluxes, x1 faces
-    o += visc ? 3 * ntj * (nx1 + 1) : 0;
-    vf2 = o;  // viscous momentum fluxes, x2 faces
-    o += (visc && has2) ? 3 * (ntj + 1) * nx1 : 0;
+    // the viscous momentum fluxes of the x1 and x2 faces take the place of
+    // the reference and the perturbations, which the x1 faces read last,
+    // where they fit there
+    const int n1 = visc ? 3 * ntj * (nx1 + 1) : 0;
+    const int n2 = visc && has2 ? 3 * (ntj + 1) * nx1 : 0;
+    b += (wb ? 2 * ntj * nc1 : 0) + (o - refend) + n1 + n2;
+    if (ref + n1 + n2 <= refend) {
+      vf1 = ref;
+      vf2 = ref + n1;
+    } else {
+      vf1 = o;
+      o += n1;
+      vf2 = o;
+      o += n2;
+    }
     total = o;
+    bound = b;
   }
 };
 
@@ -211,28 +230,35 @@ __device__ __forceinline__ double col_p(const real* pres, const double* pb,
 }
 
 #ifndef SG_REAL_IS_FLOAT
-__device__ __forceinline__ void ref_scan(const real* rho, const real* pres,
-                                         const double* pb, int nc1, int iu,
-                                         double dx, double grav,
-                                         double* psf_lo, double* psf_hi) {
-  const double minp = 2.2250738585072014e-308;
-  double rdt_top = col_p(pres, pb, iu) / as_f64(rho[iu]);
-  double top = col_p(pres, pb, iu) * sg_exp(-grav * 0.5 * dx / rdt_top);
+// the face pressures PF [nc1 + 1] of a column, face f below cell f, from the
+// pressure steps grav rho dx of its cells, which PF[0 .. nc1 - 1] holds
+// before.  The serial scan is the tile's longest chain on the FP64 pipe (64
+// cycles an instruction, one lane's worth of work), so it keeps the addition
+// of each cell alone: the steps are formed by all threads before, and the
+// floor is compared on the bit patterns (a NaN takes the floor, as it
+// compares false)
+__device__ __forceinline__ void ref_scan(double* PF, double rdt_top,
+                                         double ptop, int nc1, int iu,
+                                         double dx, double grav) {
+  auto floored = [](double x) -> double {
+    const double minp = 2.2250738585072014e-308;
+    const long long b = __double_as_longlong(x);
+    return b > __double_as_longlong(minp) && b <= 0x7ff0000000000000ll ? x : minp;
+  };
+  const double top = ptop * sg_exp(-grav * 0.5 * dx / rdt_top);
   double face = top;
+  double up = PF[iu + 1];  // the step of the cell above the top face
+  PF[iu + 1] = floored(top);
+#pragma unroll 4
   for (int i = iu; i >= 0; --i) {
-    double dp = grav * as_f64(rho[i]) * dx;
-    double lo = face + dp, hi = face;
-    psf_lo[i] = lo > minp ? lo : minp;
-    psf_hi[i] = hi > minp ? hi : minp;
-    face = lo;
+    face = face + PF[i];
+    PF[i] = floored(face);
   }
   face = top;
   for (int i = iu + 1; i < nc1; ++i) {
-    double dp = grav * as_f64(rho[i]) * dx;
-    double lo = face, hi = lo - dp;
-    psf_lo[i] = lo > minp ? lo : minp;
-    psf_hi[i] = hi > minp ? hi : minp;
-    face = hi;
+    face = face - up;
+    up = i + 1 < nc1 ? PF[i + 1] : 0.;
+    PF[i + 1] = floored(face);
   }
 }
 
@@ -649,7 +675,6 @@ __device__ __forceinline__ bool stage_tile(const BlockDev* __restrict__ tab,
   __syncthreads();
 
   // (2) the well-balanced x1 reference of each tile column
-  double* REF = reinterpret_cast<double*>(sm + L.ref);
   const int rs_ = ntj * nc1;  // one reference array of the tile
   const bool phys_in = B.bc[0] != kBcNone, phys_out = B.bc[1] != kBcNone;
   const int iu = nc1 - 1 - ng;
@@ -660,7 +685,7 @@ __device__ __forceinline__ bool stage_tile(const BlockDev* __restrict__ tab,
   // base, densities as totals), in the reference region as floats: per
   // column PFa [nc1 + 1] (face pressure - pf_b), rop, pref' (cell pressure
   // - p_b), dref, dsf_l, dsf_r
-  float* RF = reinterpret_cast<float*>(REF);
+  float* RF = sm + L.ref;
   const int cs1 = nc1 + 1, rsf = ntj * cs1;
   if (wb) {
     const float gdx = (float)(-B.grav1 * B.dx1);
@@ -787,38 +812,45 @@ __device__ __forceinline__ bool stage_tile(const BlockDev* __restrict__ tab,
     __syncthreads();
   }
 #else
+  // per column the face pressures PF [nc1 + 1]; per cell pref, dref, dsf_l,
+  // dsf_r and rho / p
+  double* PF = sm + L.ref;
+  const int cs1 = nc1 + 1;
+  double* REF = PF + ntj * cs1;
   if (wb) {
-    for (int jt = threadIdx.x; jt < ntj; jt += blockDim.x) {
-      const real* rho = W + IDN * wstride + (hj + jt) * nc1;
-      const real* pres = W + IPR * wstride + (hj + jt) * nc1;
-      ref_scan(rho, pres, pbc, nc1, iu, B.dx1, -B.grav1,
-               REF + 0 * rs_ + jt * nc1, REF + 1 * rs_ + jt * nc1);
-    }
-    // rho / p of every cell once (rop_smooth reads up to five per cell)
+    const double grav = -B.grav1, dx = B.dx1;
+    // the pressure step and rho / p of every cell once (rop_smooth reads up
+    // to five per cell)
     for (int idx = threadIdx.x; idx < ntj * nc1; idx += blockDim.x) {
       const int jt = idx / nc1, i = idx - jt * nc1;
-      const real* rho = W + IDN * wstride + (hj + jt) * nc1;
+      const double rho = W[IDN * wstride + (hj + jt) * nc1 + i];
       const real* pres = W + IPR * wstride + (hj + jt) * nc1;
-      REF[6 * rs_ + idx] = as_f64(rho[i]) / col_p(pres, pbc, i);
+      PF[jt * cs1 + i] = grav * rho * dx;
+      REF[4 * rs_ + idx] = rho / col_p(pres, pbc, i);
+    }
+    __syncthreads();
+    for (int jt = threadIdx.x; jt < ntj; jt += blockDim.x) {
+      const double rho = W[IDN * wstride + (hj + jt) * nc1 + iu];
+      const double ptop = col_p(W + IPR * wstride + (hj + jt) * nc1, pbc, iu);
+      ref_scan(PF + jt * cs1, ptop / rho, ptop, nc1, iu, dx, grav);
     }
     __syncthreads();
     for (int idx = threadIdx.x; idx < ntj * nc1; idx += blockDim.x) {
       const int jt = idx / nc1, i = idx - jt * nc1;
-      ref_cell(REF + 6 * rs_ + jt * nc1, REF + jt * nc1, REF + rs_ + jt * nc1,
-               i, nc1, iu, phys_in, phys_out, B.wb_wall_clamp != 0,
-               REF + 2 * rs_ + jt * nc1, REF + 3 * rs_ + jt * nc1,
-               REF + 4 * rs_ + jt * nc1 /* dsf, becomes dsf_l */);
+      ref_cell(REF + 4 * rs_ + jt * nc1, PF + jt * cs1, PF + jt * cs1 + 1, i, nc1,
+               iu, phys_in, phys_out, B.wb_wall_clamp != 0, REF + jt * nc1,
+               REF + rs_ + jt * nc1, REF + 2 * rs_ + jt * nc1 /* dsf, becomes dsf_l */);
     }
     __syncthreads();
     // dsf_lr: the cp5 row on dref guarded by the two cells' range; a
     // reflecting wall face takes the mean of its two sides.  Face f reads
-    // dsf[f] alone, so the ILT side overwrites dsf in place (slot 4); the
-    // IRT side goes to slot 5
+    // dsf[f] alone, so the ILT side overwrites dsf in place; the IRT side
+    // goes to the next slot
     for (int idx = threadIdx.x; idx < ntj * nc1; idx += blockDim.x) {
       const int jt = idx / nc1, f = idx - jt * nc1;
-      const double* dref = REF + 3 * rs_ + jt * nc1;
-      double* DL = REF + 4 * rs_ + jt * nc1;
-      double* DR = REF + 5 * rs_ + jt * nc1;
+      const double* dref = REF + 1 * rs_ + jt * nc1;
+      double* DL = REF + 2 * rs_ + jt * nc1;
+      double* DR = REF + 3 * rs_ + jt * nc1;
       double dsf = DL[f];
       double l = dsf, r = dsf;
       if (nc1 >= 6 && f >= 2 && f <= nc1 - 2) {
@@ -845,8 +877,8 @@ __device__ __forceinline__ bool stage_tile(const BlockDev* __restrict__ tab,
       // the perturbations the x1 reconstruction reads, once per cell
       const real* rho = W + IDN * wstride + (hj + jt) * nc1;
       const real* pres = W + IPR * wstride + (hj + jt) * nc1;
-      PP[idx] = real(col_p(pres, pbc, f) - REF[2 * rs_ + idx]);
-      PD[idx] = real(as_f64(rho[f]) - REF[3 * rs_ + idx]);
+      PP[idx] = real(col_p(pres, pbc, f) - REF[idx]);
+      PD[idx] = real(as_f64(rho[f]) - REF[rs_ + idx]);
     }
     __syncthreads();
   }
@@ -900,14 +932,14 @@ __device__ __forceinline__ bool stage_tile(const BlockDev* __restrict__ tab,
 #else
       // the totals in FP64; the Riemann solve takes the anomaly about the
       // base face pressure where there is a base
-      const double psf = REF[0 * rs_ + jt * nc1 + f];
+      const double psf = PF[jt * cs1 + f];
       double pl = as_f64(wl[IPR]) + psf, pr = as_f64(wr[IPR]) + psf;
       pl = pl > 0. ? pl : psf;
       pr = pr > 0. ? pr : psf;
       wl[IPR] = real(pbf ? pl - pbf[f] : pl);
       wr[IPR] = real(pbf ? pr - pbf[f] : pr);
-      real dl = real(as_f64(wl[IDN]) + REF[4 * rs_ + jt * nc1 + f]);
-      real dr = real(as_f64(wr[IDN]) + REF[5 * rs_ + jt * nc1 + f]);
+      real dl = real(as_f64(wl[IDN]) + REF[2 * rs_ + jt * nc1 + f]);
+      real dr = real(as_f64(wr[IDN]) + REF[3 * rs_ + jt * nc1 + f]);
 #endif
       const real* rho = W + IDN * wstride + (hj + jt) * nc1;
       wl[IDN] = dl > real(0) ? dl : rho[f > 0 ? f - 1 : 0];
@@ -2506,6 +2538,13 @@ extern "C" size_t SG_NAME(sg_stage_smem)(int nc1, int tj, int has2, int wb,
                                           int cov, int visc) {
   TileLayout L(tj, nc1, 3, has2 != 0, wb != 0, cov != 0, visc != 0);
   return (size_t)L.total * sizeof(real);
+}
+
+// what a tile of that size is held to at sg_create (TileLayout::bound)
+extern "C" size_t SG_NAME(sg_stage_bound)(int nc1, int tj, int has2, int wb,
+                                           int cov, int visc) {
+  TileLayout L(tj, nc1, 3, has2 != 0, wb != 0, cov != 0, visc != 0);
+  return (size_t)L.bound * sizeof(real);
 }
 
 extern "C" int SG_NAME(sg_launch_stage)(const BlockDev* tab, StageParams p,
