@@ -42,24 +42,24 @@
 //
 // What bounds it: the bytes a cell moves (about 0.7 KB in the factor sweep,
 // 0.4 KB in a residual, 0.4 KB in a correction), and, with few columns, the
-// chain of a column's layers.  Measured per launch (us), in three forms: a
-// column on eight lanes with LU factors and three right-hand sides; this
-// layout swept one way by a warp, the Woodbury vectors solved with b; this
-// one.  64-member ensemble (21,120 columns, 1.44 M cells): first sweep 815 /
-// 286 / 256, residual 634 / 222 / 160, correction 613 / 129 / 119, acceptance
-// and sum - / 93 / 60.  384 columns of 100: first sweep - / 154 / 65,
-// correction - / 83 / 42, sum - / 26 / 5; 4,096 of 64: first sweep - / 101 /
-// 63, correction - / 56 / 29.  Steps: ensemble 14.88 / 7.57 / 6.95 ms, 384 x
-// 100 with a tracer 2.66 / 1.86 / 1.29 ms, 64^3 3.48 / 1.86 / 1.51 ms.
+// instructions of a column's layers one after the other: a layer's copies are
+// at constant offsets from pointers that step by a layer, and |x| and its
+// finiteness are one integer maximum.  Measured per launch (us), in four
+// forms: a column on eight lanes with LU factors and three right-hand sides;
+// this layout swept one way by a warp, the Woodbury vectors solved with b;
+// from both walls; and this one.  64-member ensemble (21,120 columns, 1.44 M
+// cells): first sweep 815 / 286 / 256 / 226, residual 634 / 222 / 160 / 160,
+// correction 613 / 129 / 119 / 95, acceptance and sum - / 93 / 60 / 60.  384
+// columns of 100: first sweep - / 154 / 65 / 57, correction - / 83 / 42 / 24;
+// 4,096 of 64: first sweep - / 101 / 63 / 60, correction - / 56 / 29 / 24.
 #pragma once
 
 __device__ __forceinline__ bool vfinite32(float x) {
   return ((__float_as_uint(x) >> 23) & 0xffu) != 0xffu;
 }
 
-__device__ __forceinline__ void cpa16(void* s, const void* g) {
-  const unsigned a = static_cast<unsigned>(__cvta_generic_to_shared(s));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(a), "l"(g)
+__device__ __forceinline__ void cpa16(unsigned s, const void* g) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(g)
                : "memory");
 }
 __device__ __forceinline__ void cpa_commit() {
@@ -71,10 +71,15 @@ __device__ __forceinline__ void cpa_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// the warp's copy of nf floats (a multiple of 4, both ends on 16 bytes)
-__device__ __forceinline__ void tile_fill(float* s, const float* g, int nf,
+// a lane's share of the warp's copy of nf floats (a multiple of 4, both ends
+// on 16 bytes), to its own shared address s from its own source g (each 16
+// bytes a lane past the span's first): with nf known, copies at constant
+// offsets and one predicate
+__device__ __forceinline__ void tile_fill(unsigned s, const float* g, int nf,
                                           int lane) {
-  for (int e = 4 * lane; e < nf; e += 128) cpa16(s + e, g + e);
+#pragma unroll
+  for (int e = 0; e < 800; e += 128)
+    if (e + 4 * lane < nf) cpa16(s + 4 * e, g + e);
 }
 
 // 1 / p to about half an ulp without a branch: the approximate reciprocal and
@@ -187,16 +192,30 @@ __device__ __forceinline__ bool rtile_at(const BlockDev* __restrict__ tab,
 // what the two warps of a tile trade: the upper side's relation at the
 // middle, the middle's solution, each side's column flags and largest |x|
 struct MeetSmem {
-  float c[25][32], y[5][32], x[5][32], mx[2][32];
+  float c[25][32], y[5][32], x[5][32];
+  unsigned mx[2][32];
   int ok[2][32];
 };
 
-constexpr int kFacBack = 8;  // layers in a warp's ring, the factor's way out
+constexpr unsigned kInfBits = 0x7f800000u;
+__device__ __forceinline__ unsigned largest(const float (&x)[5]) {
+  unsigned m = 0;
+#pragma unroll
+  for (int r = 0; r < 5; ++r) m = max(m, __float_as_uint(x[r]) & 0x7fffffffu);
+  return m;
+}
+
+// The rings' depth costs a big batch warps per SM and gains a small one
+// nothing: the sweeps are bound by their instructions (the correction, 384
+// columns of 100, 41 us per launch with rings of 3 to 6 layers; 64 members 118
+// with 6, two CTAs an SM, and 103 with 3, five; the factor sweep's 259 with 8,
+// 235 with 5)
+constexpr int kFacBack = 5;  // layers in a warp's ring, the factor's way out
 constexpr int kBackSlot = 800 + 160;
 constexpr int kFacFloats = 2 * kFacBack * kBackSlot;  // both warps' rings
-constexpr int kCorRing = 6;  // the correction's way in
+constexpr int kCorRing = 3;  // the correction's way in
 constexpr int kCorSlot = 2 * 800 + 160;
-constexpr int kCorBack = 11;  // and its way out
+constexpr int kCorBack = 5;  // and its way out
 constexpr int kCorFloats = 2 * kCorRing * kCorSlot;
 static_assert(kCorBack * kBackSlot <= kCorRing * kCorSlot, "ring");
 
@@ -210,23 +229,31 @@ __device__ __forceinline__ void row_get(float (&v)[N], const float* g, int w) {
 // the way out from the middle of one side: x_i = y_i - C' x_prev for its cnt
 // layers from the middle's neighbour to the wall, into X; the wall layer
 // takes off e x[its third point].  y and C' arrive through a ring of RING
-// layers.  Returns the largest |x| and clears ok where one is not finite
+// layers.  Returns the bits of the largest |x| (at or above infinity's where
+// one is not finite)
 template <int RING>
-__device__ __forceinline__ float sweep_out(const float* CP, const float* Y,
-                                           float* X, int c25, int c5, int w,
-                                           int n, int cnt, bool up,
-                                           const float (&e)[5], float (&x)[5],
-                                           float* ring, bool& ok) {
+__device__ __forceinline__ unsigned sweep_out(const float* CP, const float* Y,
+                                              float* X, int c25, int c5, int w,
+                                              int n, int cnt, bool up,
+                                              const float (&e)[5], float (&x)[5],
+                                              float* ring) {
   const int lane = threadIdx.x & 31;
   const bool on = lane < w;
-  float mx = 0.f;
-  int islot = 0, gslot = 0;
-  auto layer = [&](int s) { return (size_t)(up ? n - 1 - s : s); };
-  auto issue = [&](int s) {
-    if (s >= 0) {
-      float* q = ring + islot * kBackSlot;
-      tile_fill(q, CP + layer(s) * c25, c25, lane);
-      tile_fill(q + 800, Y + layer(s) * c5, c5, lane);
+  unsigned mx = 0;  // the bits order like the magnitudes, NaN above infinity
+  const size_t first = up ? n - cnt : cnt - 1;  // the middle's neighbour
+  const ptrdiff_t s25 = up ? c25 : -c25, s5 = up ? c5 : -c5;
+  const float *gc = CP + first * c25 + 4 * lane, *gy = Y + first * c5 + 4 * lane;
+  float* px = X + first * c5 + lane;
+  const unsigned rb = smem_u32(ring) + 16 * lane;
+  int islot = 0, gslot = 0, left = cnt;
+  auto issue = [&]() {
+    if (left > 0) {
+      const unsigned q = rb + islot * (4 * kBackSlot);
+      tile_fill(q, gc, c25, lane);
+      tile_fill(q + 3200, gy, c5, lane);
+      gc += s25;
+      gy += s5;
+      --left;
     }
     islot = islot + 1 == RING ? 0 : islot + 1;
     cpa_commit();
@@ -242,7 +269,7 @@ __device__ __forceinline__ float sweep_out(const float* CP, const float* Y,
                   float (&nu)[5]) {
     cpa_wait<RING - 2>();  // the next layer is here
     __syncwarp();          // and this one's slot is read
-    issue(s - RING);
+    issue();
     get(nc, nu);
     msub5(c, x, u);
     if (s == 0) {
@@ -254,17 +281,17 @@ __device__ __forceinline__ float sweep_out(const float* CP, const float* Y,
 #pragma unroll
     for (int r = 0; r < 5; ++r) {
       x[r] = u[r];
-      mx = fmaxf(mx, fabsf(x[r]));
-      ok = ok && vfinite32(x[r]);
+      mx = max(mx, __float_as_uint(x[r]) & 0x7fffffffu);
     }
     if (on) {
 #pragma unroll
-      for (int r = 0; r < 5; ++r) X[layer(s) * c5 + r * w + lane] = x[r];
+      for (int r = 0; r < 5; ++r) px[r * w] = x[r];
     }
+    px += s5;
   };
   float c0[25], u0[5], c1[25], u1[5];
 #pragma unroll
-  for (int j = 0; j < RING; ++j) issue(cnt - 1 - j);
+  for (int j = 0; j < RING; ++j) issue();
   cpa_wait<RING - 1>();
   __syncwarp();
   get(c0, u0);
@@ -415,18 +442,17 @@ __device__ __forceinline__ void factor_tile(const RTile& T, const StageParams& p
 #pragma unroll
     for (int r = 0; r < 5; ++r) x[r] = sm.x[r][lane];
   }
-  float mx = 0.f;
-#pragma unroll
-  for (int r = 0; r < 5; ++r) mx = fmaxf(mx, fabsf(x[r]));
-  bool fin = true;
-  mx = fmaxf(mx, sweep_out<kFacBack>(T.CP, T.R, T.X0, c25, c5, w, n, cnt, up, e, x,
-                                     ring + (up ? kFacBack * kBackSlot : 0), fin));
+  unsigned mx = largest(x);
+  mx = max(mx, sweep_out<kFacBack>(T.CP, T.R, T.X0, c25, c5, w, n, cnt, up, e, x,
+                                   ring + (up ? kFacBack * kBackSlot : 0)));
   sm.mx[up][lane] = mx;
-  sm.ok[up][lane] = ok && (fin || !last);
+  sm.ok[up][lane] = ok;
   __syncthreads();
   if (up || !on) return;
-  T.stat[lane * 6] = fmaxf(mx, sm.mx[1][lane]);
-  T.mask[lane] = sm.ok[0][lane] && sm.ok[1][lane] ? 0 : 1;
+  mx = max(mx, sm.mx[1][lane]);
+  T.stat[lane * 6] = __uint_as_float(mx);
+  const bool fin = sm.ok[0][lane] && sm.ok[1][lane] && (mx < kInfBits || !last);
+  T.mask[lane] = fin ? 0 : 1;
 }
 
 __global__ void __launch_bounds__(64)
@@ -584,19 +610,28 @@ __device__ __forceinline__ void correct_tile(const RTile& T, int corr, int nk,
   const int steps = up ? cnt : cnt + 1;  // the lower warp's last: the middle
   const float* near = up ? T.C : T.B;
   float* X = T.DK + (size_t)(corr - 1) * T.dk;
-  auto layer = [&](int s) { return (size_t)(up ? n - 1 - s : s); };
   ring += up ? kCorRing * kCorSlot : 0;
   float e[5];
 #pragma unroll
   for (int r = 0; r < 5; ++r) e[r] = T.E[(up ? 5 + r : r) * w + at];
 
-  int islot = 0, gslot = 0;
-  auto issue = [&](int s) {
-    if (s < steps) {
-      float* q = ring + islot * kCorSlot;
-      tile_fill(q, T.PI + layer(s) * c25, c25, lane);
-      tile_fill(q + 800, near + layer(s) * c25, c25, lane);
-      tile_fill(q + 1600, T.R + layer(s) * c5, c5, lane);
+  const ptrdiff_t s25 = up ? -c25 : c25, s5 = up ? -c5 : c5;
+  const size_t first = up ? n - 1 : 0;
+  const float *gp = T.PI + first * c25 + 4 * lane, *gn = near + first * c25 + 4 * lane;
+  const float* gr = T.R + first * c5 + 4 * lane;
+  float* py = T.R + first * c5 + lane;
+  const unsigned rb = smem_u32(ring) + 16 * lane;
+  int islot = 0, gslot = 0, left = steps;
+  auto issue = [&]() {
+    if (left > 0) {
+      const unsigned q = rb + islot * (4 * kCorSlot);
+      tile_fill(q, gp, c25, lane);
+      tile_fill(q + 3200, gn, c25, lane);
+      tile_fill(q + 6400, gr, c5, lane);
+      gp += s25;
+      gn += s25;
+      gr += s5;
+      --left;
     }
     islot = islot + 1 == kCorRing ? 0 : islot + 1;
     cpa_commit();
@@ -609,29 +644,30 @@ __device__ __forceinline__ void correct_tile(const RTile& T, int corr, int nk,
     tile_get(pi, q, w);
   };
   float y[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-  auto step = [&](int s, float (&pi)[25], float (&b)[25], float (&t)[5],
+  auto step = [&](float (&pi)[25], float (&b)[25], float (&t)[5],
                   float (&npi)[25], float (&nb)[25], float (&nt)[5]) {
-    cpa_wait<kCorRing - 2>();  // layer s + 1 is here
-    __syncwarp();              // and layer s's slot is read
-    issue(s + kCorRing);
+    cpa_wait<kCorRing - 2>();  // the next layer is here
+    __syncwarp();              // and this one's slot is read
+    issue();
     get(npi, nb, nt);
     msub5(b, y, t);
     mul5(pi, t, y);
     if (on) {
 #pragma unroll
-      for (int r = 0; r < 5; ++r) T.R[layer(s) * c5 + r * w + lane] = y[r];
+      for (int r = 0; r < 5; ++r) py[r * w] = y[r];
     }
+    py += s5;
   };
 #pragma unroll
-  for (int j = 0; j < kCorRing; ++j) issue(j);
+  for (int j = 0; j < kCorRing; ++j) issue();
   float p0[25], b0[25], t0[5], p1[25], b1[25], t1[5];
   cpa_wait<kCorRing - 1>();
   __syncwarp();
   get(p0, b0, t0);
   for (int s = 0; s < cnt; s += 2) {
-    step(s, p0, b0, t0, p1, b1, t1);
+    step(p0, b0, t0, p1, b1, t1);
     if (s + 1 < cnt) {
-      step(s + 1, p1, b1, t1, p0, b0, t0);
+      step(p1, b1, t1, p0, b0, t0);
     } else {
 #pragma unroll
       for (int k = 0; k < 25; ++k) p0[k] = p1[k], b0[k] = b1[k];
@@ -666,23 +702,16 @@ __device__ __forceinline__ void correct_tile(const RTile& T, int corr, int nk,
 #pragma unroll
     for (int r = 0; r < 5; ++r) x[r] = sm.x[r][lane];
   }
-  bool ok = true;
-  float mx = 0.f;
-#pragma unroll
-  for (int r = 0; r < 5; ++r) {
-    mx = fmaxf(mx, fabsf(x[r]));
-    ok = ok && vfinite32(x[r]);
-  }
-  mx = fmaxf(mx, sweep_out<kCorBack>(T.CP, T.R, X, c25, c5, w, n, cnt, up, e, x,
-                                     ring, ok));
+  unsigned mx = largest(x);
+  mx = max(mx, sweep_out<kCorBack>(T.CP, T.R, X, c25, c5, w, n, cnt, up, e, x, ring));
   sm.mx[up][lane] = mx;
-  sm.ok[up][lane] = ok;
   __syncthreads();
   if (up || !on) return;
+  mx = max(mx, sm.mx[1][lane]);
   float* st = T.stat + lane * 6;
-  const float dl = fmaxf(mx, sm.mx[1][lane]), dp = st[corr - 1];
+  const float dl = __uint_as_float(mx), dp = st[corr - 1];
   st[corr] = dl;
-  bool fin = sm.ok[0][lane] && sm.ok[1][lane];
+  bool fin = mx < kInfBits;
   if (corr == nk) {
     const float rho = dp > 0.f ? fminf(dl / dp, 1.f) : 0.f;
     fin = fin && dl * rho <= 0x1p-44f * st[0];
