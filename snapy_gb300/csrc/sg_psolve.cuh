@@ -253,7 +253,7 @@ __device__ __forceinline__ void psw_sub_mv(double (&t)[5], const double* M,
   }
 }
 
-// one warp per column: grid (columns, blocks), 32 threads.
+// one column on a warp.
 // BLK32 false: the FP64-assembled blocks with the partitioned form on
 // (sg_set_sweep), every column; its region holds E, F and the mask.
 // BLK32 true: the FP32-assembled blocks' columns that the refined solve
@@ -262,24 +262,17 @@ __device__ __forceinline__ void psw_sub_mv(double (&t)[5], const double* M,
 // leave free by then.  A column it solves gets mask 3 (done), one it
 // cannot mask 2 (the serial FP64 solve takes it, without counting it again)
 template <bool BLK32>
-__global__ void __launch_bounds__(32)
-    vic_psolve_kernel(const BlockDev* __restrict__ tab, StageParams p) {
-  __shared__ PswSmem sm;
-  const BlockDev& Bk = tab[blockIdx.y];
-  if (!Bk.implicit || Bk.implicit == 1) return;
-  if (BLK32 ? !Bk.implicit_f32 : (Bk.implicit_f32 || !Bk.psw)) return;
-  const VicScratch S = vic_scratch(Bk);
+__device__ __forceinline__ void psolve_column(const BlockDev& Bk,
+                                              const StageParams& p,
+                                              const VicScratch& S, size_t ncol,
+                                              size_t col, PswSmem& sm) {
   const int n = Bk.nc1 - 2 * Bk.ng;
-  const size_t ncol = S.cells / n;
-  const size_t col = blockIdx.x;
-  if (col >= ncol || n < kPswMinLayers) return;
   const unsigned full = 0xffffffffu;
   PswScratch W;
   int* maskp;
   const VicScratch32 F32 = BLK32 ? vic_scratch32(Bk, S, n) : VicScratch32{};
   if (BLK32) {
     maskp = F32.mask + col;
-    if (*maskp != 1) return;  // uniform over the warp
     W.E = S.A;
     W.F = S.B;
     if (threadIdx.x == 0) count_fp64_column(p, blockIdx.y);
@@ -689,5 +682,34 @@ __global__ void __launch_bounds__(32)
       *maskp = good ? 0 : 1;
       if (!good) atomicAdd(&p.fallbacks[blockIdx.y], 1ull);
     }
+  }
+}
+
+// grid (columns / per, blocks), a warp per CTA: BLK32 false one column (per
+// 1); BLK32 true those of the CTA's `per` columns that are masked, usually
+// none (a CTA costs its launch, about 1 us a thousand: one per column took 31
+// us of each launch of the 64-member ensemble, 53 of four served requests)
+template <bool BLK32>
+__global__ void __launch_bounds__(32)
+    vic_psolve_kernel(const BlockDev* __restrict__ tab, StageParams p, int per) {
+  __shared__ PswSmem sm;
+  const BlockDev& Bk = tab[blockIdx.y];
+  if (!Bk.implicit || Bk.implicit == 1) return;
+  if (BLK32 ? !Bk.implicit_f32 : (Bk.implicit_f32 || !Bk.psw)) return;
+  const VicScratch S = vic_scratch(Bk);
+  const int n = Bk.nc1 - 2 * Bk.ng;
+  const size_t ncol = S.cells / n, first = (size_t)blockIdx.x * per;
+  if (first >= ncol || n < kPswMinLayers) return;
+  if (!BLK32) {
+    psolve_column<false>(Bk, p, S, ncol, first, sm);
+    return;
+  }
+  const int lane = threadIdx.x;
+  const int* mask = vic_scratch32(Bk, S, n).mask;
+  unsigned todo = __ballot_sync(0xffffffffu, lane < per && first + lane < ncol &&
+                                                 mask[first + lane] == 1);
+  for (; todo; todo &= todo - 1) {
+    psolve_column<true>(Bk, p, S, ncol, first + (__ffs(todo) - 1), sm);
+    __syncwarp();
   }
 }

@@ -52,3 +52,27 @@ def test_fp32_solution_at_a_ragged_tile(cuda):
     want, _ = solution(cuda, 12, 33, 0)
     assert left == 0
     assert (torch.linalg.norm(got - want) / torch.linalg.norm(want)).item() <= 1e-4
+
+
+def test_masked_columns_of_a_wide_batch(cuda):
+    """A batch of more columns than the left-over solve has CTAs (several
+    columns a CTA): a NaN in one cell leaves the columns its stencils reach to
+    the FP64 solve, each counted once and failed there, the others untouched."""
+    opts = sg.MeshBlockOptions.from_yaml("snapy_gb300/decks/convection3d.yaml")
+    c = opts.coord()
+    c.nx1, c.nx2, c.nx3 = 16, 96, 90
+    c.x1max, c.x2max, c.x3max = 800.0, 4800.0, 4500.0
+    opts.hydro().precision = opts.hydro().icorr.precision = "float32"
+    opts.execution = "eager"
+    opts.autotune = False
+    blk = sg.MeshBlock(opts).to(cuda)
+    vars = {"hydro_w": problems.convection3d(opts, cuda, seed=1)}
+    blk.initialize(vars)
+    dt = blk.max_time_step(vars)
+    vars["hydro_u"][0, 3 + 40, 3 + 50, 3 + 8] = float("nan")
+    blk.forward(vars, dt, 0)
+    bad = torch.isnan(vars["hydro_u"][:, 3:-3, 3:-3, 3:-3]).any(dim=0).any(dim=-1)
+    where = torch.nonzero(bad).cpu().tolist()
+    want = {(40, 50)} | {(40 + d, 50) for d in range(-3, 4)} | {(40, 50 + d) for d in range(-3, 4)}
+    assert {tuple(w) for w in where} == want
+    assert blk.batch.solve_fallbacks()[0] == len(want)
