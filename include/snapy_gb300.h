@@ -149,6 +149,11 @@ int sg_fill_ghosts(sg_handle* h, sg_stream_t stream);
 /* dt_dev_out[b] = cfl 2^-redo[b] min over block b (no host sync) */
 int sg_max_dt(sg_handle* h, const int32_t* redo_dev, double* dt_dev_out,
               sg_stream_t stream);
+/* the same with the redo count `redo` for every block (stored in redo_dev),
+ * and the dt of every block in host memory too, dt_host[nblock]: waits for
+ * the stream */
+int sg_max_dt_host(sg_handle* h, int32_t redo, int32_t* redo_dev,
+                   double* dt_dev_out, double* dt_host, sg_stream_t stream);
 /* per-block retry flags into flags_dev (int32[nblock]): bit 0 floor, bit 3
  * NaN, bit 5 a failed column of the implicit solve (meshblock_redo.cpp),
  * bit 6 a tile whose shared-memory staging did not arrive within the stage

@@ -101,6 +101,7 @@ SIGNATURES = {
     "sg_stage": (ctypes.c_int, [_vp, _i32, _vp, _vp]),
     "sg_fill_ghosts": (ctypes.c_int, [_vp, _vp]),
     "sg_max_dt": (ctypes.c_int, [_vp, _vp, _vp, _vp]),
+    "sg_max_dt_host": (ctypes.c_int, [_vp, _i32, _vp, _vp, _vp, _vp]),
     "sg_check": (ctypes.c_int, [_vp, _vp, _vp]),
     "sg_init_from_prim": (ctypes.c_int, [_vp, ctypes.POINTER(_vp), _vp]),
     "sg_restore": (ctypes.c_int, [_vp]),

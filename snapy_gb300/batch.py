@@ -254,6 +254,15 @@ class Batch:
                                     _stream(stream)), "sg_max_dt")
         return self.dt
 
+    def max_dt_host(self, redo: int, stream=None) -> list:
+        """max_dt with the redo count of every block set to `redo`, the dts
+        also on the host (waits for the stream)."""
+        out = (ctypes.c_double * self.nblock)()
+        _lib.check(self.L.sg_max_dt_host(self.h, redo, self.redo.data_ptr(),
+                                         self.dt.data_ptr(), out, _stream(stream)),
+                   "sg_max_dt_host")
+        return list(out)
+
     def check(self, stream=None) -> torch.Tensor:
         _lib.check(self.L.sg_check(self.h, self.flags.data_ptr(), _stream(stream)),
                    "sg_check")

@@ -80,15 +80,20 @@ __device__ __forceinline__ double unkey(unsigned long long k) {
 
 // dt[b] = (2^-redo[b] cfl) dt_min[b]  (meshblock_advance.cpp:61-72); a NaN
 // anywhere makes the step's dt NaN, as torch's min does
+// with `host` (pinned memory) the redo count is `set` for every block, stored
+// in redo, and the dt goes to the host too
 __global__ void finish_dt_kernel(int nblock, unsigned long long* red, int* nan,
-                                 const int32_t* redo, double cfl,
-                                 double* dt_out) {
+                                 int32_t* redo, double cfl, double* dt_out,
+                                 int32_t set = 0, double* host = nullptr) {
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nblock) return;
   double dtm = unkey(red[4 * b]);
+  if (host) redo[b] = set;
   // 2^-redo, exact (pow would take longer than the reduction)
   double f = redo ? ldexp(1., -redo[b]) : 1.;
-  dt_out[b] = nan[b] ? __longlong_as_double(0x7ff8000000000000ll) : f * cfl * dtm;
+  const double dt = nan[b] ? __longlong_as_double(0x7ff8000000000000ll) : f * cfl * dtm;
+  dt_out[b] = dt;
+  if (host) host[b] = dt;
   red[4 * b] = red[4 * b + 1] = red[4 * b + 2] = kKeyInf;
   nan[b] = 0;
 }
@@ -227,6 +232,7 @@ struct sg_handle {
   int* nan = nullptr;
   void** ptrs = nullptr;  // device array of nblock pointers (sg_prim)
   void** ptrs_host = nullptr;  // pinned staging
+  double* dt_host = nullptr;   // pinned: sg_max_dt_host's result
   int32_t nblock = 0, ntile = 0;
   int32_t cur = 0, base = 0;  // current buffer, stage-0 buffer
   bool bound_all = false, dirty = true;
@@ -1088,6 +1094,7 @@ int sg_create(const sg_scheme* scheme, const sg_block_desc* blocks,
   if (e == cudaSuccess)
     e = cudaMemset(h->counts, 0, sizeof(unsigned long long) * sg::kCountSlots * nblock);
   if (e == cudaSuccess) e = cudaMallocHost(&h->ptrs_host, sizeof(void*) * nblock);
+  if (e == cudaSuccess) e = cudaMallocHost(&h->dt_host, sizeof(double) * nblock);
   if (e != cudaSuccess) {
     sg_destroy(h);
     return cuda_fail(e, "sg_create");
@@ -1112,6 +1119,7 @@ int sg_destroy(sg_handle* h) {
   if (h->fallbacks) cudaFree(h->fallbacks);
   if (h->counts) cudaFree(h->counts);
   if (h->ptrs_host) cudaFreeHost(h->ptrs_host);
+  if (h->dt_host) cudaFreeHost(h->dt_host);
   for (cudaEvent_t e : h->events) cudaEventDestroy(e);
   for (double* t : h->x1tabs) cudaFree(t);
   if (h->psw_mem) cudaFree(h->psw_mem);
@@ -1544,10 +1552,9 @@ int sg_fill_ghosts(sg_handle* h, sg_stream_t stream) {
   return 0;
 }
 
-int sg_max_dt(sg_handle* h, const int32_t* redo_dev, double* dt_out,
-              sg_stream_t stream) {
-  if (!h || !dt_out) return fail(SG_ERR_ARG, "sg_max_dt: null");
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+namespace {
+int max_dt(sg_handle* h, int32_t* redo_dev, double* dt_out, int32_t set,
+           double* host, cudaStream_t s) {
   int rc = upload(h, s);
   if (rc) return rc;
   rc = f64(h) ? sg_launch_reduce_f64(h->dev, h->nblock, h->cur, h->red,
@@ -1556,9 +1563,30 @@ int sg_max_dt(sg_handle* h, const int32_t* redo_dev, double* dt_out,
                                      h->nan, h->max_cells, s);
   if (rc) return cuda_fail((cudaError_t)rc, "sg_max_dt: reduce");
   finish_dt_kernel<<<(h->nblock + 127) / 128, 128, 0, s>>>(
-      h->nblock, h->red, h->nan, redo_dev, h->scheme.cfl, dt_out);
+      h->nblock, h->red, h->nan, redo_dev, h->scheme.cfl, dt_out, set, host);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "sg_max_dt: finish");
+  return 0;
+}
+}  // namespace
+
+int sg_max_dt(sg_handle* h, const int32_t* redo_dev, double* dt_out,
+              sg_stream_t stream) {
+  if (!h || !dt_out) return fail(SG_ERR_ARG, "sg_max_dt: null");
+  return max_dt(h, const_cast<int32_t*>(redo_dev), dt_out, 0, nullptr,
+                reinterpret_cast<cudaStream_t>(stream));
+}
+
+int sg_max_dt_host(sg_handle* h, int32_t redo, int32_t* redo_dev,
+                   double* dt_out, double* dt_host, sg_stream_t stream) {
+  if (!h || !redo_dev || !dt_out || !dt_host)
+    return fail(SG_ERR_ARG, "sg_max_dt_host: null");
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  int rc = max_dt(h, redo_dev, dt_out, redo, h->dt_host, s);
+  if (rc) return rc;
+  cudaError_t e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess) return cuda_fail(e, "sg_max_dt_host");
+  memcpy(dt_host, h->dt_host, sizeof(double) * h->nblock);
   return 0;
 }
 

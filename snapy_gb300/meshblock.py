@@ -562,9 +562,7 @@ class MeshBlock:
 
     def max_time_step(self, vars: dict) -> float:
         with torch.cuda.device(self.device):
-            self.batch.redo.fill_(self.intg.current_redo)
-            dt = self.batch.max_dt()
-            return float(dt[0].item())
+            return self.batch.max_dt_host(self.intg.current_redo)[0]
 
     def check_redo(self, vars: dict) -> int:
         with torch.cuda.device(self.device):
