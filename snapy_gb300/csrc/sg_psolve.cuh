@@ -698,7 +698,7 @@ __global__ void __launch_bounds__(32)
   if (BLK32 ? !Bk.implicit_f32 : (Bk.implicit_f32 || !Bk.psw)) return;
   const VicScratch S = vic_scratch(Bk);
   const int n = Bk.nc1 - 2 * Bk.ng;
-  const size_t ncol = S.cells / n, first = (size_t)blockIdx.x * per;
+  const size_t ncol = udiv(S.cells, n), first = (size_t)blockIdx.x * per;
   if (first >= ncol || n < kPswMinLayers) return;
   if (!BLK32) {
     psolve_column<false>(Bk, p, S, ncol, first, sm);

@@ -525,14 +525,14 @@ __device__ __forceinline__ void tf_madd(float& sh, float& mh, float& ml, float t
 //   T d in float-float on the FP32 pipe (its error, 2^-48 of the sum of
 //   |t d| with |d| about 2^-22 |x|, is far below the FP64 rounding of r).
 // Every load is a tile's row of 32 consecutive values.
-template <int W>
+template <bool FIRST, int W>
 __device__ __forceinline__ void residual_row(const RTile& T, int i, int corr,
                                              bool keep, double dtc) {
   const int w = W ? W : T.w, n = T.n;
   const int lane = threadIdx.x & 31;
   if (lane >= w) return;
   const int c25 = VicTile::chunk(25, w), c5 = VicTile::chunk(5, w);
-  const float* X = (corr == 1 ? T.X0 : T.DK + (size_t)(corr - 2) * T.dk) + lane;
+  const float* X = (FIRST ? T.X0 : T.DK + (size_t)(corr - 2) * T.dk) + lane;
   double* r64 = T.r64 + (size_t)i * 5 * w + lane;
   double t[5];
 #pragma unroll
@@ -547,7 +547,7 @@ __device__ __forceinline__ void residual_row(const RTile& T, int i, int corr,
 #pragma unroll
     for (int k = 0; k < 5; ++k) x[k] = X[e + k * w];
     const float* M = (m == 0 ? T.A : (m == 1 ? T.B : T.C)) + (size_t)i * c25 + lane;
-    if (corr == 1) {
+    if (FIRST) {
 #pragma unroll
       for (int r = 0; r < 5; ++r)
 #pragma unroll
@@ -562,8 +562,11 @@ __device__ __forceinline__ void residual_row(const RTile& T, int i, int corr,
     }
   }
 #pragma unroll
-  for (int r = 0; r < 5; ++r)
-    t[r] = ((t[r] - widen_exact(sh[r])) - widen_exact(mh[r])) - widen_exact(ml[r]);
+  for (int r = 0; r < 5; ++r) t[r] = (t[r] - widen_exact(sh[r])) - widen_exact(mh[r]);
+  if (FIRST) {  // (a later one leaves ml at zero)
+#pragma unroll
+    for (int r = 0; r < 5; ++r) t[r] = t[r] - widen_exact(ml[r]);
+  }
   // the wall rows' third points
   if (i == 0)
     t[4] -= (-vic_krows(*T.blk, n, 0).t0 / dtc) * widen_exact(X[(size_t)2 * c5]);
@@ -578,7 +581,8 @@ __device__ __forceinline__ void residual_row(const RTile& T, int i, int corr,
 }
 
 // eight layers of a tile per CTA (lg CTAs a tile)
-__global__ void __launch_bounds__(kThreads)
+template <bool FIRST>
+__global__ void __launch_bounds__(kThreads, 3)
     vic_residual_kernel(const BlockDev* __restrict__ tab, StageParams p,
                         int corr, int lg) {
   RTile T;
@@ -588,9 +592,9 @@ __global__ void __launch_bounds__(kThreads)
   const bool keep = corr < p.refine;  // a later correction reads r
   const double dtc = p.w2 * p.dt[blockIdx.y];
   if (T.w == 32)
-    residual_row<32>(T, i, corr, keep, dtc);
+    residual_row<FIRST, 32>(T, i, corr, keep, dtc);
   else
-    residual_row<0>(T, i, corr, keep, dtc);
+    residual_row<FIRST, 0>(T, i, corr, keep, dtc);
 }
 
 // A correction's sweeps of a tile, the factor's on r with its factors, and

@@ -1522,6 +1522,17 @@ __global__ void __launch_bounds__(kThreads)
 // of the two sides' ratios, rho and u_n of the hydro's face means, D1 the
 // centred x1 difference), and the positivity limiter below follows.
 // ---------------------------------------------------------------------------
+// the base's density in the storage type after the stage kernel (null: the
+// state holds totals): FP32 reads the stage's table, whose values are the
+// base's rounded, instead of converting on the FP64 pipe at every use
+__device__ __forceinline__ const real* base_rho_real(const BlockDev& B) {
+#ifdef SG_REAL_IS_FLOAT
+  return B.base ? ref_tab(B.refb, B.nc1).rb : nullptr;
+#else
+  return B.base ? base_rho(B.base, B.nc1) : nullptr;
+#endif
+}
+
 // the ratio of one side of face q (stride st) of tracer sv
 template <typename RHO>
 __device__ __forceinline__ real scalar_face_ratio(const real* sv, RHO rho,
@@ -1557,14 +1568,14 @@ __global__ void __launch_bounds__(kThreads)
   const size_t n3f = has3 ? (size_t)(nx3 + 1) * nx2 * nx1 : 0;
   const real* u = static_cast<const real*>(B.buf[p.in]);
   const real* s = static_cast<const real*>(B.sbuf[p.in]);
-  const double* rb = B.base ? base_rho(B.base, nc1) : nullptr;
+  const real* rb = base_rho_real(B);
   const real gammad = real(B.gammad);
   const bool scale = p.scale != 0;
   const bool covs = B.flux_cov && nc1 >= 3;
   // the total dry density (the state holds an anomaly under a base)
   auto rho = [&](size_t c) -> real {
     real v = u[IDN * plane + c];
-    if (rb) v = v + real(rb[c % nc1]);
+    if (rb) v = v + rb[(unsigned)c % (unsigned)nc1];
     return v;
   };
   for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1682,10 +1693,10 @@ __global__ void __launch_bounds__(kThreads)
   const bool act[3] = {true, has2, has3};
   const real* u = static_cast<const real*>(B.buf[p.in]);
   const real* s = static_cast<const real*>(B.sbuf[p.in]);
-  const double* rb = B.base ? base_rho(B.base, nc1) : nullptr;
+  const real* rb = base_rho_real(B);
   auto rho = [&](size_t c) -> real {
     real v = u[IDN * plane + c];
-    if (rb) v = v + real(rb[c % nc1]);
+    if (rb) v = v + rb[(unsigned)c % (unsigned)nc1];
     return v;
   };
   // theta of a channel: densities q (by a functor), face fluxes F[d]
@@ -2378,7 +2389,7 @@ __global__ void __launch_bounds__(32 * kVicScalarWarps)
   const real* s0 = static_cast<const real*>(B.sbuf[p.u0]) + v * plane + row;
   real* so = static_cast<real*>(B.sbuf[p.out]) + v * plane + row;
   const real* u = static_cast<const real*>(B.buf[p.in]) + IDN * plane + row;
-  const double* rb = B.base ? base_rho(B.base, nc1) : nullptr;
+  const real* rb = base_rho_real(B);
   const double* ds = B.sds + v * plane + row;
   const double* q = B.vicq + row;
   double* P = B.sflux[0] + v * plane + row;
@@ -2386,7 +2397,7 @@ __global__ void __launch_bounds__(32 * kVicScalarWarps)
   const int il = ng, iu = ng + n - 1;
   auto ratio = [&](int i) -> double {
     real rho = u[i];
-    if (rb) rho = rho + real(rb[i]);
+    if (rb) rho = rho + rb[i];
     return (double)(s[i] / rho);
   };
   auto held = [&](int i) -> double {
@@ -2723,8 +2734,8 @@ extern "C" int SG_NAME(sg_launch_vic)(const BlockDev* tab, StageParams p,
     vic_factor32_kernel<<<dim3(gt, p.nblock), 64, kFacFloats * sizeof(float),
                           stream>>>(tab, p);
     for (int k = 1; k <= p.refine; ++k) {
-      vic_residual_kernel<<<dim3(gt * lg, p.nblock), kThreads, 0, stream>>>(
-          tab, p, k, lg);
+      (k == 1 ? vic_residual_kernel<true> : vic_residual_kernel<false>)
+          <<<dim3(gt * lg, p.nblock), kThreads, 0, stream>>>(tab, p, k, lg);
       vic_correct32_kernel<<<dim3(gt, p.nblock), 64, kCorFloats * sizeof(float),
                              stream>>>(tab, p, k);
     }

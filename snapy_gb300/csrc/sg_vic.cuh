@@ -26,6 +26,13 @@
 // for bit the CPU oracle's.
 #pragma once
 
+// Divisions of column and layer counts run in 32 bits: a block's interior
+// cells take 800 bytes of scratch each, so there are fewer than 2^32 of them,
+// and a 64-bit division costs a hundred instructions a thread
+__device__ __forceinline__ unsigned udiv(size_t a, int b) {
+  return (unsigned)a / (unsigned)b;
+}
+
 struct VicScratch {
   double *du, *du0, *A, *B, *C, *D, *Z0, *Z1;
   size_t cells;
@@ -97,7 +104,7 @@ __device__ __forceinline__ VicScratch32 vic_scratch32(const BlockDev& B,
   VicScratch32 t;
   const size_t c = S.cells;
   float* f = reinterpret_cast<float*>(B.vic + (size_t)kVicDoublesPerCell * c);
-  t.ncol = c / n;
+  t.ncol = udiv(c, n);
   const size_t t25 = VicTile::total(25, t.ncol, n);
   const size_t t5 = VicTile::total(5, t.ncol, n);
   t.A = f;
@@ -136,9 +143,10 @@ struct VicCol32 {
 // the padded (x3, x2) row of interior column `col` (x2 fastest)
 __device__ __forceinline__ size_t vic_row(const BlockDev& B, size_t col) {
   const int ng = B.ng;
-  const size_t nx2 = B.nc2 > 1 ? B.nc2 - 2 * ng : 1;
-  const size_t j = col % nx2, k = col / nx2;
-  return (B.nc3 > 1 ? k + ng : 0) * B.nc2 + (B.nc2 > 1 ? j + ng : 0);
+  if (B.nc3 == 1) return B.nc2 > 1 ? col + ng : 0;
+  const int nx2 = B.nc2 > 1 ? B.nc2 - 2 * ng : 1;
+  const unsigned k = udiv(col, nx2), j = (unsigned)col - k * nx2;
+  return (size_t)(k + ng) * B.nc2 + (B.nc2 > 1 ? j + ng : 0);
 }
 
 // bit of the per-block status word: a column's solve failed this step
@@ -592,11 +600,11 @@ __global__ void __launch_bounds__(AsmShape<T>::threads, AsmShape<T>::ctas)
     return;
   const int nc1 = B.nc1, n = nc1 - 2 * B.ng;
   const VicScratch S = vic_scratch(B);
-  const size_t ncol = S.cells / n, run = ((ncol + cw - 1) / cw) * (n + 2);
+  const size_t ncol = udiv(S.cells, n), run = ((ncol + cw - 1) / cw) * (n + 2);
   const size_t first = (size_t)blockIdx.x * (rows - 2);
   if (first + 2 >= run) return;
   const int t = threadIdx.x, row = t / cw;
-  const size_t at = first + row, g = at / (n + 2);
+  const size_t at = first + row, g = udiv(at, n + 2);
   const int i = (int)(at - g * (n + 2)) - 1;  // -1: the ghost below, n: above
   const size_t col = g * cw + t % cw;
   const bool on = at < run && col < ncol;
@@ -1031,7 +1039,7 @@ __global__ void __launch_bounds__(32)
   if (!Bk.implicit || Bk.implicit == 1) return;  // scheme 1: vic_solve3
   const VicScratch S = vic_scratch(Bk);
   const int n = Bk.nc1 - 2 * Bk.ng;
-  const size_t ncol = S.cells / n;
+  const size_t ncol = udiv(S.cells, n);
   if (!BLK32 && Bk.wsolve && !Bk.psw) {
     if (blockIdx.x < ncol)
       vic_column_warp(Bk, S, blockIdx.x, n, p.w2 * p.dt[blockIdx.y], smem.one, status);
@@ -1417,7 +1425,7 @@ __global__ void __launch_bounds__(kThreads)
   if (Bk.implicit != 1) return;
   const VicScratch S = vic_scratch(Bk);
   const int n = Bk.nc1 - 2 * Bk.ng;
-  const size_t ncol = S.cells / n;
+  const size_t ncol = udiv(S.cells, n);
   const size_t col = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= ncol) return;
   const double dtc = p.w2 * p.dt[blockIdx.y];
@@ -1636,7 +1644,7 @@ __global__ void __launch_bounds__(kFinThreads, 3)
   const VicScratch S = vic_scratch(B);
   const int ng = B.ng, nc1 = B.nc1, n = nc1 - 2 * ng;
   const int cols = fin_cols(n, p.fin_len);
-  const size_t ncol = S.cells / n, col0 = (size_t)blockIdx.x * cols;
+  const size_t ncol = udiv(S.cells, n), col0 = (size_t)blockIdx.x * cols;
   if (col0 >= ncol) return;
   const int nc = ncol - col0 < (size_t)cols ? (int)(ncol - col0) : cols;
   const int tid = threadIdx.x, lane = tid & 31, wq = tid >> 5;
