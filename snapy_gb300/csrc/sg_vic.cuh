@@ -323,7 +323,7 @@ __device__ __forceinline__ VicK vic_krows(const BlockDev& B, int n, int k) {
 }
 
 // (1) the blocks of every interior cell, the K coupling in their (IPR, IDN)
-// entries and du[IPR] -= K du0[IDN]
+// entries and du[IPR] -= K du[IDN] (its explicit row kept in du0)
 // the blocks of interior cell e (column e / n, layer e % n) in the compute
 // type T: double, or float under implicit-precision float32 (the FP32
 // state's blocks, exact in FP32 and in the FP64 copies the residuals of the
@@ -383,7 +383,8 @@ struct AsmConst {
 template <typename T>
 __device__ __forceinline__ void vic_assemble_cell(
     const BlockDev& B, const VicScratch& S, double dtc, double rdtc, size_t col,
-    int i, bool f32copy, const AsmConst<T>& kc, const AsmSmem<T>& sm, int t) {
+    int i, bool f32copy, const AsmConst<T>& kc, const AsmSmem<T>& sm, int t,
+    const double (&du0)[5]) {
   constexpr int cw = AsmShape<T>::cw;
   const int ng = B.ng, n = B.nc1 - 2 * ng;
   const T grav = kc.grav, gm1 = kc.gm1;
@@ -453,12 +454,9 @@ __device__ __forceinline__ void vic_assemble_cell(
     return v;
   };
   const size_t cell = col * n + i;
-  double du0[5];
-#pragma unroll
-  for (int v = 0; v < 5; ++v) {
-    du0[v] = S.du[v * S.cells + cell];
-    S.du0[v * S.cells + cell] = du0[v];
-  }
+  // (the finish reads the explicit energy row only of a column that failed;
+  // the other rows stay in du)
+  S.du0[4 * S.cells + cell] = du0[4];
   double du4 = du0[4];
   // the partial matrix (implicit-scheme 1, assembled in FP64 or FP32 and
   // solved in FP64 by vic_solve3_kernel): its 3x3
@@ -611,6 +609,13 @@ __global__ void __launch_bounds__(AsmShape<T>::threads, AsmShape<T>::ctas)
   const double dtc = p.w2 * p.dt[blockIdx.y];
   const double rdtc = 1. / dtc;
   const AsmConst<T> kc(B, dtc, rdtc);
+  const bool inner = on && i >= 0 && i < n && row > 0 && row < rows - 1;
+  // the tendency arrives while the primitives and the |A| are formed
+  double du0[5] = {0., 0., 0., 0., 0.};
+  if (inner) {
+#pragma unroll
+    for (int v = 0; v < 5; ++v) du0[v] = S.du[v * S.cells + col * n + i];
+  }
   T w[5];
   if (on) {
     const real* uin = static_cast<const real*>(B.buf[p.in]);
@@ -640,10 +645,10 @@ __global__ void __launch_bounds__(AsmShape<T>::threads, AsmShape<T>::ctas)
     for (int k = 0; k < 25; ++k) sm.A[k][t] = A[k];
   }
   __syncthreads();
-  if (on && i >= 0 && i < n && row > 0 && row < rows - 1)
+  if (inner)
     vic_assemble_cell<T>(B, S, dtc, rdtc, col, i,
                          sizeof(T) == sizeof(float) && p.refine != 0 && B.implicit == 9,
-                         kc, sm, t);
+                         kc, sm, t, du0);
 }
 
 // ludcmp<double, 5, Implicit> on a row-major 5x5 in shared memory
@@ -1663,7 +1668,7 @@ __global__ void __launch_bounds__(kFinThreads, 3)
   double* aR = aM + len;  // the density, the available mass, the IDN row
   double* aQ = aR + len;  // rho V, then the moved mass q
   double* aV = aQ + len;  // q / V
-  double* aW = aV + len;  // D_rho - du0_rho
+  double* aW = aV + len;  // D_rho - du_rho
   double* aT2 = aW + len;  // partial: the tangential velocities, 0 .. n
   double* aT3 = aT2 + len;
   if (tid < nc) sok[tid] = vfinite(S.D[(col0 + tid) * n * 5]);
@@ -1681,9 +1686,9 @@ __global__ void __launch_bounds__(kFinThreads, 3)
     vic_prim(uin, plane, base + i, B.gammad, w, B.base, nc1);
     aR[o] = w[0];
     aQ[o] = w[0] * vol;
-    const double d = S.D[g * 5];
-    aM[o] = (d - S.du[g]) * vol;
-    aW[o] = d - S.du0[g];
+    const double rest = S.D[g * 5] - S.du[g];
+    aM[o] = rest * vol;
+    aW[o] = rest;
     if (partial) {
       aT2[o] = w[2];
       aT3[o] = w[3];
@@ -1803,7 +1808,7 @@ __global__ void __launch_bounds__(kFinThreads, 3)
     if (tid < nc) {
       const size_t col = col0 + tid;
       const bool ok = sok[tid] != 0;
-      const double *D = S.D + col * n * 5, *du0 = S.du0 + col * n;
+      const double *D = S.D + col * n * 5, *du = S.du + col * n;
       const int o = tid * pitch;
       double sy = 0., sz = 0.;
       for (int f = 0; f < nf; ++f) {
@@ -1816,8 +1821,8 @@ __global__ void __launch_bounds__(kFinThreads, 3)
         } else if (ok) {
           double py = 0., pz = 0.;
           if (f > 0) {
-            sy = sy + (D[(f - 1) * 5 + 2] - du0[2 * cs + f - 1]) * vol;
-            sz = sz + (D[(f - 1) * 5 + 3] - du0[3 * cs + f - 1]) * vol;
+            sy = sy + (D[(f - 1) * 5 + 2] - du[2 * cs + f - 1]) * vol;
+            sz = sz + (D[(f - 1) * 5 + 3] - du[3 * cs + f - 1]) * vol;
             py = -sy;
             pz = -sz;
           }
@@ -1837,7 +1842,7 @@ __global__ void __launch_bounds__(kFinThreads, 3)
   for (int e = tid; e < cells; e += kFinThreads) {
     const int c = e / n, i = e - c * n, o = c * pitch + i;
     const size_t col = col0 + c, g = col * n + i;
-    const double* du0 = S.du0 + g;
+    const double* du = S.du + g;
     double d[5];
     if (sok[c]) {
       const double* D = S.D + g * 5;
@@ -1882,9 +1887,9 @@ __global__ void __launch_bounds__(kFinThreads, 3)
         vic_slope_tab(B, n, i, wt, &i0);
         const VicK K = vic_krows(B, n, i);
         const int s0 = i0 - i;
-        double sl = wt[0] * (aR[o + s0] - du0[s0]);
-        sl += wt[1] * (aR[o + s0 + 1] - du0[s0 + 1]);
-        sl += wt[2] * (aR[o + s0 + 2] - du0[s0 + 2]);
+        double sl = wt[0] * (aR[o + s0] - du[s0]);
+        sl += wt[1] * (aR[o + s0 + 1] - du[s0 + 1]);
+        sl += wt[2] * (aR[o + s0 + 2] - du[s0 + 2]);
         double wk = K.gv * sl;
         double s = K.mid * aW[o];
         if (i >= 1) s += K.lo * aW[o - 1];
@@ -1897,7 +1902,8 @@ __global__ void __launch_bounds__(kFinThreads, 3)
       d[4] = e4;
     } else {
 #pragma unroll
-      for (int v = 0; v < 5; ++v) d[v] = du0[v * cs];
+      for (int v = 0; v < 4; ++v) d[v] = du[v * cs];
+      d[4] = S.du0[4 * cs + g];
     }
     const size_t cell = vic_row(B, col) * nc1 + ng + i;
 #pragma unroll
