@@ -126,7 +126,8 @@ __host__ __device__ inline const double* base_e(const double* b, int nc1) { retu
 __host__ __device__ inline const double* base_pf(const double* b, int nc1) { return b + 3 * nc1; }
 __host__ __device__ inline const double* base_r(const double* b, int nc1) { return b + 4 * nc1 + 1; }
 
-// doubles of VIC scratch per interior cell: du, du0 (5 each), the blocks
+// doubles of VIC scratch per interior cell: du, du0 (5 each; of du0 the
+// explicit energy row is kept, the others are du's), the blocks
 // a, b, c (25 each), the solution and the two Woodbury vectors (5 each)
 constexpr int kVicDoublesPerCell = 100;
 // implicit-precision float32 blocks add, after the FP64 part, a part for

@@ -586,7 +586,8 @@ __device__ __forceinline__ void vic_assemble_cell(
 // Jacobians, both faces' |A|, the zeros' products), by its loads and stores
 // in FP32.  Measured per launch (us), before and now: 512 x 128 FP64 212 / 125,
 // 45 x 37 x 48 319 / 151, 301 x 75 108 / 64, nine members 330 / 210; FP32 64
-// members 418 / 305, four served requests 738 / 690 (two CTAs an SM: 374 and
+// members 418 / 258, four served requests 738 / 579 (with the tendency loaded
+// at its use 295 and 669; two CTAs an SM then 374 and
 // 874; a branch per store to either layout: 488 and 1155).
 template <typename T>
 __global__ void __launch_bounds__(AsmShape<T>::threads, AsmShape<T>::ctas)
@@ -1622,8 +1623,8 @@ __global__ void __launch_bounds__(kThreads)
 // per column, its passes on lane 0; wide batches three launches, a thread per
 // column for the passes) and now: 512 columns of 128 FP64 138 and 45, 301 of
 // 75 85 and 25, 384 of 100 FP32 106 and 35, 4,096 of 64 113 and 65, nine FP64
-// members 153 and 59, 64 members 477 and 313, four served requests 829 and
-// 670.
+// members 153 and 58, 64 members 477 and 287, four served requests 829 and
+// 612.
 constexpr int kFinThreads = 256;
 
 // a > b and a < 0 from the bit patterns: the order of the doubles, without
@@ -1639,7 +1640,7 @@ __device__ __forceinline__ bool dneg(double a) {
   return x < 0 && (x << 1) != 0;
 }
 
-__global__ void __launch_bounds__(kFinThreads, 3)
+__global__ void __launch_bounds__(kFinThreads, 4)
     vic_finish_kernel(const BlockDev* __restrict__ tab, StageParams p) {
   extern __shared__ __align__(16) unsigned char fin_smem[];
   __shared__ double sR[32], sS[32], sRS[32];
