@@ -301,6 +301,32 @@ size_t stage_smem(const sg_handle* h, const sg_block_desc& d, int tj,
   return f(d.nc1, tj, has2, wb, cov, visc);
 }
 
+// BlockDev::kd and kf: each constant formed in its own type, as the kernels'
+// expressions form it
+template <typename T>
+void fill_consts(T* k, const sg_block_desc& d) {
+  using namespace sg;
+  const T two = T(2.), one = T(1.);
+  k[kcGamma] = T(d.gammad);
+  k[kcRgm1] = one / (k[kcGamma] - one);
+  k[kcA1] = T(d.dx3 * d.dx2);
+  k[kcA2] = T(d.dx3 * d.dx1);
+  k[kcA3] = T(d.dx2 * d.dx1);
+  k[kcVol] = T(d.dx3 * (d.dx2 * d.dx1));
+  k[kcRvol] = one / k[kcVol];
+  k[kcGrav] = T(d.grav1);
+  k[kcNu] = T(d.nu_iso);
+  k[kcDx1] = T(d.dx1);
+  k[kcDx2] = T(d.dx2);
+  k[kcRdx1] = one / k[kcDx1];
+  k[kcRdx2] = one / k[kcDx2];
+  k[kcD2x1] = two * k[kcDx1];
+  k[kcD2x2] = two * k[kcDx2];
+  k[kcRd2x1] = one / k[kcD2x1];
+  k[kcRd2x2] = one / k[kcD2x2];
+  k[kcS2] = T(d.dx1 * d.dx1 / 12.);
+}
+
 // tile width: enough CTAs to cover the SMs, shared memory within one CTA's
 // opt-in limit (2 CTAs per SM where it fits)
 int choose_tj(const sg_handle* h, const sg_block_desc& d, int nblock) {
@@ -680,6 +706,7 @@ int sg_autotune(sg_handle* h, int32_t reps, int32_t* tj_out,
     p.w0 = h->scheme.wght[0][0];
     p.w1 = h->scheme.wght[0][1];
     p.w2 = h->scheme.wght[0][2];
+    p.wf[0] = (float)p.w0, p.wf[1] = (float)p.w1, p.wf[2] = (float)p.w2;
     p.dt = dt;
     p.first = 1;
     p.status = h->status;
@@ -904,6 +931,8 @@ int sg_create(const sg_scheme* scheme, const sg_block_desc* blocks,
       }
       h->implicit = true;
     }
+    fill_consts(B.kd, d);
+    fill_consts(B.kf, d);
     B.dt_src = INFINITY;
     if (d.nu_iso > 0.) {  // DiffusionImpl::max_time_step, kinematic nu
       int ndim = 0;
@@ -1401,6 +1430,7 @@ int sg_stage(sg_handle* h, int32_t stage, const double* dt_dev,
   p.w0 = h->scheme.wght[stage][0];
   p.w1 = h->scheme.wght[stage][1];
   p.w2 = h->scheme.wght[stage][2];
+  p.wf[0] = (float)p.w0, p.wf[1] = (float)p.w1, p.wf[2] = (float)p.w2;
   p.dt = dt_dev;
   p.first = stage == 0;
   p.status = h->status;

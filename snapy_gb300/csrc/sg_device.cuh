@@ -328,12 +328,13 @@ __device__ __forceinline__ void hllc_flux(const T* wl, const T* wr, T gammad,
 // LMARS face flux, ideal gas (h = p/(g-1)/rho + ...), no species
 template <typename T>
 __device__ __forceinline__ void lmars_flux(const T* wl, const T* wr, T gammad,
-                                           int d, T* flx, T* face_pressure) {
+                                           T rgm1, int d, T* flx,
+                                           T* face_pressure) {
   Axes ax = face_axes(d);
   const int ivx = ax.x, ivy = ax.y, ivz = ax.z;
   // the quotients by gamma - 1 and by each side's density divide through
-  // the reciprocals (vdiv: the same bits)
-  const T gm1 = gammad - T(1), rgm1 = T(1) / gm1;
+  // the reciprocals (vdiv: the same bits; rgm1 = 1 / (gamma - 1))
+  const T gm1 = gammad - T(1);
   const T rl0 = T(1) / wl[IDN], rr0 = T(1) / wr[IDN];
   T hl = vdiv(vdiv(wl[IPR], gm1, rgm1), wl[IDN], rl0);
   T hr = vdiv(vdiv(wr[IPR], gm1, rgm1), wr[IDN], rr0);
@@ -371,14 +372,14 @@ __device__ __forceinline__ void lmars_flux(const T* wl, const T* wr, T gammad,
 // anomaly.
 template <typename T>
 __device__ __forceinline__ void lmars_flux_anom(const T* wl, const T* wr,
-                                                T gammad, int d, T pb,
+                                                T gammad, T rgm1, int d, T pb,
                                                 T* flx) {
   Axes ax = face_axes(d);
   const int ivx = ax.x, ivy = ax.y, ivz = ax.z;
   T l0 = wl[IDN], l1 = wl[ivx], l2 = wl[ivy], l3 = wl[ivz], l4 = wl[IPR];
   T r0 = wr[IDN], r1 = wr[ivx], r2 = wr[ivy], r3 = wr[ivz], r4 = wr[IPR];
   T pl = pb + l4, pr = pb + r4;
-  const T gm1 = gammad - T(1), rgm1 = T(1) / gm1;
+  const T gm1 = gammad - T(1);
   const T rl0 = T(1) / l0, rr0 = T(1) / r0;
   T hl = vdiv(vdiv(pl, gm1, rgm1), l0, rl0);
   T hr = vdiv(vdiv(pr, gm1, rgm1), r0, rr0);

@@ -41,6 +41,22 @@ namespace {
 typedef SG_REAL real;
 constexpr int kThreads = 256;
 
+// the block's constants and the stage's RK weights in the compute type
+__device__ __forceinline__ const real* block_consts(const BlockDev& B) {
+#ifdef SG_REAL_IS_FLOAT
+  return B.kf;
+#else
+  return B.kd;
+#endif
+}
+__device__ __forceinline__ real weight(const StageParams& p, int k) {
+#ifdef SG_REAL_IS_FLOAT
+  return p.wf[k];
+#else
+  return k == 0 ? p.w0 : (k == 1 ? p.w1 : p.w2);
+#endif
+}
+
 __device__ __forceinline__ int find_block(const BlockDev* tab, int nblock,
                                           int tile) {
   int lo = 0, hi = nblock - 1;
@@ -147,14 +163,14 @@ __device__ __forceinline__ void face_states(const real* q, int vstride,
 // monitor's riemann.pstar_clamp event, src/riemann/riemann.cpp:330-339)
 template <int RK>
 __device__ __forceinline__ void riemann(const real* wl, const real* wr,
-                                        real gammad, int d, real* flx,
-                                        unsigned& nclamp) {
+                                        real gammad, real rgm1, int d,
+                                        real* flx, unsigned& nclamp) {
   if (RK == kHllc) {
     real cp;
     hllc_flux<real>(wl, wr, gammad, d, flx, &cp);
     nclamp += cp <= real(0) ? 1u : 0u;
   } else {
-    lmars_flux<real>(wl, wr, gammad, d, flx, nullptr);
+    lmars_flux<real>(wl, wr, gammad, rgm1, d, flx, nullptr);
   }
 }
 
@@ -579,7 +595,8 @@ __device__ __forceinline__ bool stage_tile(const BlockDev* __restrict__ tab,
   const real* __restrict__ uin = static_cast<const real*>(B.buf[p.in]);
   const real* __restrict__ u0 = static_cast<const real*>(B.buf[p.u0]);
   real* uout = static_cast<real*>(B.buf[p.out]);
-  const real gammad = real(B.gammad);
+  const real* KC = block_consts(B);
+  const real gammad = KC[kcGamma], rgm1 = KC[kcRgm1];
   const bool scale = p.scale != 0;
   const int il = ng, iu1 = nc1 - ng;  // interior x1 cells il..iu1-1
   const double dt = p.dt[bi];
@@ -953,12 +970,12 @@ __device__ __forceinline__ bool stage_tile(const BlockDev* __restrict__ tab,
     }
     if (pbf)
 #ifdef SG_REAL_IS_FLOAT
-      lmars_flux_anom<real>(wl, wr, gammad, 1, T.pbf[f], flx);
+      lmars_flux_anom<real>(wl, wr, gammad, rgm1, 1, T.pbf[f], flx);
 #else
-      lmars_flux_anom<real>(wl, wr, gammad, 1, real(pbf[f]), flx);
+      lmars_flux_anom<real>(wl, wr, gammad, rgm1, 1, real(pbf[f]), flx);
 #endif
     else
-      riemann<RK>(wl, wr, gammad, 1, flx, nclamp);
+      riemann<RK>(wl, wr, gammad, rgm1, 1, flx, nclamp);
     if ((fi == 0 && B.bc[0] == kBcReflecting) ||
         (fi == nx1 && B.bc[1] == kBcReflecting))
       flx[IDN] = flx[IPR] = real(0);
@@ -984,18 +1001,18 @@ __device__ __forceinline__ bool stage_tile(const BlockDev* __restrict__ tab,
         for (int v = 0; v < NHYDRO; ++v) wb_[v] = real(0.5) * (wl[v] + wr[v]);
         real pbar = wb_[IPR];
         if (pbc) pbar = pb_r(i) + pbar;  // the total
-        real enth = pbar / (gammad - real(1)) + pbar;
+        real enth = vdiv(pbar, gammad - real(1), rgm1) + pbar;
         COV[0 * cstride + jf * nc1 + i] = wb_[IDN];
         COV[1 * cstride + jf * nc1 + i] = enth / wb_[IDN];
         COV[2 * cstride + jf * nc1 + i] = wb_[IVY];
       }
       if (i >= il && i < iu1) {
         if (pbc)
-          lmars_flux_anom<real>(wl, wr, gammad, 2, pb_r(i), flx);
+          lmars_flux_anom<real>(wl, wr, gammad, rgm1, 2, pb_r(i), flx);
         else {
           // a tile's last face is the next tile's first: counted there
           unsigned c = 0;
-          riemann<RK>(wl, wr, gammad, 2, flx, c);
+          riemann<RK>(wl, wr, gammad, rgm1, 2, flx, c);
           if (jf < ntj || j0 + ntj == jend) nclamp += c;
         }
 #pragma unroll
@@ -1012,8 +1029,8 @@ __device__ __forceinline__ bool stage_tile(const BlockDev* __restrict__ tab,
     const int rlo = has2 ? 0 : 1, nr = has2 ? ntj + 2 : 1, nci = nx1 + 2;
     // quotients by a shared divisor divide through its reciprocal (vdiv:
     // the same bits)
-    const real d1 = real(2.) * real(B.dx1), d2 = real(2.) * real(B.dx2);
-    const real rd1 = real(1.) / d1, rd2 = real(1.) / d2;
+    const real d1 = KC[kcD2x1], d2 = KC[kcD2x2];
+    const real rd1 = KC[kcRd2x1], rd2 = KC[kcRd2x2];
     for (int idx = threadIdx.x; idx < nr * nci; idx += blockDim.x) {
       const int rr = rlo + idx / nci, i = il - 1 + (idx - (rr - rlo) * nci);
       const int r = hj + rr - 1;  // W row
@@ -1036,7 +1053,7 @@ __device__ __forceinline__ bool stage_tile(const BlockDev* __restrict__ tab,
 
   // (5) the x2 covariance row, then the x2 wall faces
   if (has2) {
-    const real s2 = real(B.dx1 * B.dx1 / 12.);
+    const real s2 = KC[kcS2];
     for (int idx = threadIdx.x; idx < (ntj + 1) * nx1; idx += blockDim.x) {
       const int jf = idx / nx1, ii = idx - jf * nx1, i = il + ii;
       if (L.cov) {
@@ -1061,11 +1078,11 @@ __device__ __forceinline__ bool stage_tile(const BlockDev* __restrict__ tab,
   real* VF1 = sm + L.vf1;
   real* VF2 = sm + L.vf2;
   if (visc) {
-    const real nu = real(B.nu_iso);
-    const real dx1 = real(B.dx1), dx2 = real(B.dx2);
-    const real rdx1 = real(1.) / dx1, rdx2 = real(1.) / dx2;
-    const real d2x1 = real(2.) * dx1, d2x2 = real(2.) * dx2;
-    const real rd2x1 = real(1.) / d2x1, rd2x2 = real(1.) / d2x2;
+    const real nu = KC[kcNu];
+    const real dx1 = KC[kcDx1], dx2 = KC[kcDx2];
+    const real rdx1 = KC[kcRdx1], rdx2 = KC[kcRdx2];
+    const real d2x1 = KC[kcD2x1], d2x2 = KC[kcD2x2];
+    const real rd2x1 = KC[kcRd2x1], rd2x2 = KC[kcRd2x2];
     const real* vx = W + IVX * wstride;
     const real* vy = W + IVY * wstride;
     const real* vz = W + IVZ * wstride;
@@ -1218,12 +1235,12 @@ __device__ __forceinline__ bool stage_tile(const BlockDev* __restrict__ tab,
 
   // (6) divergence, du = -dt div, gravity, viscous momentum, the x1 gravity
   // energy correction, and the RK combine on the interior cells
-  const real a1 = real(B.dx3 * B.dx2), a2 = real(B.dx3 * B.dx1);
-  const real vol = real(B.dx3 * (B.dx2 * B.dx1));
-  const real rvol = real(1.) / vol;  // every quotient by vol divides by it
-  const real rdt = real(dt), mdt = real(-dt);
-  const real w0 = real(p.w0), w1 = real(p.w1), w2 = real(p.w2);
-  const real g = real(B.grav1);
+  const real a1 = KC[kcA1], a2 = KC[kcA2];
+  const real vol = KC[kcVol];
+  const real rvol = KC[kcRvol];  // every quotient by vol divides by it
+  const real rdt = as_real<real>(dt), mdt = -rdt;
+  const real w0 = weight(p, 0), w1 = weight(p, 1), w2 = weight(p, 2);
+  const real g = KC[kcGrav];
   for (int idx = threadIdx.x; idx < ntj * nx1; idx += blockDim.x) {
     const int jt = idx / nx1, ii = idx - jt * nx1;
     const int i = il + ii;
@@ -1370,7 +1387,8 @@ __global__ void __launch_bounds__(kLineThreads)
   const real* __restrict__ uin = static_cast<const real*>(B.buf[p.in]);
   const real* __restrict__ u0 = static_cast<const real*>(B.buf[p.u0]);
   real* uout = static_cast<real*>(B.buf[p.out]);
-  const real gammad = real(B.gammad);
+  const real* KC = block_consts(B);
+  const real gammad = KC[kcGamma], rgm1 = KC[kcRgm1];
   const bool scale = p.scale != 0;
   const double dt = p.dt[bi];
   const int c0 = ng + x0 - 3;  // the block cell of W's first
@@ -1406,7 +1424,7 @@ __global__ void __launch_bounds__(kLineThreads)
 #pragma unroll
     for (int v = 0; v < NHYDRO; ++v) wl[v] = WL[v][f], wr[v] = WR[v][f];
     unsigned c = 0;
-    riemann<RK>(wl, wr, gammad, 1, flx, c);
+    riemann<RK>(wl, wr, gammad, rgm1, 1, flx, c);
     // a segment's last face is the next one's first: counted and posted there
     const bool own = f < n || last;
     if (own) nclamp += c;
@@ -1427,9 +1445,9 @@ __global__ void __launch_bounds__(kLineThreads)
     }
   }
   __syncthreads();
-  const real a1 = real(B.dx3 * B.dx2), vol = real(B.dx3 * (B.dx2 * B.dx1));
-  const real rvol = real(1.) / vol, mdt = real(-dt);
-  const real w0 = real(p.w0), w1 = real(p.w1), w2 = real(p.w2);
+  const real a1 = KC[kcA1], vol = KC[kcVol], rvol = KC[kcRvol];
+  const real mdt = -as_real<real>(dt);
+  const real w0 = weight(p, 0), w1 = weight(p, 1), w2 = weight(p, 2);
   for (int idx = threadIdx.x; idx < NHYDRO * n; idx += kLineThreads) {
     const int v = idx / n, i = idx - v * n;
     const real dv = a1 * F[v][i + 1] - a1 * F[v][i];
@@ -1569,7 +1587,8 @@ __global__ void __launch_bounds__(kThreads)
   const real* u = static_cast<const real*>(B.buf[p.in]);
   const real* s = static_cast<const real*>(B.sbuf[p.in]);
   const real* rb = base_rho_real(B);
-  const real gammad = real(B.gammad);
+  const real* KC = block_consts(B);
+  const real gammad = KC[kcGamma], rgm1 = KC[kcRgm1];
   const bool scale = p.scale != 0;
   const bool covs = B.flux_cov && nc1 >= 3;
   // the total dry density (the state holds an anomaly under a base)
@@ -1986,11 +2005,12 @@ __global__ void __launch_bounds__(kX3Threads)
   const int nch = (nx3 + chunk - 1) / chunk;
   const size_t plane = (size_t)nc1 * nc2 * nc3, kst = (size_t)nc1 * nc2;
   const real* __restrict__ uin = static_cast<const real*>(B.buf[p.in]);
-  const real gammad = real(B.gammad);
+  const real* KC = block_consts(B);
+  const real gammad = KC[kcGamma], rgm1 = KC[kcRgm1];
   const bool scale = p.scale != 0;
   const double* rb = B.base ? base_rho(B.base, nc1) : nullptr;
   const double* pbc = B.base ? base_p(B.base, nc1) : nullptr;
-  const real a3 = real(B.dx2 * B.dx1);
+  const real a3 = KC[kcA3];
   const bool wlo = B.bc[4] == kBcReflecting, whi = B.bc[5] == kBcReflecting;
   // the covariance row of the x3 faces (_flux_covariance, dim 3) needs each
   // face's mean state on the x1 rows either side: a warp then covers 32
@@ -2034,6 +2054,9 @@ __global__ void __launch_bounds__(kX3Threads)
       if (rb) uc[IDN] = real(rb[i]) + uc[IDN];
       cons2prim<real>(uc, w, gammad);
     };
+    // the covariance row's x1 spacing either side of the row
+    const real cdx1 = cov && own ? real(B.x1v[i + 1] - B.x1v[i - 1]) : real(1.);
+    const real crdx1 = real(1.) / cdx1;
     // window: cells f-3 .. f+2 of face f
     real W[6][NHYDRO];
 #pragma unroll
@@ -2061,29 +2084,26 @@ __global__ void __launch_bounds__(kX3Threads)
 #pragma unroll
         for (int v = 0; v < NHYDRO; ++v) wb_[v] = real(0.5) * (wl[v] + wr[v]);
         real pbar = wb_[IPR];
-        if (pbc) pbar = real(pbc[i]) + pbar;
-        const real enth = pbar / (gammad - real(1)) + pbar;
+        if (pbc) pbar = pb + pbar;
+        const real enth = vdiv(pbar, gammad - real(1), rgm1) + pbar;
         const real hh = enth / wb_[IDN], un = wb_[IVZ];
         const unsigned full = 0xffffffffu;
         const real hm = __shfl_up_sync(full, hh, 1), hp = __shfl_down_sync(full, hh, 1);
         const real um = __shfl_up_sync(full, un, 1), up = __shfl_down_sync(full, un, 1);
         if (own) {
-          const real dx1 = real(B.x1v[i + 1] - B.x1v[i - 1]);
-          const real s2 = real(B.dx1 * B.dx1 / 12.);
-          const real s2rho = s2 * wb_[IDN];
-          const real rdx1 = real(1.) / dx1;
-          const real d1h = vdiv(hp - hm, dx1, rdx1);
-          const real dun = vdiv(up - um, dx1, rdx1);
+          const real s2rho = KC[kcS2] * wb_[IDN];
+          const real d1h = vdiv(hp - hm, cdx1, crdx1);
+          const real dun = vdiv(up - um, cdx1, crdx1);
           dcov = s2rho * d1h * dun;
         }
       }
       if (pbc)
-        lmars_flux_anom<real>(wl, wr, gammad, 3, pb, flx);
+        lmars_flux_anom<real>(wl, wr, gammad, rgm1, 3, pb, flx);
       else {
         // a chunk owns its faces but the top one (the next chunk's), except
         // the block's last face
         unsigned c = 0;
-        riemann<RK>(wl, wr, gammad, 3, flx, c);
+        riemann<RK>(wl, wr, gammad, rgm1, 3, flx, c);
         if (c && own && (f < k1 || k1 == ng + nx3) && p.counts)
           atomicAdd(&p.counts[blockIdx.y * kCountSlots + kCountPstar], 1ull);
       }
@@ -2104,7 +2124,7 @@ __global__ void __launch_bounds__(kX3Threads)
       if (visc) {
         const size_t c = (size_t)f * kst + col, cm = c - kst;
         const real* VP = static_cast<const real*>(B.visc3);
-        const real nu = real(B.nu_iso);
+        const real nu = KC[kcNu];
         const real dx3 = real(B.dx3), rdx3 = real(1.) / dx3;
         const real rf = real(0.5) * (W[3][IDN] + W[2][IDN]);
         const real divf = real(0.5) * (VP[c] + VP[cm]);

@@ -21,8 +21,21 @@ enum BcKind : int32_t {
 
 enum RiemannKind : int32_t { kHllc = 0, kLmars = 1 };
 
+// indices of BlockDev::kd, kf: gamma, 1 / (gamma - 1), the face areas and the
+// cell volume with its reciprocal, x1 gravity, nu, dx and 2 dx of x1 and x2 with
+// their reciprocals, dx1^2 / 12
+enum BlockConst : int {
+  kcGamma, kcRgm1, kcA1, kcA2, kcA3, kcVol, kcRvol, kcGrav, kcNu, kcDx1, kcDx2,
+  kcRdx1, kcRdx2, kcD2x1, kcD2x2, kcRd2x1, kcRd2x2, kcS2
+};
+
 // one block of the batch, as the device sees it
 struct BlockDev {
+  // constants of the block in both types (fill_consts): formed per thread
+  // they would be some forty FP64 instructions of every tile, conversions and
+  // divisions, on the pipe that a FP32 tile otherwise leaves alone
+  double kd[18];
+  float kf[18];
   void* buf[3];         // (nvar, nc3, nc2, nc1) state buffers, storage dtype
   int32_t nc1, nc2, nc3, ng;
   int32_t tj;           // x2 columns per tile
@@ -181,6 +194,7 @@ struct StageParams {
   int32_t shock;        // 1: every row weno5
   int32_t scale;        // InterpOptions::scale
   double w0, w1, w2;    // RK weights of this stage
+  float wf[3];          // and in FP32
   const double* dt;     // device scalar: the host dt or a captured graph's
   int32_t first;        // stage 0: the step fields start from zero
   int32_t refine;       // corrections of the refined implicit solve of
