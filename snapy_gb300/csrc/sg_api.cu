@@ -236,7 +236,7 @@ struct sg_handle {
   int32_t nblock = 0, ntile = 0;
   int32_t cur = 0, base = 0;  // current buffer, stage-0 buffer
   bool bound_all = false, dirty = true;
-  size_t smem = 0, max_plane = 0, max_cells = 0;
+  size_t smem = 0, max_plane = 0, max_cells = 0, max_ghost = 0;
   int32_t max_nc1 = 0;
   int32_t launches = 0;
   int* status = nullptr;  // per-block solve status bits (VIC failures)
@@ -1056,6 +1056,7 @@ int sg_create(const sg_scheme* scheme, const sg_block_desc* blocks,
     size_t icols = (size_t)(d.nc2 > 1 ? d.nc2 - 2 * d.ng : 1) *
                    (size_t)(d.nc3 > 1 ? d.nc3 - 2 * d.ng : 1);
     size_t icells = (size_t)(d.nc1 - 2 * d.ng) * icols;
+    h->max_ghost = std::max(h->max_ghost, plane - icells);
     // the block's scratch: the implicit solve's FP64 arrays, then (3-D) the
     // x3 flux differences a3 dF3 of every interior cell in the storage type
     size_t vic_bytes = d.implicit_scheme ? icells * sg::kVicDoublesPerCell *
@@ -1526,8 +1527,8 @@ int sg_stage(sg_handle* h, int32_t stage, const double* dt_dev,
     // (implicit blocks: and the solve's transfer)
     launches += h->implicit ? 6 : 5;
   }
-  rc = f64(h) ? sg_launch_ghost_f64(h->dev, h->nblock, out, h->max_plane, s)
-              : sg_launch_ghost_f32(h->dev, h->nblock, out, h->max_plane, s);
+  rc = f64(h) ? sg_launch_ghost_f64(h->dev, h->nblock, out, h->max_ghost, s)
+              : sg_launch_ghost_f32(h->dev, h->nblock, out, h->max_ghost, s);
   if (rc) return cuda_fail((cudaError_t)rc, "sg_stage: ghost kernel");
   if (h->scalars) {
     rc = f64(h) ? sg_launch_scalar_ghost_f64(h->dev, h->nblock, out,
@@ -1569,8 +1570,8 @@ int sg_fill_ghosts(sg_handle* h, sg_stream_t stream) {
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   int rc = upload(h, s);
   if (rc) return rc;
-  rc = f64(h) ? sg_launch_ghost_f64(h->dev, h->nblock, h->cur, h->max_plane, s)
-              : sg_launch_ghost_f32(h->dev, h->nblock, h->cur, h->max_plane, s);
+  rc = f64(h) ? sg_launch_ghost_f64(h->dev, h->nblock, h->cur, h->max_ghost, s)
+              : sg_launch_ghost_f32(h->dev, h->nblock, h->cur, h->max_ghost, s);
   if (rc) return cuda_fail((cudaError_t)rc, "sg_fill_ghosts");
   if (h->scalars) {
     rc = f64(h) ? sg_launch_scalar_ghost_f64(h->dev, h->nblock, h->cur,
