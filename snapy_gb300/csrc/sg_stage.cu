@@ -2825,14 +2825,22 @@ extern "C" int SG_NAME(sg_launch_vic)(const BlockDev* tab, StageParams p,
   if (ev) cudaEventRecord(ev[1], stream);
   const size_t fin = (size_t)p.fin_len * sizeof(double) *
                      (kFinArrays + ((p.vic_kinds & 2) ? kFinPartial : 0));
-  static size_t fin_granted[64] = {};
+  // the opt-in shared memory, all that a CTA may have: threads with handles
+  // of different lengths set the same value
+  static bool fin_granted[64] = {};
   int fin_dev = 0;
   cudaGetDevice(&fin_dev);
-  if (fin_dev >= 64 || fin > fin_granted[fin_dev]) {
-    e = cudaFuncSetAttribute(vic_finish_kernel,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fin);
+  if (fin_dev >= 64 || !fin_granted[fin_dev]) {
+    int most = 0;
+    cudaFuncAttributes at;
+    e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, fin_dev);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, vic_finish_kernel);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(vic_finish_kernel,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               most - (int)at.sharedSizeBytes);
     if (e != cudaSuccess) return (int)e;
-    if (fin_dev < 64) fin_granted[fin_dev] = fin;
+    if (fin_dev < 64) fin_granted[fin_dev] = true;
   }
   vic_finish_kernel<<<dim3(p.fin_ctas, p.nblock), kFinThreads, fin, stream>>>(tab, p);
   return (int)cudaGetLastError();
