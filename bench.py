@@ -260,6 +260,13 @@ def refined(opts):
                 and ic.precision == "float32" and opts.solve_corrections() > 0)
 
 
+def block_bytes(opts):
+    """The bytes of a cell's A, B and C blocks as the assembly writes them."""
+    ic = opts.hydro().icorr
+    return 300 if (ic is not None and opts.hydro().precision == "float32"
+                   and ic.precision == "float32") else 600
+
+
 def solve_phase(opts):
     """The implicit solve phase timed as vic_solve_kernel (the events
     between the assembly and the finish): what runs in it, its algorithmic
@@ -274,18 +281,21 @@ def solve_phase(opts):
         return ("vic_solve_kernel", 600 + 40 + 200 + 120 + 200 + 120 + 120,
                 FP64_ISSUE)
     k = opts.solve_corrections()
-    # the FP32 sweep: A, B, C (300) and du (40) in; factors (128), c' (112),
-    # y (60) and x (120) out; back: c' and y in
-    first = 300 + 40 + 128 + 112 + 60 + 120 + 112 + 60
-    # a residual: FP64 blocks (600), x (120), du (40) in; r (60) out
-    residual = 600 + 120 + 40 + 60
-    # a correction: factors, b, r in and y out; back: c', y, x in, x out
-    correct = 128 + 112 + 64 + 60 + 112 + 60 + 120 + 120
-    return (f"refined solve phase: vic_solve32_kernel, then {k} x "
-            "(vic_residual_kernel, vic_correct32_kernel)",
-            first + k * (residual + correct),
-            "the FP64 residuals (FP64 issue rate) and the corrections' "
-            "per-layer latency")
+    # the first sweep: A, B, C (300) and du (40) in; the inverses and C', B'
+    # (200) and y (20) out; back out: C', B' and y in, x (20) out
+    first = 300 + 40 + 200 + 20 + 120 + 20
+    # a residual: the FP32 blocks, x or d (20), du or the last r (40) in; the
+    # FP32 r (20) out, and all but the last the FP64 r (40)
+    residual = 300 + 20 + 40 + 20
+    # a correction: the inverses, the coupling blocks (200) and r in, y out;
+    # back out: C', B' and y in, d (20) out
+    correct = 200 + 20 + 20 + 120 + 20
+    # the sum: x and every d in, D (40) out
+    total = 20 * (k + 1) + 40
+    return (f"refined solve phase: vic_factor32_kernel, {k} x "
+            "(vic_residual_kernel, vic_correct32_kernel), vic_sum_kernel",
+            first + k * (residual + correct) + 40 * (k - 1) + total,
+            "the bytes and issue slots of the sweeps and residuals")
 
 
 def peaks():
@@ -534,9 +544,9 @@ def run_native(args):
     per_launch = {
         "stage_kernel": ((5 * s_bytes + 40) if implicit else
                          5 * s_bytes * (2 + 3 + 3) / 3) * cells,
-        "vic_assemble_kernel": (5 * s_bytes + 40 + 40 + 600) * cells,
+        "vic_assemble_kernel": (5 * s_bytes + 40 + 8 + block_bytes(opts)) * cells,
         "vic_solve_kernel": solve_phase(opts)[1] * cells,
-        "vic_finish_kernel": (120 + 15 * s_bytes) * cells,
+        "vic_finish_kernel": (88 + 15 * s_bytes) * cells,
         "ghost_kernel": 2 * 5 * s_bytes * ghost_cells,
         # per tracer: s read twice (faces, update) and s0, s_out written, the
         # two FP64 face fluxes written and read; the mass fluxes and rho once
@@ -732,9 +742,10 @@ def run_ensemble(args, ranks=None, emit=True):
     s_bytes = 4 if precision == "float32" else 8
     per_launch = {
         "stage_kernel": (5 * s_bytes + 40) * cells,
-        "vic_assemble_kernel": (5 * s_bytes + 40 + 40 + 600) * cells,
+        "vic_assemble_kernel": (5 * s_bytes + 40 + 8 +
+                                block_bytes(members[0][0])) * cells,
         "vic_solve_kernel": solve_phase(members[0][0])[1] * cells,
-        "vic_finish_kernel": (120 + 15 * s_bytes) * cells,
+        "vic_finish_kernel": (88 + 15 * s_bytes) * cells,
         "ghost_kernel": 0,
     }
     dom = max(kt, key=lambda k: kt[k][0])
@@ -1173,8 +1184,8 @@ def serving_scratch(opts):
     """Bytes of implementation scratch (the implicit solve's and the x3
     sweep's) moved per interior cell per RK3 step: not algorithmic."""
     c = opts.coord()
-    per_stage = solve_phase(opts)[1] + (40 + 600 + 40)  # solve phase, assembly
-    per_stage += 120  # the finish's D, du, du0
+    per_stage = solve_phase(opts)[1] + (40 + block_bytes(opts) + 8)  # and assembly
+    per_stage += 88  # the finish's D, du, du0's energy row
     if c.nx3 > 1:
         per_stage += 2 * 5 * 4  # a3 dF3 written and read
     return 3 * per_stage
