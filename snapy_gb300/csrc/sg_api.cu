@@ -237,7 +237,8 @@ struct sg_handle {
   int32_t cur = 0, base = 0;  // current buffer, stage-0 buffer
   bool bound_all = false, dirty = true;
   size_t smem = 0, max_plane = 0, max_cells = 0, max_ghost = 0;
-  int32_t max_nc1 = 0;
+  int max_inx1 = 0;  // the longest column of an implicit block
+  int res_ctas = 1;  // the refined solve's CTAs of eight layers a tile
   int32_t launches = 0;
   int* status = nullptr;  // per-block solve status bits (VIC failures)
   unsigned long long* fallbacks = nullptr;  // per block: refined-solve
@@ -382,7 +383,9 @@ void plan_x3(sg_handle* h) {
 // its shared arrays): the fewest that leave at most two CTAs an SM, up to
 // kFinLen; form 2 takes twice as many.  The serial passes cost a CTA the same
 // for one column or 32, and with one CTA's worth of warps on an SM nothing
-// hides them.  Measured per launch (us) with 1 / 2 / 4 / 8 / 16 / 32 columns:
+// hides them.  One column at least fits a CTA: only the implicit blocks'
+// columns count, and their own tile (sg_stage_bound) holds them to about 2,200
+// layers, 89 KB here (the partial matrix 125 KB).  Measured per launch (us) with 1 / 2 / 4 / 8 / 16 / 32 columns:
 // 512 columns of 128, FP64: 73 / 44 / 45 / 61 / 91 / -; 301 of 75: 26 / 25 /
 // 32 / 40 / 56 / 94; 1,665 of 48: 106 / 58 / 49 / 37 / 39 / 63; 4,096 of 64,
 // FP32: 313 / 168 / 113 / 84 / 67 / 90.  kFinLen of 516 / 1032 / 1376 / 2064
@@ -404,7 +407,7 @@ void plan_finish(sg_handle* h) {
       most = std::max(most, n);
     }
   };
-  const int one = sg::fin_pitch(h->max_nc1 - 6);
+  const int one = sg::fin_pitch(h->max_inx1);
   const int top = std::max(one, sg::kFinLen);
   int len = one;
   for (count(len); ctas > 2 * (size_t)sms && len < top; count(len))
@@ -713,7 +716,7 @@ int sg_autotune(sg_handle* h, int32_t reps, int32_t* tj_out,
     p.refine = h->refine;
     p.psw = h->psw_on;
     p.fallbacks = h->fallbacks;
-    p.max_nc1 = h->max_nc1;
+    p.res_ctas = h->res_ctas;
     p.asm_ctas[0] = h->asm_ctas[0];
     p.asm_ctas[1] = h->asm_ctas[1];
     p.solve_ctas = h->solve_ctas;
@@ -1052,7 +1055,6 @@ int sg_create(const sg_scheme* scheme, const sg_block_desc* blocks,
     size_t plane = (size_t)d.nc1 * d.nc2 * d.nc3;
     h->max_plane = std::max(h->max_plane, plane);
     h->max_cells = std::max(h->max_cells, plane);
-    h->max_nc1 = std::max(h->max_nc1, d.nc1);
     size_t icols = (size_t)(d.nc2 > 1 ? d.nc2 - 2 * d.ng : 1) *
                    (size_t)(d.nc3 > 1 ? d.nc3 - 2 * d.ng : 1);
     size_t icells = (size_t)(d.nc1 - 2 * d.ng) * icols;
@@ -1099,6 +1101,11 @@ int sg_create(const sg_scheme* scheme, const sg_block_desc* blocks,
       B.asmc[5] = 1. / (gm1r + 1.);
       h->max_icells = std::max(h->max_icells, icells);
       h->max_icols = std::max(h->max_icols, icols);
+      const int nx1 = d.nc1 - 2 * d.ng;
+      h->max_inx1 = std::max(h->max_inx1, nx1);
+      if (B.implicit_f32 && d.implicit_scheme == 9)
+        h->res_ctas = std::max(h->res_ctas,
+                               (int)((icols + 31) / 32) * ((nx1 + 7) / 8));
     }
   }
   h->ntile = tile;
@@ -1439,7 +1446,7 @@ int sg_stage(sg_handle* h, int32_t stage, const double* dt_dev,
   p.counts = h->counts;
   p.psw = h->psw_on;
   p.fallbacks = h->fallbacks;
-  p.max_nc1 = h->max_nc1;
+  p.res_ctas = h->res_ctas;
   p.asm_ctas[0] = h->asm_ctas[0];
   p.asm_ctas[1] = h->asm_ctas[1];
   p.solve_ctas = h->solve_ctas;

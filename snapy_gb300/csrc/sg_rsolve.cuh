@@ -189,6 +189,15 @@ __device__ __forceinline__ bool rtile_at(const BlockDev* __restrict__ tab,
   return true;
 }
 
+// the tile and the first of the eight layers that CTA blockIdx.x takes
+__device__ __forceinline__ bool rtile_layers(const BlockDev* __restrict__ tab,
+                                             RTile& t, int& i0) {
+  const BlockDev& B = tab[blockIdx.y];
+  const unsigned lg = (unsigned)(B.nc1 - 2 * B.ng + 7) / 8, x = blockIdx.x / lg;
+  i0 = 8 * (int)(blockIdx.x - x * lg);
+  return rtile_at(tab, x, t) && t.n >= 5;
+}
+
 // what the two warps of a tile trade: the upper side's relation at the
 // middle, the middle's solution, each side's column flags and largest |x|
 struct MeetSmem {
@@ -580,14 +589,15 @@ __device__ __forceinline__ void residual_row(const RTile& T, int i, int corr,
   }
 }
 
-// eight layers of a tile per CTA (lg CTAs a tile)
+// eight layers of a tile per CTA
 template <bool FIRST>
 __global__ void __launch_bounds__(kThreads, 3)
     vic_residual_kernel(const BlockDev* __restrict__ tab, StageParams p,
-                        int corr, int lg) {
+                        int corr) {
   RTile T;
-  if (!rtile_at(tab, blockIdx.x / lg, T) || T.n < 5) return;
-  const int i = 8 * (int)(blockIdx.x % lg) + (threadIdx.x >> 5);
+  int i0;
+  if (!rtile_layers(tab, T, i0)) return;
+  const int i = i0 + (threadIdx.x >> 5);
   if (i >= T.n) return;
   const bool keep = corr < p.refine;  // a later correction reads r
   const double dtc = p.w2 * p.dt[blockIdx.y];
@@ -741,12 +751,11 @@ __global__ void __launch_bounds__(64)
 // corrections), eight layers of a tile per CTA: read by rows of columns,
 // written by columns (40 consecutive values) through shared memory
 __global__ void __launch_bounds__(kThreads)
-    vic_sum_kernel(const BlockDev* __restrict__ tab, StageParams p, int lg) {
+    vic_sum_kernel(const BlockDev* __restrict__ tab, StageParams p) {
   __shared__ double s[32][41];
   RTile T;
-  if (!rtile_at(tab, blockIdx.x / lg, T) || T.n < 5) return;
-  const int i0 = 8 * (int)(blockIdx.x % lg);
-  if (i0 >= T.n) return;
+  int i0;
+  if (!rtile_layers(tab, T, i0)) return;
   const int lane = threadIdx.x & 31, q = threadIdx.x >> 5, w = T.w;
   const int nk = p.refine > 0 ? p.refine : 0;
   if (i0 + q < T.n && lane < w) {

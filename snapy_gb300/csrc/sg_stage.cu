@@ -2766,7 +2766,6 @@ extern "C" int SG_NAME(sg_launch_vic)(const BlockDev* tab, StageParams p,
   int gs = (int)((max_cols + kVicCols - 1) / kVicCols);
   if (p.refine) {
     const unsigned gt = (unsigned)((max_cols + 31) / 32);  // tiles of columns
-    const int lg = (p.max_nc1 - 6 + 7) / 8;  // CTAs of eight layers a tile
     // the rings' opt-in shared memory, once a device (a handle's first launch
     // is eager)
     static bool granted[64] = {};
@@ -2787,11 +2786,11 @@ extern "C" int SG_NAME(sg_launch_vic)(const BlockDev* tab, StageParams p,
                           stream>>>(tab, p);
     for (int k = 1; k <= p.refine; ++k) {
       (k == 1 ? vic_residual_kernel<true> : vic_residual_kernel<false>)
-          <<<dim3(gt * lg, p.nblock), kThreads, 0, stream>>>(tab, p, k, lg);
+          <<<dim3(p.res_ctas, p.nblock), kThreads, 0, stream>>>(tab, p, k);
       vic_correct32_kernel<<<dim3(gt, p.nblock), 64, kCorFloats * sizeof(float),
                              stream>>>(tab, p, k);
     }
-    vic_sum_kernel<<<dim3(gt * lg, p.nblock), kThreads, 0, stream>>>(tab, p, lg);
+    vic_sum_kernel<<<dim3(p.res_ctas, p.nblock), kThreads, 0, stream>>>(tab, p);
     // the columns left to FP64: the partitioned FP64 solve first (a warp
     // per column, four chunks at once), the serial one for what it cannot
     const size_t share = (max_cols * p.nblock + 4095) / 4096;

@@ -206,7 +206,8 @@ struct StageParams {
   int32_t* status;      // per-block status bits (kStatusStaging: a tile's
                         // staging wait ran out)
   int32_t smem_rows;    // x1 lines held in shared memory per tile
-  int32_t max_nc1;
+  int32_t res_ctas;     // the refined solve's CTAs of eight layers a tile, per
+                        // block
   int32_t asm_ctas[2];  // the assembly's CTAs per block: FP64, FP32
   int32_t solve_ctas;   // the direct solve's CTAs per block
   int32_t fin_len;      // doubles of a finish CTA's array
