@@ -206,8 +206,8 @@ def implicit_solve(opts):
                     "residuals, the FP64 solve for columns that do not converge")
         if opts.implicit_solve == "fp32":
             return ("FP32 (the reference's FP32 implicit compute): the FP32 "
-                    "block-Thomas sweep and its Woodbury step, the FP64 solve "
-                    "for columns whose sweep fails")
+                    "block elimination and one correction accepted to FP32's "
+                    "rounding, the FP64 solve for columns that fail")
     if opts.implicit_sweep == "partitioned":
         return ("direct FP64, partitioned: four chunks per column swept at "
                 "once, a separator system, then every layer")

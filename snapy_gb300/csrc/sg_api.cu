@@ -257,7 +257,7 @@ struct sg_handle {
   int vic_kinds = 0;  // bit 0: a block with the full 5x5 matrix, bit 1: 3x3
   bool ref32 = false;  // an FP32 block under gravity: base_ref_kernel runs
   int asm_kinds = 0;   // implicit blocks assembled in FP64 (bit 0), FP32 (1)
-  int refine = 0;  // corrections of the refined implicit solve (0: direct)
+  int refine = 0;  // sg_set_solve's corrections (0: direct, -1: FP32 form)
   // the partitioned form of the scheme-9 solve of FP64-assembled blocks:
   // the requested mode (sg_set_sweep: 0 serial, 1 partitioned, 2 the
   // autotuner's choice), whether it runs now, and its region (per block,
@@ -292,6 +292,12 @@ struct sg_handle {
 namespace {
 
 bool f64(const sg_handle* h) { return h->scheme.dtype == SG_F64; }
+
+// the corrections and the acceptance of sg_set_solve's forms
+void set_solve_params(const sg_handle* h, StageParams& p) {
+  p.refine = h->refine < 0 ? 1 : h->refine;
+  p.accept = h->refine < 0 ? 0x1p-24f : 0x1p-44f;
+}
 
 size_t stage_smem(const sg_handle* h, const sg_block_desc& d, int tj,
                   bool bound = false) {
@@ -713,7 +719,7 @@ int sg_autotune(sg_handle* h, int32_t reps, int32_t* tj_out,
     p.dt = dt;
     p.first = 1;
     p.status = h->status;
-    p.refine = h->refine;
+    set_solve_params(h, p);
     p.psw = h->psw_on;
     p.fallbacks = h->fallbacks;
     p.res_ctas = h->res_ctas;
@@ -1442,7 +1448,7 @@ int sg_stage(sg_handle* h, int32_t stage, const double* dt_dev,
   p.dt = dt_dev;
   p.first = stage == 0;
   p.status = h->status;
-  p.refine = h->refine;
+  set_solve_params(h, p);
   p.counts = h->counts;
   p.psw = h->psw_on;
   p.fallbacks = h->fallbacks;
@@ -1517,7 +1523,7 @@ int sg_stage(sg_handle* h, int32_t stage, const double* dt_dev,
     // columns' solve
     launches += 3 + (h->vic_kinds == 3 ? 1 : 0) +
                 (h->asm_kinds == 3 ? 1 : 0) +
-                (h->refine ? 3 + 2 * std::max(h->refine, 0) : 0) +
+                (p.refine ? 3 + 2 * p.refine : 0) +
                 (h->psw_on ? 1 : 0);
   }
   if (h->scalars) {

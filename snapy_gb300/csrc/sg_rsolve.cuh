@@ -8,7 +8,11 @@
 // layer n - 1's that of layer n - 3), and b = du / dt_corr.  It is solved by
 // mixed-precision iterative refinement (the scheme of LAPACK's dsgesv): an
 // FP32 solve M^-1, then p.refine corrections d = M^-1 r with r = b - T x
-// formed beyond FP64 accuracy and x summed in FP64.
+// formed beyond FP64 accuracy and x summed in FP64.  The last correction's
+// size and its gain estimate the error it leaves; p.accept bounds it.  The
+// FP32 form (sg_set_solve -1) makes one correction and accepts FP32's
+// rounding, 2^-24 of the solution: M^-1 alone can lose digits in a strong
+// wind, which nothing would show.
 //
 //   vic_factor32_kernel    M^-1's factors and the first solution
 //   vic_residual_kernel    r = b - T x (or the previous r less T d)
@@ -33,8 +37,8 @@
 // mean and worst: 1e-7 to 3e-6 and 9e-5 (with scaled partial pivoting 1e-7 to
 // 1e-6 and 6e-5; tangential momenta before the energy 1e-7 to 3e-5 and 3e-3,
 // which left one column in eleven to FP64).  A pivot that cancels to below 40 eps
-// of its diagonal, a value that is not finite, or an estimated error above 2^-44
-// of the solution after the last correction masks the column,
+// of its diagonal, a value that is not finite, or an estimated error above
+// p.accept (2^-44) of the solution masks the column,
 // and it takes the FP64 solve (vic_psolve_kernel, vic_solve_kernel), as the
 // reference retries a failed FP32 column in FP64 (src/hydro/hydro.cpp:436-466).
 //
@@ -327,7 +331,7 @@ __device__ __forceinline__ unsigned sweep_out(const float* CP, const float* Y,
 // width at compile time (32), or 0 to take it from the tile
 template <int W>
 __device__ __forceinline__ void factor_tile(const RTile& T, const StageParams& p,
-                                            bool last, MeetSmem& sm, float* ring) {
+                                            MeetSmem& sm, float* ring) {
   const int w = W ? W : T.w, n = T.n, m = T.m;
   const int lane = threadIdx.x & 31;
   const bool up = threadIdx.x >= 32;
@@ -467,8 +471,7 @@ __device__ __forceinline__ void factor_tile(const RTile& T, const StageParams& p
   if (up || !on) return;
   mx = max(mx, sm.mx[1][lane]);
   T.stat[lane * 6] = __uint_as_float(mx);
-  const bool fin = sm.ok[0][lane] && sm.ok[1][lane] && (mx < kInfBits || !last);
-  T.mask[lane] = fin ? 0 : 1;
+  T.mask[lane] = sm.ok[0][lane] && sm.ok[1][lane] ? 0 : 1;
 }
 
 __global__ void __launch_bounds__(64)
@@ -482,11 +485,10 @@ __global__ void __launch_bounds__(64)
     return;
   }
   float* ring = reinterpret_cast<float*>(smem_raw);
-  const bool last = p.refine < 0;  // no corrections: accepted where finite
   if (T.w == 32)
-    factor_tile<32>(T, p, last, sm, ring);
+    factor_tile<32>(T, p, sm, ring);
   else
-    factor_tile<0>(T, p, last, sm, ring);
+    factor_tile<0>(T, p, sm, ring);
 }
 
 // s_h + s_l += t d in float-float arithmetic, t and d floats: the product
@@ -617,10 +619,10 @@ __global__ void __launch_bounds__(kThreads, 3)
 // A correction's sweeps of a tile, the factor's on r with its factors, and
 // after the last one the column's acceptance: the error it leaves is about
 // |d| rho, rho = |d| / |d_prev| the observed contraction, accepted at or
-// below 2^-44 of the largest |x|
+// below p.accept of the largest |x|
 template <int W>
-__device__ __forceinline__ void correct_tile(const RTile& T, int corr, int nk,
-                                             MeetSmem& sm, float* ring) {
+__device__ __forceinline__ void correct_tile(const RTile& T, const StageParams& p,
+                                             int corr, MeetSmem& sm, float* ring) {
   const int w = W ? W : T.w, n = T.n, m = T.m;
   const int lane = threadIdx.x & 31;
   const bool up = threadIdx.x >= 32;
@@ -733,9 +735,9 @@ __device__ __forceinline__ void correct_tile(const RTile& T, int corr, int nk,
   const float dl = __uint_as_float(mx), dp = st[corr - 1];
   st[corr] = dl;
   bool fin = mx < kInfBits;
-  if (corr == nk) {
+  if (corr == p.refine) {
     const float rho = dp > 0.f ? fminf(dl / dp, 1.f) : 0.f;
-    fin = fin && dl * rho <= 0x1p-44f * st[0];
+    fin = fin && dl * rho <= p.accept * st[0];
   }
   if (!fin) T.mask[lane] = 1;
 }
@@ -749,14 +751,13 @@ __global__ void __launch_bounds__(64)
   if (!rtile_at(tab, blockIdx.x, T) || T.n < 5) return;
   float* ring = reinterpret_cast<float*>(smem_raw);
   if (T.w == 32)
-    correct_tile<32>(T, corr, p.refine, sm, ring);
+    correct_tile<32>(T, p, corr, sm, ring);
   else
-    correct_tile<0>(T, corr, p.refine, sm, ring);
+    correct_tile<0>(T, p, corr, sm, ring);
 }
 
-// D = x0 + d1 + ... in FP64 (the FP32 solve, p.refine < 0, has no
-// corrections), eight layers of a tile per CTA: read by rows of columns,
-// written by columns (40 consecutive values) through shared memory
+// D = x0 + d1 + ... in FP64, eight layers of a tile per CTA: read by rows of
+// columns, written by columns (40 consecutive values) through shared memory
 __global__ void __launch_bounds__(kThreads)
     vic_sum_kernel(const BlockDev* __restrict__ tab, StageParams p) {
   __shared__ double s[32][41];
@@ -764,7 +765,7 @@ __global__ void __launch_bounds__(kThreads)
   int i0;
   if (!rtile_layers(tab, T, i0)) return;
   const int lane = threadIdx.x & 31, q = threadIdx.x >> 5, w = T.w;
-  const int nk = p.refine > 0 ? p.refine : 0;
+  const int nk = p.refine;
   if (i0 + q < T.n && lane < w) {
     const size_t o = (size_t)(i0 + q) * VicTile::chunk(5, w) + lane;
     float x[4][5];

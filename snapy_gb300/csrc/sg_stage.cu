@@ -2761,8 +2761,8 @@ extern "C" int SG_NAME(sg_launch_vic)(const BlockDev* tab, StageParams p,
   if (e != cudaSuccess) return (int)e;
   if (ev) cudaEventRecord(ev[0], stream);
   // implicit-precision float32 blocks: the FP32 sweep, then the refined
-  // solve's corrections (FP64 residuals), or (refine < 0) the FP32 solve's
-  // Woodbury step alone; the columns either leaves are solved directly
+  // solve's corrections (FP64 residuals); the columns it leaves are solved
+  // directly
   int gs = (int)((max_cols + kVicCols - 1) / kVicCols);
   if (p.refine) {
     const unsigned gt = (unsigned)((max_cols + 31) / 32);  // tiles of columns

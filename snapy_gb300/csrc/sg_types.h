@@ -199,6 +199,7 @@ struct StageParams {
   int32_t first;        // stage 0: the step fields start from zero
   int32_t refine;       // corrections of the refined implicit solve of
                         // implicit-precision float32 blocks (0: direct)
+  float accept;         // the error they may leave, of the solution
   unsigned long long* fallbacks;  // per block: columns the refined solve left
                                   // to the direct FP64 solve (a running count)
   unsigned long long* counts;     // per block, kCountSlots: this step's

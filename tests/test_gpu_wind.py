@@ -42,3 +42,16 @@ def test_refined_solution_in_a_strong_wind(cuda, flat, wind):
     want, _ = solution(cuda, flat, wind, 0)
     assert left == 0
     assert (torch.linalg.norm(got - want) / torch.linalg.norm(want)).item() <= 1e-13
+
+
+@pytest.mark.parametrize("flat,wind", [(1, 0.0), (8, 0.0), (8, 300.0), (50, 0.0), (50, 100.0),
+                                       (50, 300.0)])
+def test_fp32_solution_is_held_to_fp32_rounding(cuda, flat, wind):
+    """The FP32 form (sg_set_solve -1): every column it accepts within FP32's
+    rounding of its largest value (2^-24 by its own estimate; twice that here),
+    the others solved in FP64.  No column of these fails."""
+    got, left = solution(cuda, flat, wind, -1)
+    want, _ = solution(cuda, flat, wind, 0)
+    assert left == 0
+    err = (got - want).abs().amax(1) / want.abs().amax(1)
+    assert err.max().item() <= 2.0 ** -23
