@@ -39,7 +39,7 @@ using sg::StageParams;
   extern "C" int sg_launch_x3##sfx(const BlockDev*, StageParams, size_t,      \
                                    cudaStream_t);                              \
   extern "C" int sg_launch_reduce##sfx(const BlockDev*, int, int,              \
-                                       unsigned long long*, int*, size_t,      \
+                                       unsigned long long*, int*, int,         \
                                        cudaStream_t);                          \
   extern "C" int sg_launch_budget_totals##sfx(const BlockDev*, int, int,       \
                                               double*, cudaStream_t);          \
@@ -248,6 +248,7 @@ struct sg_handle {
   std::vector<double*> x1tabs;  // per-block geometry tables (gravity)
   bool has3 = false;            // a 3-D block: the x3 sweep runs
   bool visc3 = false;           // a 3-D block with viscosity: the prep runs
+  int red_ctas = 1;               // the reduction's per block (plan_reduce)
   int x3_chunk = 1, x3_ctas = 1;  // the x3 sweep's schedule (plan_x3)
   int line_seg = 0, line_ctas = 0;  // line_kernel's (plan_line)
   int fin_len = 0, fin_ctas = 0;  // the finish's schedule (plan_finish)
@@ -383,6 +384,25 @@ void plan_x3(sg_handle* h) {
   size_t w = 1;
   for (const sg_block_desc& d : h->descs) w = std::max(w, warps(d, h->x3_chunk));
   h->x3_ctas = (int)std::min<size_t>((w + 3) / 4, 8192);
+}
+
+// The reduction's CTAs per block: a cell a thread, the largest block's share
+// of about four CTAs an SM (each that has cells ends in three atomics on its
+// block's keys; one that has none still costs its launch).  Blocks much
+// smaller than the largest leave theirs empty, so from ten blocks up the share
+// stops at 64.  Forty FP64 blocks, one of 2048 x 128 and the rest 24 x 24, a
+// step: 2,110 us with 15 CTAs a block, 1,867 with 64
+void plan_reduce(sg_handle* h) {
+  size_t most = 0, sum = 0;
+  for (const sg_block_desc& d : h->descs) {
+    const size_t cells = (size_t)d.nc1 * d.nc2 * d.nc3;
+    most = std::max(most, cells);
+    sum += cells;
+  }
+  const size_t ctas = 608, share = ctas * most / sum;
+  h->red_ctas = (int)std::max<size_t>(
+      1, std::min({(most + 255) / 256, std::max<size_t>(share, 8),
+                   std::max<size_t>(ctas / h->nblock, 64)}));
 }
 
 // The columns a CTA of the implicit solve's finish takes (as the length of
@@ -1115,6 +1135,7 @@ int sg_create(const sg_scheme* scheme, const sg_block_desc* blocks,
     }
   }
   h->ntile = tile;
+  plan_reduce(h);
   if (h->has3) plan_x3(h);
   plan_line(h);
   if (h->implicit) {
@@ -1602,9 +1623,9 @@ int max_dt(sg_handle* h, int32_t* redo_dev, double* dt_out, int32_t set,
   int rc = upload(h, s);
   if (rc) return rc;
   rc = f64(h) ? sg_launch_reduce_f64(h->dev, h->nblock, h->cur, h->red,
-                                     h->nan, h->max_cells, s)
+                                     h->nan, h->red_ctas, s)
               : sg_launch_reduce_f32(h->dev, h->nblock, h->cur, h->red,
-                                     h->nan, h->max_cells, s);
+                                     h->nan, h->red_ctas, s);
   if (rc) return cuda_fail((cudaError_t)rc, "sg_max_dt: reduce");
   finish_dt_kernel<<<(h->nblock + 127) / 128, 128, 0, s>>>(
       h->nblock, h->red, h->nan, redo_dev, h->scheme.cfl, dt_out, set, host);
@@ -1640,9 +1661,9 @@ int sg_check(sg_handle* h, int32_t* flags, sg_stream_t stream) {
   int rc = upload(h, s);
   if (rc) return rc;
   rc = f64(h) ? sg_launch_reduce_f64(h->dev, h->nblock, h->cur, h->red,
-                                     h->nan, h->max_cells, s)
+                                     h->nan, h->red_ctas, s)
               : sg_launch_reduce_f32(h->dev, h->nblock, h->cur, h->red,
-                                     h->nan, h->max_cells, s);
+                                     h->nan, h->red_ctas, s);
   if (rc) return cuda_fail((cudaError_t)rc, "sg_check: reduce");
   finish_check_kernel<<<(h->nblock + 127) / 128, 128, 0, s>>>(
       h->nblock, h->red, h->nan, h->status, h->scheme.density_floor,
@@ -1664,9 +1685,9 @@ int sg_check_retry(sg_handle* h, int32_t* flags, int32_t* redo,
   int rc = upload(h, s);
   if (rc) return rc;
   rc = f64(h) ? sg_launch_reduce_f64(h->dev, h->nblock, h->cur, h->red,
-                                     h->nan, h->max_cells, s)
+                                     h->nan, h->red_ctas, s)
               : sg_launch_reduce_f32(h->dev, h->nblock, h->cur, h->red,
-                                     h->nan, h->max_cells, s);
+                                     h->nan, h->red_ctas, s);
   if (rc) return cuda_fail((cudaError_t)rc, "sg_check_retry: reduce");
   finish_check_kernel<<<(h->nblock + 127) / 128, 128, 0, s>>>(
       h->nblock, h->red, h->nan, h->status, h->scheme.density_floor,

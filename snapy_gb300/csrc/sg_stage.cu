@@ -2342,6 +2342,7 @@ __global__ void __launch_bounds__(kThreads)
   int nan = 0;
   // rows of 32-cell pieces, a warp a piece
   const unsigned pieces = (nx1 + 31) / 32, rows = (unsigned)nx2 * nx3;
+  if (blockIdx.x * (kThreads / 32) >= pieces * rows) return;
   for (unsigned e = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
        e < pieces * rows; e += gridDim.x * (kThreads / 32)) {
     const unsigned row = e / pieces, kr = row / nx2;
@@ -2855,14 +2856,10 @@ extern "C" int SG_NAME(sg_launch_psw_rcp)(const double* x, double* r,
 
 extern "C" int SG_NAME(sg_launch_reduce)(const BlockDev* tab, int nblock,
                                          int which, unsigned long long* red,
-                                         int* flag, size_t max_cells,
+                                         int* flag, int ctas,
                                          cudaStream_t stream) {
-  // a cell a thread, up to about four CTAs an SM over the blocks (each ends
-  // in three atomics on its block's keys)
-  const size_t most = std::max<size_t>(608 / nblock, 8);
-  const int gx = (int)std::min((max_cells + kThreads - 1) / kThreads, most);
-  reduce_kernel<<<dim3(gx, nblock), kThreads, 0, stream>>>(tab, which, red,
-                                                           flag);
+  reduce_kernel<<<dim3(ctas, nblock), kThreads, 0, stream>>>(tab, which, red,
+                                                             flag);
   return (int)cudaGetLastError();
 }
 
