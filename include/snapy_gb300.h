@@ -335,6 +335,8 @@ const char* sg_version(void);
  * --------------------------------------------------------------------- */
 typedef struct sg_cs_handle sg_cs_handle;
 typedef struct sg_cs_desc {
+  /* the tables below stay the caller's and keep their values: SG_F32 reads
+   * them in sg_cs_create, SG_F64 from the first stage on */
   int32_t n, ng, dtype, nstage;
   double wght[3][3];
   double cfl;

@@ -838,7 +838,8 @@ __global__ void cs_seam_rows(const double* tab, int nseam, int n, int nc, int* r
     const int p = (int)(di / fst), c = (int)(di % fst);
     const int k = x2 ? c / (nc + 1) : c / nc, j = x2 ? c % (nc + 1) : c % nc;
     const int side = x2 ? (j == kNg ? 0 : 1) : (k == kNg ? 2 : 3);
-    row[(p * 4 + side) * n + (x2 ? k : j) - kNg] = e;
+    const int along = (x2 ? k : j) - kNg;
+    if (p < 6 && along >= 0 && along < n) row[(p * 4 + side) * n + along] = e;
   }
 }
 
@@ -847,6 +848,7 @@ struct sg_cs_handle {
   void* w = nullptr;     // the primitives
   void* fgeo = nullptr;  // the faces' derived geometry
   int* srow = nullptr;   // the seam faces' rows
+  bool derived = false;  // fgeo and srow are formed
   // SG_F32: FP32 copies of the geometry and of the two seam tables
   float* geo32 = nullptr;
   float* gtab32 = nullptr;
@@ -859,6 +861,25 @@ struct sg_cs_handle {
   double* s2 = nullptr;  // the step fields (FP64, caller's memory)
   double* s3 = nullptr;
 };
+
+// What the stage reads of the tables in another form, once a handle: FP32 with
+// its copies at sg_cs_create, FP64, which reads the caller's tables in place,
+// before the first kernel that uses them (within a capture the launches become
+// part of the graph, and the next call makes them again)
+static void cs_derive(sg_cs_handle* h, cudaStream_t s) {
+  if (h->derived) return;
+  const int n = h->d.n, nc = n + 2 * kNg;
+  const int gf = grid_for((size_t)2 * nc * (nc + 1));
+  cs_seam_rows<<<grid_for(h->d.nseam), kThreads, 0, s>>>(h->d.seam_tab, h->d.nseam,
+                                                         n, nc, h->srow);
+  if (h->d.dtype == SG_F64)
+    cs_face_geo<double><<<gf, kThreads, 0, s>>>(h->d.geo, static_cast<double*>(h->fgeo), nc);
+  else
+    cs_face_geo<float><<<gf, kThreads, 0, s>>>(h->geo32, static_cast<float*>(h->fgeo), nc);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(s, &capture);
+  h->derived = capture == cudaStreamCaptureStatusNone;
+}
 
 extern "C" {
 
@@ -878,6 +899,12 @@ int sg_cs_create(const sg_cs_desc* d, sg_cs_handle** out) {
   if (!d->seam_state_tab || d->nseam_state != 24 * d->n)
     return cs_fail(SG_ERR_ARG, "sg_cs_create: the seam face-state table needs "
                    "24 n = %d rows (got %d)", 24 * d->n, d->nseam_state);
+  const size_t nc = (size_t)d->n + 2 * kNg, srows = (size_t)24 * d->n;
+  // the FP32 kernels read FP32 copies; the tables' flat indices (cells,
+  // and faces up to 6 nc (nc + 1)) stay exact in FP32 below 2^24
+  if (d->dtype == SG_F32 && 6 * nc * (nc + 1) >= (size_t)1 << 24)
+    return cs_fail(SG_ERR_UNSUPPORTED, "sg_cs_create: FP32 needs fewer than "
+                   "2^24 faces in the six panels (n %d)", d->n);
   auto* h = new sg_cs_handle();
   h->d = *d;
   // key[0]: the min key, key[1]: a NaN flag
@@ -887,30 +914,12 @@ int sg_cs_create(const sg_cs_desc* d, sg_cs_handle** out) {
     e = cudaMemcpy(h->key, init, sizeof(init), cudaMemcpyHostToDevice);
   }
   const size_t esz = d->dtype == SG_F64 ? 8 : 4;
-  const size_t ncp = (size_t)d->n + 2 * kNg, srows = (size_t)24 * d->n;
-  if (e == cudaSuccess) e = cudaMalloc(&h->w, 6 * 4 * ncp * ncp * esz);
-  if (e == cudaSuccess) e = cudaMalloc(&h->fgeo, 4 * ncp * (ncp + 1) * esz);
+  if (e == cudaSuccess) e = cudaMalloc(&h->w, 6 * 4 * nc * nc * esz);
+  if (e == cudaSuccess) e = cudaMalloc(&h->fgeo, 4 * nc * (nc + 1) * esz);
   if (e == cudaSuccess) e = cudaMalloc(&h->srow, srows * sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(h->srow, 0xff, srows * sizeof(int));
   if (e == cudaSuccess) e = cudaDeviceSynchronize();  // the tables are written
-  if (e == cudaSuccess) {
-    cs_seam_rows<<<grid_for(d->nseam), kThreads>>>(d->seam_tab, d->nseam, d->n,
-                                                   (int)ncp, h->srow);
-    if (d->dtype == SG_F64)
-      cs_face_geo<double><<<grid_for(2 * ncp * (ncp + 1)), kThreads>>>(
-          d->geo, static_cast<double*>(h->fgeo), (int)ncp);
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
-  }
   if (e == cudaSuccess && d->dtype == SG_F32) {
-    // the FP32 kernels read FP32 copies; the tables' flat indices (cells,
-    // and faces up to 6 nc (nc + 1)) stay exact in FP32 below 2^24
-    const size_t nc = (size_t)d->n + 2 * kNg;
-    if (6 * nc * (nc + 1) >= (size_t)1 << 24) {
-      sg_cs_destroy(h);
-      return cs_fail(SG_ERR_UNSUPPORTED, "sg_cs_create: FP32 needs fewer than "
-                     "2^24 faces in the six panels (n %d)", d->n);
-    }
     const size_t ng = 7 * nc * nc + 6 * nc * (nc + 1);
     const size_t nt = (size_t)kGhostStride * d->nghost;
     const size_t ns = (size_t)kSeamStride * d->nseam;
@@ -924,8 +933,7 @@ int sg_cs_create(const sg_cs_desc* d, sg_cs_handle** out) {
       to_f32<<<grid_for(nt), kThreads>>>(d->ghost_tab, h->gtab32, nt);
       to_f32<<<grid_for(ns), kThreads>>>(d->seam_tab, h->stab32, ns);
       to_f32<<<grid_for(nss), kThreads>>>(d->seam_state_tab, h->sst32, nss);
-      cs_face_geo<float><<<grid_for(2 * ncp * (ncp + 1)), kThreads>>>(
-          h->geo32, static_cast<float*>(h->fgeo), (int)ncp);
+      cs_derive(h, 0);
       e = cudaGetLastError();
       if (e == cudaSuccess) e = cudaDeviceSynchronize();
     }
@@ -1058,6 +1066,7 @@ int sg_cs_stage(sg_cs_handle* h, int32_t stage, const double* dt_dev,
   if (stage < 0 || stage >= h->d.nstage)
     return cs_fail(SG_ERR_ARG, "sg_cs_stage: stage %d of %d", stage, h->d.nstage);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  cs_derive(h, s);
   int in, u0, out;
   cs_plan(h, stage, &in, &u0, &out);
   CsParams P = cs_params(h);
