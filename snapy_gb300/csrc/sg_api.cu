@@ -34,7 +34,7 @@ using sg::StageParams;
                                      double* const*, size_t,                   \
                                      cudaStream_t);                            \
   extern "C" int sg_launch_vic##sfx(const BlockDev*, StageParams, size_t,     \
-                                    size_t, int*, cudaStream_t,                \
+                                    int*, cudaStream_t,                        \
                                     cudaEvent_t*);                             \
   extern "C" int sg_launch_x3##sfx(const BlockDev*, StageParams, size_t,      \
                                    cudaStream_t);                              \
@@ -269,7 +269,7 @@ struct sg_handle {
   double* psw_mem = nullptr;
   std::vector<size_t> psw_off;
   int any_f32 = 0;  // a block assembles its implicit blocks in FP32
-  size_t max_icells = 0, max_icols = 0;
+  size_t max_icols = 0;
   std::vector<sg_block_desc> descs;   // as created (tile re-layout)
   int32_t finish = 0;  // implicit finish form: 0 and 1 the rule's columns a
                        // CTA, 2 twice as many
@@ -768,10 +768,8 @@ int sg_autotune(sg_handle* h, int32_t reps, int32_t* tj_out,
       return r ? cuda_fail((cudaError_t)r, "sg_autotune: trial stage") : 0;
     };
     auto vic = [&]() -> int {
-      int r = f64(h) ? sg_launch_vic_f64(h->dev, p, h->max_icells, h->max_icols,
-                                         h->status, s, nullptr)
-                     : sg_launch_vic_f32(h->dev, p, h->max_icells, h->max_icols,
-                                         h->status, s, nullptr);
+      int r = f64(h) ? sg_launch_vic_f64(h->dev, p, h->max_icols, h->status, s, nullptr)
+                     : sg_launch_vic_f32(h->dev, p, h->max_icols, h->status, s, nullptr);
       return r ? cuda_fail((cudaError_t)r, "sg_autotune: trial solve") : 0;
     };
     auto timed = [&](auto&& launch, double* ms) -> int {
@@ -1125,7 +1123,6 @@ int sg_create(const sg_scheme* scheme, const sg_block_desc* blocks,
       B.asmc[3] = (gm1 + 1.) / gm1;
       B.asmc[4] = 1. / gm1r;
       B.asmc[5] = 1. / (gm1r + 1.);
-      h->max_icells = std::max(h->max_icells, icells);
       h->max_icols = std::max(h->max_icols, icols);
       const int nx1 = d.nc1 - 2 * d.ng;
       h->max_inx1 = std::max(h->max_inx1, nx1);
@@ -1531,11 +1528,9 @@ int sg_stage(sg_handle* h, int32_t stage, const double* dt_dev,
   if (rc) return cuda_fail((cudaError_t)rc, "sg_stage: stage kernel");
   if (timed) cudaEventRecord(ev[1], s);
   if (h->implicit) {
-    rc = f64(h) ? sg_launch_vic_f64(h->dev, p, h->max_icells, h->max_icols,
-                                    h->status, s,
+    rc = f64(h) ? sg_launch_vic_f64(h->dev, p, h->max_icols, h->status, s,
                                     timed ? ev + 2 : nullptr)
-                : sg_launch_vic_f32(h->dev, p, h->max_icells, h->max_icols,
-                                    h->status, s,
+                : sg_launch_vic_f32(h->dev, p, h->max_icols, h->status, s,
                                     timed ? ev + 2 : nullptr);
     if (rc) return cuda_fail((cudaError_t)rc, "sg_stage: implicit solve");
     if (timed) cudaEventRecord(ev[4], s);

@@ -238,6 +238,9 @@ constexpr int kCorSlot = 2 * 800 + 160;
 constexpr int kCorBack = 5;  // and its way out
 constexpr int kCorFloats = 2 * kCorRing * kCorSlot;
 static_assert(kCorBack * kBackSlot <= kCorRing * kCorSlot, "ring");
+// (within the 48 KB a CTA has without asking)
+static_assert(4 * (kFacFloats > kCorFloats ? kFacFloats : kCorFloats) +
+                      sizeof(MeetSmem) <= 48 * 1024, "shared memory");
 
 // rows of N values of a lane's column straight from an array's layer
 template <int N>

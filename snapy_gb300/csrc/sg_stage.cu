@@ -2747,8 +2747,7 @@ extern "C" int SG_NAME(sg_launch_init)(const BlockDev* tab, int nblock,
 // the three VIC launches of a stage (after the stage kernel wrote the
 // explicit tendency of the implicit blocks)
 extern "C" int SG_NAME(sg_launch_vic)(const BlockDev* tab, StageParams p,
-                                      size_t max_cells, size_t max_cols,
-                                      int* status,
+                                      size_t max_cols, int* status,
                                       cudaStream_t stream, cudaEvent_t* ev) {
   if (p.asm_kinds & 1)
     vic_assemble_kernel<double>
@@ -2767,22 +2766,6 @@ extern "C" int SG_NAME(sg_launch_vic)(const BlockDev* tab, StageParams p,
   int gs = (int)((max_cols + kVicCols - 1) / kVicCols);
   if (p.refine) {
     const unsigned gt = (unsigned)((max_cols + 31) / 32);  // tiles of columns
-    // the rings' opt-in shared memory, once a device (a handle's first launch
-    // is eager)
-    static bool granted[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 64 || !granted[dev]) {
-      cudaError_t g = cudaFuncSetAttribute(
-          vic_factor32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-          kFacFloats * (int)sizeof(float));
-      if (g == cudaSuccess)
-        g = cudaFuncSetAttribute(vic_correct32_kernel,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kCorFloats * (int)sizeof(float));
-      if (g != cudaSuccess) return (int)g;
-      if (dev < 64) granted[dev] = true;
-    }
     vic_factor32_kernel<<<dim3(gt, p.nblock), 64, kFacFloats * sizeof(float),
                           stream>>>(tab, p);
     for (int k = 1; k <= p.refine; ++k) {
