@@ -254,10 +254,11 @@ FP64_ISSUE = ("FP64 issue rate (one FP64 warp instruction per SM sub-partition "
 
 
 def refined(opts):
-    """True when the deck's implicit blocks take the refined solve."""
+    """True when the deck's implicit blocks take the refined solve (its FP32
+    form is one correction of it)."""
     ic = opts.hydro().icorr
     return bool(ic is not None and opts.hydro().precision == "float32"
-                and ic.precision == "float32" and opts.solve_corrections() > 0)
+                and ic.precision == "float32" and opts.solve_corrections() != 0)
 
 
 def block_bytes(opts):
@@ -265,6 +266,11 @@ def block_bytes(opts):
     ic = opts.hydro().icorr
     return 300 if (ic is not None and opts.hydro().precision == "float32"
                    and ic.precision == "float32") else 600
+
+
+def runs(dom, opts):
+    """What runs in the phase that kernel_times calls `dom`."""
+    return solve_phase(opts)[0] if dom == "vic_solve_kernel" else dom
 
 
 def solve_phase(opts):
@@ -280,7 +286,7 @@ def solve_phase(opts):
     if not refined(opts):
         return ("vic_solve_kernel", 600 + 40 + 200 + 120 + 200 + 120 + 120,
                 FP64_ISSUE)
-    k = opts.solve_corrections()
+    k = max(opts.solve_corrections(), 1)
     # the first sweep: A, B, C (300) and du (40) in; the inverses and C', B'
     # (200) and y (20) out; back out: C', B' and y in, x (20) out
     first = 300 + 40 + 200 + 20 + 120 + 20
@@ -606,9 +612,8 @@ def run_native(args):
                          "peak_kind": peak_kind, "traffic": None,
                          "basis": f"B_alg = {b_alg(s_bytes)} B per cell-update "
                                   "per RK3 step x the device-timed rate",
-                         "dominant_kernel": dom,
-                         "dominant_runs": solve_phase(opts)[0]
-                                          if dom == "vic_solve_kernel" else dom,
+                         "dominant_kernel": runs(dom, opts),
+                         "dominant_runs": runs(dom, opts),
                          "dominant_bytes_per_launch": per_launch[dom],
                          "dominant_mean_launch_us": dom_ms / dom_n * 1e3,
                          "dominant_kernel_gbs": achieved,
@@ -825,7 +830,7 @@ def run_ensemble(args, ranks=None, emit=True):
                          "peak_kind": peak_kind, "traffic": None,
                          "basis": f"B_alg = {b_alg(s_bytes)} B per cell-update "
                                   "per RK3 step x the device-timed rate",
-                         "dominant_kernel": dom,
+                         "dominant_kernel": runs(dom, members[0][0]),
                          "dominant_bytes_per_launch": per_launch[dom],
                          "dominant_mean_launch_us": dom_ms / dom_n * 1e3,
                          "dominant_kernel_gbs": achieved,
@@ -1161,7 +1166,7 @@ def run_serving(args, ranks=None, emit=True):
                                   "per RK3 step (5 reads + 3 writes x 5 "
                                   f"variables x {s_bytes} B) x the device-timed "
                                   "cell-updates/s of the whole step",
-                         "dominant_kernel": dom,
+                         "dominant_kernel": runs(dom, reqs[0].options),
                          "dominant_share": kms[dom][0] / ktot,
                          "scratch_bytes_per_cell_step": serving_scratch(reqs[0].options),
                          "limiter": solve_phase(reqs[0].options)[2]

@@ -411,12 +411,13 @@ void plan_reduce(sg_handle* h) {
 // for one column or 32, and with one CTA's worth of warps on an SM nothing
 // hides them.  One column at least fits a CTA: only the implicit blocks'
 // columns count, and their own tile (sg_stage_bound) holds them to about 2,200
-// layers, 89 KB here (the partial matrix 125 KB).  Measured per launch (us) with 1 / 2 / 4 / 8 / 16 / 32 columns:
-// 512 columns of 128, FP64: 73 / 44 / 45 / 61 / 91 / -; 301 of 75: 26 / 25 /
-// 32 / 40 / 56 / 94; 1,665 of 48: 106 / 58 / 49 / 37 / 39 / 63; 4,096 of 64,
-// FP32: 313 / 168 / 113 / 84 / 67 / 90.  kFinLen of 516 / 1032 / 1376 / 2064
-// / 4128: 64-member ensemble 525 / 399 / 311 / 346 / 515, four served requests
-// 1155 / 864 / 667 / 736 / 1122 (larger ones leave an SM two CTAs or one)
+// layers, 89 KB here (the partial matrix 125 KB).  Measured per launch (us)
+// with 1 / 2 / 4 / 8 / 16 / 32 columns: 512 columns of 128, FP64: 73 / 44 / 45
+// / 61 / 91 / -; 301 of 75: 26 / 25 / 32 / 40 / 56 / 94; 1,665 of 48: 106 / 58
+// / 49 / 37 / 39 / 63; 4,096 of 64, FP32: 313 / 168 / 113 / 84 / 67 / 90.
+// kFinLen of 516 / 1032 / 1376 / 2064 / 4128: 64-member ensemble 525 / 399 /
+// 311 / 346 / 515, four served requests 1155 / 864 / 667 / 736 / 1122 (larger
+// ones leave an SM two CTAs or one)
 void plan_finish(sg_handle* h) {
   int sms = 152;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);

@@ -53,14 +53,13 @@
 // 0.4 KB in a residual, 0.4 KB in a correction), and, with few columns, the
 // instructions of a column's layers one after the other: a layer's copies are
 // at constant offsets from pointers that step by a layer, and |x| and its
-// finiteness are one integer maximum.  Measured per launch (us), in four
-// forms: a column on eight lanes with LU factors and three right-hand sides;
-// this layout swept one way by a warp, the Woodbury vectors solved with b;
-// from both walls; and this one.  64-member ensemble (21,120 columns, 1.44 M
-// cells): first sweep 815 / 286 / 256 / 226, residual 634 / 222 / 160 / 160,
-// correction 613 / 129 / 119 / 95, acceptance and sum - / 93 / 60 / 60.  384
-// columns of 100: first sweep - / 154 / 65 / 57, correction - / 83 / 42 / 24;
-// 4,096 of 64: first sweep - / 101 / 63 / 60, correction - / 56 / 29 / 24.
+// finiteness are one integer maximum.  Measured per launch (us), before (a
+// column on eight lanes, one way, LU factors and three right-hand sides) and
+// now, 64-member ensemble (21,120 columns, 1.44 M cells): first sweep 815 and
+// 225, a residual 634 and 166 (the first) or 126, a correction 613 and
+// 95; the sum, apart now, 56.  384 columns of 100: first sweep 56,
+// correction 24 (this layout swept one way 154 and 83, from both walls with
+// the Woodbury vectors 65 and 42); 4,096 of 64: 60 and 25.
 #pragma once
 
 __device__ __forceinline__ bool vfinite32(float x) {
@@ -226,10 +225,10 @@ __device__ __forceinline__ unsigned largest(const float (&x)[5]) {
 }
 
 // The rings' depth costs a big batch warps per SM and gains a small one
-// nothing: the sweeps are bound by their instructions (the correction, 384
-// columns of 100, 41 us per launch with rings of 3 to 6 layers; 64 members 118
-// with 6, two CTAs an SM, and 103 with 3, five; the factor sweep's 259 with 8,
-// 235 with 5)
+// nothing: the sweeps are bound by their instructions (64 members, us per
+// launch when the depths were set: the correction 118 with 6 layers, two CTAs
+// an SM, and 103 with 3, five; the first sweep 259 with 8 and 235 with 5; 384
+// columns the same with 3 to 6)
 constexpr int kFacBack = 5;  // layers in a warp's ring, the factor's way out
 constexpr int kBackSlot = 800 + 160;
 constexpr int kFacFloats = 2 * kFacBack * kBackSlot;  // both warps' rings

@@ -2323,7 +2323,7 @@ __device__ __forceinline__ int warp_or(int x) {
 // order) and are widened once per CTA: an FP32 state's would otherwise sit on
 // the FP64 pipe, ten instructions a cell (64^3 FP32 32 us per
 // launch, now 6; 512 x 128 FP32 10.7 and 4.1, FP64 26 and 15; 64 members 86 and
-// 37; four requests 210 and 55).
+// 24; four requests 210 and 55).
 __global__ void __launch_bounds__(kThreads)
     reduce_kernel(const BlockDev* __restrict__ tab, int which,
                   unsigned long long* red, int* flag) {
@@ -2744,7 +2744,7 @@ extern "C" int SG_NAME(sg_launch_init)(const BlockDev* tab, int nblock,
   return (int)cudaGetLastError();
 }
 
-// the three VIC launches of a stage (after the stage kernel wrote the
+// the implicit solve's launches of a stage (after the stage kernel wrote the
 // explicit tendency of the implicit blocks)
 extern "C" int SG_NAME(sg_launch_vic)(const BlockDev* tab, StageParams p,
                                       size_t max_cols, int* status,

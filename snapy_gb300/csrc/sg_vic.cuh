@@ -15,15 +15,14 @@
 //   src/implicit/vic_kernels.h:100-160        back substitution, Woodbury
 //   src/implicit/vic_redistribute_impl.h      constituent column, cell map
 //   src/implicit/implicit_hydro.cpp:713-792   the gravity-work remainder
-// Three launches per stage, as the work's parallelism dictates: the blocks
-// of every cell in parallel (vic_assemble_kernel, one thread per cell), the
-// serial block-Thomas sweep of each column (vic_solve_kernel, one WARP per
-// column: the 5x5 block products run one entry per lane through warp
-// shuffles, the 8 right-hand sides of the LU back-solve one per lane, the
-// factorisation on the warp's shared-memory tile), and the column's
+// Per stage, as the work's parallelism dictates: the blocks of every cell
+// (vic_assemble_kernel, a thread per cell, the cells' and faces' common values
+// through its CTA's shared memory), the block-Thomas sweep of each column
+// (vic_solve_kernel, four columns a warp or a warp a column; sg_psolve.cuh and
+// sg_rsolve.cuh hold the partitioned and the refined forms), and the column's
 // redistribution, remainder and RK combine (vic_finish_kernel, a CTA per few
-// columns).  Every product is summed in index order, so the results are bit
-// for bit the CPU oracle's.
+// columns).  In the FP64 forms but the partitioned one every product is summed
+// in index order, so the results are bit for bit the CPU oracle's.
 #pragma once
 
 // Divisions of column and layer counts run in 32 bits: a block's interior
@@ -284,9 +283,8 @@ __device__ __forceinline__ void vic_prim32(const real* u, size_t plane,
   cons2prim<float>(uc, w, gammad);
 }
 
-// the corrected-PE slope weights of layer k of n (centres x)
-// the same weights from the block's x1 geometry table (computed once, with
-// these operations)
+// the corrected-PE slope weights of layer k of n, from the block's x1 geometry
+// table, and the first of their three layers
 __device__ __forceinline__ void vic_slope_tab(const BlockDev& B, int n, int k,
                                               double* wt, int* i0) {
   const double* t = B.x1tab + 6 * k;
@@ -323,12 +321,9 @@ __device__ __forceinline__ VicK vic_krows(const BlockDev& B, int n, int k) {
 }
 
 // (1) the blocks of every interior cell, the K coupling in their (IPR, IDN)
-// entries and du[IPR] -= K du[IDN] (its explicit row kept in du0)
-// the blocks of interior cell e (column e / n, layer e % n) in the compute
-// type T: double, or float under implicit-precision float32 (the FP32
-// state's blocks, exact in FP32 and in the FP64 copies the residuals of the
-// refined solve read).  The FP64 instantiation performs the reference's
-// operations in its order.
+// entries and du[IPR] -= K du[IDN] (its explicit row kept in du0), in the
+// compute type T: double, or float under implicit-precision float32.  The FP64
+// instantiation performs the reference's operations in its order.
 #ifndef SG_ASM32_CTAS
 #define SG_ASM32_CTAS 3
 #endif
@@ -584,11 +579,11 @@ __device__ __forceinline__ void vic_assemble_cell(
 // Bound by the FP64 pipe in FP64 (about 700 instructions a cell; a thread
 // that assembled its cell alone took 1280: three cells' primitives, two
 // Jacobians, both faces' |A|, the zeros' products), by its loads and stores
-// in FP32.  Measured per launch (us), before and now: 512 x 128 FP64 212 / 125,
-// 45 x 37 x 48 319 / 151, 301 x 75 108 / 64, nine members 330 / 210; FP32 64
-// members 418 / 258, four served requests 738 / 579 (with the tendency loaded
-// at its use 295 and 669; two CTAs an SM then 374 and
-// 874; a branch per store to either layout: 488 and 1155).
+// in FP32, which at three CTAs an SM spills 156 B a thread (80 registers; two
+// CTAs an SM do not, and take 1.3 times as long).  Measured per launch (us),
+// before and now: 512 x 128 FP64 212 / 125, 45 x 37 x 48 319 / 151, 301 x 75
+// 108 / 64, nine members 330 / 210; FP32 64 members 418 / 258, four served
+// requests 738 / 579.
 template <typename T>
 __global__ void __launch_bounds__(AsmShape<T>::threads, AsmShape<T>::ctas)
     vic_assemble_kernel(const BlockDev* __restrict__ tab, StageParams p) {
@@ -652,8 +647,6 @@ __global__ void __launch_bounds__(AsmShape<T>::threads, AsmShape<T>::ctas)
                          kc, sm, t, du0);
 }
 
-// ludcmp<double, 5, Implicit> on a row-major 5x5 in shared memory
-// (src/math/ludcmp.h); one lane runs it
 // ---------------------------------------------------------------------------
 // (2) the block-Thomas sweep, back substitution and Woodbury update.
 //
@@ -1623,7 +1616,7 @@ __global__ void __launch_bounds__(kThreads)
 // per column, its passes on lane 0; wide batches three launches, a thread per
 // column for the passes) and now: 512 columns of 128 FP64 138 and 45, 301 of
 // 75 85 and 25, 384 of 100 FP32 106 and 35, 4,096 of 64 113 and 65, nine FP64
-// members 153 and 58, 64 members 477 and 287, four served requests 829 and
+// members 153 and 58, 64 members 477 and 286, four served requests 829 and
 // 612.
 constexpr int kFinThreads = 256;
 
