@@ -1067,7 +1067,8 @@ int sg_create(const sg_scheme* scheme, const sg_block_desc* blocks,
     if (d.nc3 > 1) h->has3 = true;
     B.tile0 = tile;
     tile += B.ntile;
-    // (a tile is refused by the size of its regions laid apart)
+    // the largest block accepted is set by the tile's regions laid apart, so it
+    // does not move with the layout that stage_smem gives
     size_t sm = stage_smem(h, d, B.tj, true);
     if ((long)sm > optin) {
       sg_destroy(h);
